@@ -36,6 +36,7 @@
 //
 // Flop count per interaction (FMA = 2, rsqrt = 1): monopole 20, quadrupole
 // cell 59.  These are the per-interaction figures used for the roofline.
+#include <climits>
 #include <cstring>
 #include "hc_internal.cuh"
 #include "hc_mlp.cuh"
@@ -166,29 +167,55 @@ __device__ __forceinline__ unsigned hash2(unsigned a, unsigned b)
     return h;
 }
 
-__device__ __forceinline__ float wmin(float v)
+// Warp minima and maxima by the integer reduction instruction (one per 32-bit
+// word) on keys that order like the values.  A chain of floating compares costs
+// five shuffles, and for doubles five steps on the FP64 pipe, which one warp
+// instruction holds for 16 cycles: the group's centre and relative positions
+// took about 70 of those.  The float versions see no NaN; the double versions
+// leave NaN out as fmin and fmax do (all NaN: NaN).
+__device__ __forceinline__ int order_key(float v)
 {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(FULL, v, o));
-    return v;
+    const int i = __float_as_int(v);
+    return i ^ ((i >> 31) & 0x7fffffff);
 }
-__device__ __forceinline__ float wmax(float v)
+__device__ __forceinline__ float order_val(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+__device__ __forceinline__ float wmin(float v) { return order_val(__reduce_min_sync(FULL, order_key(v))); }
+__device__ __forceinline__ float wmax(float v) { return order_val(__reduce_max_sync(FULL, order_key(v))); }
+
+__device__ __forceinline__ long long order_key(double v)
 {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULL, v, o));
-    return v;
+    const long long i = __double_as_longlong(v);
+    return i ^ ((i >> 63) & 0x7fffffffffffffffll);
 }
-__device__ __forceinline__ double wmind(double v)
+__device__ __forceinline__ double order_val(long long k)
 {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmin(v, __shfl_xor_sync(FULL, v, o));
-    return v;
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
-__device__ __forceinline__ double wmaxd(double v)
+__device__ __forceinline__ long long wminll(long long k)
 {
+    const int hi = __reduce_min_sync(FULL, (int)(k >> 32));
+    const unsigned lo = __reduce_min_sync(FULL, (int)(k >> 32) == hi ? (unsigned)k : 0xffffffffu);
+    return (long long)((unsigned long long)(unsigned)hi << 32 | lo);
+}
+__device__ __forceinline__ long long wmaxll(long long k)
+{
+    const int hi = __reduce_max_sync(FULL, (int)(k >> 32));
+    const unsigned lo = __reduce_max_sync(FULL, (int)(k >> 32) == hi ? (unsigned)k : 0u);
+    return (long long)((unsigned long long)(unsigned)hi << 32 | lo);
+}
+// centre of the range of the warp's values, 0.5 (min + max), NV values per lane
+template <int NV>
+__device__ __forceinline__ double wcentre(const double (&v)[NV])
+{
+    long long lo = LLONG_MAX, hi = LLONG_MIN;     // both decode to NaN
 #pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL, v, o));
-    return v;
+    for (int k = 0; k < NV; k++) {
+        const long long q = order_key(v[k]);
+        if ((hc_dbits(v[k]) << 1) > 0xffe0000000000000ull) continue;      // NaN
+        lo = q < lo ? q : lo;
+        hi = q > hi ? q : hi;
+    }
+    return 0.5 * (order_val(wminll(lo)) + order_val(wmaxll(hi)));
 }
 
 __device__ __forceinline__ void kahan_add(float &sum, float &comp, float x)
@@ -344,36 +371,20 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
         const unsigned vmask = __ballot_sync(FULL, valid[0]);
 
         // group centre (FP64) and body positions relative to it (FP32)
-        double gx, gy, gz;
-        {
-            double lox = xd[0], hix = xd[0], loy = yd[0], hiy = yd[0], loz = zd[0], hiz = zd[0];
-#pragma unroll
-            for (int k = 1; k < BPL; k++) {
-                lox = fmin(lox, xd[k]);
-                hix = fmax(hix, xd[k]);
-                loy = fmin(loy, yd[k]);
-                hiy = fmax(hiy, yd[k]);
-                loz = fmin(loz, zd[k]);
-                hiz = fmax(hiz, zd[k]);
-            }
-            gx = 0.5 * (wmind(lox) + wmaxd(hix));
-            gy = 0.5 * (wmind(loy) + wmaxd(hiy));
-            gz = 0.5 * (wmind(loz) + wmaxd(hiz));
-        }
-        const float ghx = __double2float_rn(gx), ghy = __double2float_rn(gy), ghz = __double2float_rn(gz);
-        const float glx = __double2float_rn(gx - (double)ghx), gly = __double2float_rn(gy - (double)ghy),
-                    glz = __double2float_rn(gz - (double)ghz);
+        const double gx = wcentre(xd), gy = wcentre(yd), gz = wcentre(zd);
+        // hi and lo parts by integer operations (hc_f32split.h): no FP64-pipe conversions
+        float ghx, ghy, ghz, glx, gly, glz;
+        hc_split_hilo(gx, &ghx, &glx);
+        hc_split_hilo(gy, &ghy, &gly);
+        hc_split_hilo(gz, &ghz, &glz);
         // low parts: body-body separations are formed as (hi - hi) + (lo - lo)
         float bx[BPL], by[BPL], bz[BPL], blx[BPL], bly[BPL], blz[BPL];
         float mnx = 3.0e38f, mxx = -3.0e38f, mny = 3.0e38f, mxy = -3.0e38f, mnz = 3.0e38f, mxz = -3.0e38f, r2m = 0.f;
 #pragma unroll
         for (int k = 0; k < BPL; k++) {
-            bx[k] = __double2float_rn(xd[k] - gx);
-            by[k] = __double2float_rn(yd[k] - gy);
-            bz[k] = __double2float_rn(zd[k] - gz);
-            blx[k] = __double2float_rn((xd[k] - gx) - (double)bx[k]);
-            bly[k] = __double2float_rn((yd[k] - gy) - (double)by[k]);
-            blz[k] = __double2float_rn((zd[k] - gz) - (double)bz[k]);
+            hc_split_hilo(xd[k] - gx, &bx[k], &blx[k]);
+            hc_split_hilo(yd[k] - gy, &by[k], &bly[k]);
+            hc_split_hilo(zd[k] - gz, &bz[k], &blz[k]);
             mnx = fminf(mnx, bx[k]);
             mxx = fmaxf(mxx, bx[k]);
             mny = fminf(mny, by[k]);
@@ -650,10 +661,20 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             // ---- classify each candidate against the group ----
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
             int2 C = make_int2(0, 0);
+            // The error rule reads the cell's radius beside its quadrupole: loading
+            // both with the node saves the accepted cells a second round trip
+            // (Hernquist 2^22: 10.86 -> 10.70 ms).  The other rules read the
+            // quadrupole of accepted cells only; early loads did not help there.
+            constexpr bool QEARLY = QUAD && MODE == 2;
+            float4 Q0 = A, Q1 = A;
             if (have) {
                 A = g.nodeA[my_node];
                 B = g.nodeB[my_node];
                 C = g.nodeC[my_node];
+                if (QEARLY) {
+                    Q0 = g.nodeQ[2 * (int64_t)my_node];
+                    Q1 = g.nodeQ[2 * (int64_t)my_node + 1];
+                }
             }
             if (MODE == 3 && mlp_round) {
                 // lane r builds the feature row of the round's candidate r (rows
@@ -750,7 +771,7 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
                             bd_err = err;
                         }
                     } else if (MODE == 2) {
-                        const float b = g.nodeQ[2 * (int64_t)my_node + 1].w;
+                        const float b = QEARLY ? Q1.w : g.nodeQ[2 * (int64_t)my_node + 1].w;
                         const float gap = dmin2 * rsqrtf(dmin2) - b;          // as in MODE 3
                         bool acc_ok = gap > 0.f && tmin >= dsq * 0.0625f;     // never beyond size/dmin = 4
                         if (acc_ok) {
@@ -866,13 +887,16 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
                 f[4] = cz;
                 f[6] = A.w;
                 if (QUAD) {
-                    const float4 q0 = g.nodeQ[2 * (int64_t)my_node], q1 = g.nodeQ[2 * (int64_t)my_node + 1];
-                    f[8] = -q0.x;
-                    f[10] = -q0.y;
-                    f[12] = -q0.z;
-                    f[14] = -q0.w;
-                    f[16] = -q1.x;
-                    f[18] = -q1.y;
+                    if (!QEARLY) {
+                        Q0 = g.nodeQ[2 * (int64_t)my_node];
+                        Q1 = g.nodeQ[2 * (int64_t)my_node + 1];
+                    }
+                    f[8] = -Q0.x;
+                    f[10] = -Q0.y;
+                    f[12] = -Q0.z;
+                    f[14] = -Q0.w;
+                    f[16] = -Q1.x;
+                    f[18] = -Q1.y;
                 }
                 if (MASKED) (pos & 1 ? S.cmask[pos >> 1].y : S.cmask[pos >> 1].x) = accm;
                 gc += MODE == 0 ? __popc(accm) : (unsigned)cnt;
@@ -1170,18 +1194,7 @@ __global__ void __launch_bounds__(128) k_label(WalkArgs g, const int *gstart, co
         yd[k] = py[o[k]];
         zd[k] = pz[o[k]];
     }
-    double lox = xd[0], hix = xd[0], loy = yd[0], hiy = yd[0], loz = zd[0], hiz = zd[0];
-#pragma unroll
-    for (int k = 1; k < BPL; k++) {
-        lox = fmin(lox, xd[k]);
-        hix = fmax(hix, xd[k]);
-        loy = fmin(loy, yd[k]);
-        hiy = fmax(hiy, yd[k]);
-        loz = fmin(loz, zd[k]);
-        hiz = fmax(hiz, zd[k]);
-    }
-    const double gx = 0.5 * (wmind(lox) + wmaxd(hix)), gy = 0.5 * (wmind(loy) + wmaxd(hiy)),
-                 gz = 0.5 * (wmind(loz) + wmaxd(hiz));
+    const double gx = wcentre(xd), gy = wcentre(yd), gz = wcentre(zd);
     const float ghx = __double2float_rn(gx), ghy = __double2float_rn(gy), ghz = __double2float_rn(gz);
     const float glx = __double2float_rn(gx - (double)ghx), gly = __double2float_rn(gy - (double)ghy),
                 glz = __double2float_rn(gz - (double)ghz);
