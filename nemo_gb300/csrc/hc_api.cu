@@ -75,7 +75,9 @@ void free_all(hc_ctx *c)
     void *mptrs[] = {c->mlp_p, c->mlp_m, c->mlp_v, c->mlp_grad, c->mlp_loss, c->mlp_gpart, c->mlp_lpart,
                      c->mlp_packed, c->sample_count, c->sample_x, c->sample_amin, c->sample_y, c->sample_rel,
                      c->sample_w, c->sample_group, c->sample_node, c->guard_idx, c->guard_part, c->guard,
-                     c->rcrit2, c->phi_ext};
+                     c->rcrit2, c->phi_ext, c->split.ctl, c->split.out, c->split.task[0], c->split.task[1],
+                     c->split.entry[0], c->split.entry[1], c->split.group, c->split.sub, c->split.part,
+                     c->split.part_cnt};
     for (void *p : mptrs)
         if (p) cudaFree(p);
     if (c->h_st) cudaFreeHost(c->h_st);
@@ -157,6 +159,29 @@ int alloc_all(hc_ctx *c)
         HC_CUDA(cudaMemset(pk, 0, sizeof(MlpSmem)));
     }
     HC_TRY(dalloc(c, &c->sample_count, 2));
+    {
+        // split walks (outlying groups only): sized for some 10^4 parts, less for small systems
+        hc_walk_split &w = c->split;
+        const int64_t small = std::max<int64_t>(64, n);
+        w.out_cap = (int)small;
+        w.slot_cap[0] = (int)std::min<int64_t>(4096, small);
+        w.slot_cap[1] = (int)std::min<int64_t>(16384, small);
+        w.entry_cap[0] = (int)std::min<int64_t>(65536, 16 * small);
+        w.entry_cap[1] = (int)std::min<int64_t>(262144, 16 * small);
+        w.slot0[0] = 0;
+        w.slot0[1] = w.slot_cap[0];
+        const int64_t slots = w.slot_cap[0] + (int64_t)w.slot_cap[1];
+        HC_TRY(dalloc(c, &w.ctl, 1));
+        HC_TRY(dalloc(c, &w.out, w.out_cap));
+        for (int k = 0; k < 2; k++) {
+            HC_TRY(dalloc(c, &w.task[k], w.slot_cap[k]));
+            HC_TRY(dalloc(c, &w.entry[k], w.entry_cap[k]));
+        }
+        HC_TRY(dalloc(c, &w.group, w.slot_cap[0]));
+        HC_TRY(dalloc(c, &w.sub, w.slot_cap[0]));
+        HC_TRY(dalloc(c, &w.part, 2 * slots * HC_GROUP2));
+        HC_TRY(dalloc(c, &w.part_cnt, slots * HC_GROUP2));
+    }
     HC_TRY(dalloc(c, &c->box, 1));
     HC_CUDA(cudaMallocHost((void **)&c->h_st, sizeof(hc_status)));
     HC_CUDA(cudaMallocHost((void **)&c->h_box, sizeof(hc_box)));

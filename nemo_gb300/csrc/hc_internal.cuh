@@ -69,6 +69,32 @@ struct hc_box {
     double dsq[HC_MAXLEVEL + 1];       // rsize^2 / 4^level (grav.c:86,105)
 };
 
+// Split walks (hc_walk.cu).
+struct hc_walk_ctl {
+    unsigned fetch[4];        // items taken by each phase
+    int nout, ntask[2], ngroup;
+};
+struct hc_walk_task {
+    int group;                // walk group
+    int entry0, n;            // its traversal entries
+    int slot;                 // of its partial sums
+};
+struct hc_walk_parts {        // a split group
+    int s0, cnt;              // first target slot, targets
+    int own, first, n;        // slot of its own partial sums, its level-0 tasks' slots
+};
+struct hc_walk_split {
+    hc_walk_ctl *ctl;
+    int *out;                 // groups whose walk exceeded its budget
+    hc_walk_task *task[2];
+    uint2 *entry[2];          // (first node << 3 | count - 1, lane mask)
+    hc_walk_parts *group;
+    int2 *sub;                // level-0 slot: first slot and number of its tasks
+    float4 *part;             // [slot][HC_GROUP2][2] partial sums (x, y, z, phi): Kahan sum, compensation
+    int2 *part_cnt;           // [slot][HC_GROUP2] interaction counts (counting walk)
+    int out_cap, entry_cap[2], slot_cap[2], slot0[2];
+};
+
 struct hc_ctx {
     int64_t n;                // bodies
     int64_t maxcell;          // (int)(fcells * n), load.c:50
@@ -124,6 +150,7 @@ struct hc_ctx {
     double *nm, *ncx, *ncy, *ncz;         // FP64 mass and centre of mass per node
     int cofm_grid;                        // co-resident blocks of the upward-pass kernel
     int walk_blocks[20];                  // resident blocks of each walk variant
+    hc_walk_split split;                  // buffers of split walks
     // learned opening criterion: network, training state, samples
     struct MlpSmem *mlp_packed;           // BF16 image used by the walk
     float *mlp_p, *mlp_m, *mlp_v;         // FP32 master weights, Adam moments

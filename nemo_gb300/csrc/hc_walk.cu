@@ -36,7 +36,9 @@
 //
 // Flop count per interaction (FMA = 2, rsqrt = 1): monopole 20, quadrupole
 // cell 59.  These are the per-interaction figures used for the roofline.
+#include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include "hc_internal.cuh"
 #include "hc_mlp.cuh"
@@ -70,7 +72,12 @@ struct WarpSmem {
     float4 cp[CCAP / 2][5];     // cell pairs, likewise: (x y) (z m) (-Qxx -Qxy) (-Qxz -Qyy) (-Qyz -Qzz)
     uint2 cmask[CCAP / 2];      // cell pairs: accept masks (per-body rule, counting walk)
     unsigned long long stat[8]; // warp totals (lane 0 writes): see the ST_* indices
-    float gu[16];               // the group's uniform values (see GU_* below), read where used
+    float gu[15];               // the group's uniform values (see GU_* below), read where used
+    // split walks: whether this one is split, bodies of a cell that becomes a
+    // task's entry, entries kept, room for entries, first entry
+    int split;
+    float light;
+    int nentry, room, entry0;
 };
 enum { ST_N2B, ST_NBC, ST_CAND, ST_MIXED, ST_EB, ST_EC, ST_MLP, ST_ROUNDS };
 
@@ -99,7 +106,10 @@ struct WalkArgs {
     int64_t nstep;
     double *vx, *vy, *vz;
     hc_status *st;
-    unsigned *group_counter;
+    hc_walk_split sp;                     // split walks: see below
+    int phase;
+    int warps;                            // resident warps of the whole GPU
+    float split_scale;                    // expected length of a group's walk, relative to theta = 0.5
     const int32_t *gstart, *gcount;       // tree-aligned groups of the massive targets
     int use_table;                        // 1: table groups, then massless targets in 32s
     float eps_acc;                        // MODE 2/3 error budget relative to |a|
@@ -282,6 +292,90 @@ __device__ __forceinline__ void cell_term(const float4 P, const float4 Q0, const
     paz = fmaf(c, dz, fmaf(-r5, qz, paz));
 }
 
+// ---- split walks ----
+// Under the group criteria a group's decisions follow its bounding box.  Where
+// outlying bodies of several small cells are packed together the box spreads
+// over the whole system and covers the core: every cell opens, and one warp
+// walks all bodies.  (One such group of a 2^20-body Plummer sphere took 25 ms
+// of a 29 ms walk, one of a 262,143-body Hernquist sphere 33 of 34 ms.)  A
+// walk that exceeds a budget of iterations is therefore given up and split
+// into tasks that any warp takes: the group's warp opens only cells of more
+// than `light` bodies, and a smaller cell that opens is kept as an entry (its
+// child range and opening mask).
+//   phase 0: all groups; the walks over budget are given up and listed.
+//   phase 1: the listed groups are split coarsely, into tasks of level 0.
+//   phase 2: the tasks of level 0 are split finely, into tasks of level 1.
+//   phase 3: the tasks of level 1 are walked.
+// Each part's sums go to a slot of its own, and k_walk_combine adds them in a
+// fixed order.  What is split, and into what, follows from the bodies alone:
+// every item has an equal share of the entries and slots and goes on by itself
+// when its share is used up.  So the results do not depend on timing.  With
+// nothing to split the later phases are four empty launches (about 10 us).
+// Measured: 2^20 bodies with such a group, error rule, 24.9 -> 5.3 ms (5.1
+// without one); the Hernquist sphere 34.3 -> 1.6 ms.  The per-body rule opens
+// cells body by body and has no such walks: it is not split.
+struct SplitRule {
+    int split;
+    float light;
+    int entries, slots;                  // an item's share
+};
+
+// Iterations after which a group's walk is given up: several times a warp's
+// average share of the work.
+__device__ __forceinline__ int split_budget(const WalkArgs &g, int64_t ngroups)
+{
+    return (int)fminf((96.f + 64.f * (float)ngroups / (float)g.warps) * g.split_scale, 1.0e9f);
+}
+
+__device__ __forceinline__ SplitRule split_rule(const WalkArgs &g, int nitem)
+{
+    SplitRule r = {0, 0.f, 0, 0};
+    if (g.phase == 3) return r;
+    const float n = (float)g.box->nmassive;
+    const int level = g.phase - 1;
+    r.entries = g.sp.entry_cap[level] / nitem;
+    r.slots = g.sp.slot_cap[level] / nitem;
+    r.split = r.entries >= 64 && r.slots >= 4;
+    // about 100 tasks for each group, then some 10^4 in all (a few thousand
+    // bodies each at most); the entries of an item have to fit its share
+    if (level == 0) r.light = fmaxf(n * (1.f / 32.f), 512.f);
+    else r.light = fmaxf(fmaxf(n * (1.f / 4096.f), 256.f), n * 0.125f / (float)r.entries);
+    return r;
+}
+
+// The end of an item of a split walk: its entries become tasks.  Returns the
+// slot of the item's own partial sums, -1 for a group that left no entries
+// (its results are final).
+__device__ __noinline__ int split_finish(const WalkArgs &g, WarpSmem &S, const SplitRule &rule, int item,
+                                         const hc_walk_task &task, int grp, int s0, int cnt, int lane)
+{
+    if (g.phase == 3) return task.slot;
+    const int E = rule.split ? S.nentry : 0, level = g.phase - 1;
+    int own = g.phase == 2 ? task.slot : -1;
+    if (E > 0) {
+        // a group's own slot is the first of its share
+        int first = g.sp.slot0[level] + item * rule.slots;
+        const int extra = own < 0 ? 1 : 0;
+        if (extra) own = first++;
+        int T = min(E, rule.slots - extra);
+        const int per = (E + T - 1) / T;
+        T = (E + per - 1) / per;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&g.sp.ctl->ntask[level], T);
+        base = __shfl_sync(FULL, base, 0);
+        for (int t = lane; t < T; t += 32)
+            g.sp.task[level][base + t] = hc_walk_task{grp, S.entry0 + t * per, min(per, E - t * per), first + t};
+        if (lane == 0) {
+            if (g.phase == 2) g.sp.sub[own] = make_int2(first, T);
+            else g.sp.group[atomicAdd(&g.sp.ctl->ngroup, 1)] = hc_walk_parts{s0, cnt, own, first, T};
+        }
+    } else if (g.phase == 2 && lane == 0) {
+        g.sp.sub[own] = make_int2(0, 0);
+    }
+    __syncwarp();
+    return own;
+}
+
 // MODE 0: the reference's per-body opening rule (exact interaction sets).
 // MODE 1: group rule -- a cell is accepted for the whole group when
 //         tol^2 * dmin^2 >= size^2 with dmin the distance from the group's
@@ -295,13 +389,18 @@ __device__ __forceinline__ void cell_term(const float4 P, const float4 Q0, const
 // network's walk carries none of its code.
 // Register budget: 96 (5 blocks of 4 warps per SM) for the per-body rule,
 // 128 (4 blocks) for the group, error and learned rules.
-template <bool QUAD, bool COUNT, int MODE, bool COLLECT = false>
+// SPLIT: the walk's split phases (groups walked in parts), compiled apart so
+// that the walk of whole groups carries none of their code.
+template <bool QUAD, bool COUNT, int MODE, bool COLLECT = false, bool SPLIT = false>
 __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs g)
 {
     if (g.run_flag && *g.run_flag == 0) return;   // guard passed: no fallback walk
     // group criteria accept a cell for the whole group (a cell holding the
     // group's own bodies is always opened): cell entries need no lane mask
     constexpr bool MASKED = MODE == 0;
+    // this launch's groups or tasks; later phases often have none
+    const int nitem = !SPLIT ? 0 : (g.phase == 1 ? g.sp.ctl->nout : g.sp.ctl->ntask[g.phase - 2]);
+    if (SPLIT && nitem == 0) return;
     extern __shared__ float4 smem_raw[];
     WarpSmem &S = reinterpret_cast<WarpSmem *>(smem_raw)[threadIdx.x >> 5];
     // MODE 3: per-warp queues after the warp areas, then the network's
@@ -338,16 +437,40 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
     if (lane < 8) S.stat[lane] = 0ull;
     __syncwarp();
     int max_sp = 0, nborder = 0;
+    // the label walk is not split: it would sample a given-up group twice
+    constexpr bool BUDGET = !SPLIT && MODE != 0 && !COLLECT;
+    SplitRule rule = {};
+    int budget = INT_MAX;
+    if (SPLIT) {
+        rule = split_rule(g, nitem);
+        if (lane == 0) {
+            S.split = rule.split;
+            S.light = rule.light;
+            S.room = rule.entries;
+        }
+        __syncwarp();
+    } else if (BUDGET && ngroups <= g.sp.out_cap) {
+        budget = split_budget(g, ngroups);
+    }
 
     while (true) {
         int64_t grp;
+        int item;
         {
             unsigned v = 0;
-            if (lane == 0) v = atomicAdd(g.group_counter, 1u);
+            if (lane == 0) v = atomicAdd(&g.sp.ctl->fetch[g.phase], 1u);
             grp = (int64_t)__shfl_sync(FULL, v, 0);
+            item = (int)grp;
         }
-        if (grp >= ngroups) break;
         int64_t s0, cnt;
+        hc_walk_task task = {};
+        if (SPLIT) {
+            if (item >= nitem) break;
+            if (g.phase >= 2) task = g.sp.task[g.phase - 2][item];
+            grp = g.phase == 1 ? g.sp.out[item] : task.group;
+        } else if (grp >= ngroups) {
+            break;
+        }
         if (grp < ng_table) {
             s0 = g.gstart[grp];
             cnt = g.gcount[grp];
@@ -571,6 +694,9 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
         };
 
         int sp = 0, nb = 0, nc = 0;
+        // iterations left; a whole group's walk that has none left is given up,
+        // a split walk has none from the start
+        int left = SPLIT ? (rule.split ? 0 : INT_MAX) : budget;
         bool overflow = false;
         int root = 0;
         if (g.sys_root) {                     // forest: this group's system root
@@ -580,9 +706,16 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
                 continue;
             }
         }
-        if (nnode > 0) {
+        if (SPLIT && g.phase >= 2) {               // a task's entries (<= STACK / 2)
+            sp = task.n;
+            for (int i = lane; i < sp; i += 32) S.stack[i] = g.sp.entry[g.phase - 2][task.entry0 + i];
+        } else if (nnode > 0) {
             if (lane == 0) S.stack[0] = make_uint2((unsigned)root << 3, vmask);   // root, one node
             sp = 1;
+        }
+        if (SPLIT && lane == 0) {
+            S.nentry = 0;
+            S.entry0 = item * rule.entries;
         }
         __syncwarp();
         int qn = 0;                                          // MODE 3: queued band candidates
@@ -844,7 +977,23 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
 
             // ---- push opened cells' child ranges ----
             // children always follow their parent and number 1..8
-            const bool push = openm != 0u && C.x > my_node && (C.y & 255) >= 1 && (C.y & 255) <= 8;
+            bool push = openm != 0u && C.x > my_node && (C.y & 255) >= 1 && (C.y & 255) <= 8;
+            if ((SPLIT || BUDGET) && --left < 0) {
+                if (!SPLIT) break;               // given up: listed below
+                const bool small = push && g.nodeQ[2 * (int64_t)my_node + 1].z <= S.light;
+                const unsigned sb = __ballot_sync(FULL, small);
+                const int have_e = S.nentry, at = have_e + __popc(sb & lt);
+                if (have_e + __popc(sb) <= S.room) {
+                    if (small)
+                        g.sp.entry[g.phase - 1][S.entry0 + at] =
+                            make_uint2(((unsigned)C.x << 3) | (unsigned)((C.y & 255) - 1), openm);
+                    push = push && !small;
+                    __syncwarp();
+                    if (lane == 0) S.nentry = have_e + __popc(sb);
+                } else {
+                    left = INT_MAX;              // no room for more entries: the rest is walked here
+                }
+            }
             const unsigned pb = __ballot_sync(FULL, push);
             const int npush = __popc(pb);
             if (sp + npush > STACK) {
@@ -915,6 +1064,10 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             __syncwarp();
         }
 #undef GUV
+        if (BUDGET && left < 0) {
+            if (lane == 0) g.sp.out[atomicAdd(&g.sp.ctl->nout, 1)] = (int)grp;
+            continue;
+        }
         if (overflow) {
             if (lane == 0) {
                 atomicCAS(&g.st->error, 0, HC_ERR_STACK);
@@ -937,11 +1090,20 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             }
         }
         __syncwarp();
+        // slot of the partial sums of a split walk (-1: the results are final)
+        const int slot = SPLIT ? split_finish(g, S, rule, item, task, (int)grp, (int)s0, (int)cnt, lane) : -1;
 
 #pragma unroll
         for (int k = 0; k < BPL; k++) {
             if (!valid[k]) continue;
             const uint32_t ok = o[k];
+            if (slot >= 0) {                      // k_walk_combine adds the parts
+                const int64_t q = (int64_t)slot * HC_GROUP2 + lane + 32 * k;
+                g.sp.part[2 * q] = make_float4(sax[k], say[k], saz[k], sphi[k]);
+                g.sp.part[2 * q + 1] = make_float4(cax[k], cay[k], caz[k], cphi[k]);
+                if (COUNT) g.sp.part_cnt[q] = make_int2(myb[k], myc[k]);
+                continue;
+            }
             const double rphi = (double)sphi[k] - (double)cphi[k];
             const double rax = (double)sax[k] - (double)cax[k], ray = (double)say[k] - (double)cay[k],
                          raz = (double)saz[k] - (double)caz[k];
@@ -986,11 +1148,99 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
     }
 }
 
+// The parts of a split group, stored as the walk's epilogue does.  A block
+// takes four bodies of a group: its 128 lanes per body add the parts of every
+// 128th task (each followed by its own tasks) and the lanes' sums are added in
+// a fixed order.  The sums run in pairs of floats (each addition's rounding
+// error is kept): on the FP64 pipe the parts of one outlying group took 0.5 ms.
+constexpr int CB = 4, CL = 128;          // bodies and lanes per body of a block
+template <bool COUNT>
+__global__ void __launch_bounds__(CB * CL) k_walk_combine(WalkArgs g)
+{
+    __shared__ float2 sum[CB][4][CL];
+    __shared__ int2 num[CB][COUNT ? CL : 1];
+    __shared__ double res[CB][4];
+    const int body = threadIdx.x % CB, part = threadIdx.x / CB;
+    const int nwork = g.sp.ctl->ngroup * (HC_GROUP2 / CB);
+    for (int i = blockIdx.x; i < nwork; i += gridDim.x) {
+        const hc_walk_parts P = g.sp.group[i / (HC_GROUP2 / CB)];
+        const int b0 = i % (HC_GROUP2 / CB) * CB, b = b0 + body;
+        if (b0 >= P.cnt) continue;
+        float2 a[4] = {};                        // (sum, error) of x, y, z, phi
+        int2 c = make_int2(0, 0);
+        auto add = [&](int slot) {
+            const int64_t q = (int64_t)slot * HC_GROUP2 + b;
+            const float4 p = g.sp.part[2 * q], e = g.sp.part[2 * q + 1];
+            const float ps[4] = {p.x, p.y, p.z, p.w}, es[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float t = __fadd_rn(a[k].x, ps[k]), u = __fsub_rn(t, a[k].x);
+                const float r = __fadd_rn(__fsub_rn(a[k].x, __fsub_rn(t, u)), __fsub_rn(ps[k], u));
+                a[k].x = t;
+                a[k].y = __fadd_rn(a[k].y, __fsub_rn(r, es[k]));
+            }
+            if (COUNT) {
+                c.x += g.sp.part_cnt[q].x;
+                c.y += g.sp.part_cnt[q].y;
+            }
+        };
+        if (b < P.cnt) {
+            if (part == CL - 1) add(P.own);
+            for (int t = part; t < P.n; t += CL) {
+                add(P.first + t);
+                const int2 sub = g.sp.sub[P.first + t];
+#pragma unroll 4
+                for (int u = 0; u < sub.y; u++) add(sub.x + u);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) sum[body][k][part] = a[k];
+        if (COUNT) num[body][part] = c;
+        __syncthreads();
+        // one warp per (body, quantity)
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double r = 0.0;
+#pragma unroll
+        for (int v = 0; v < CL / 32; v++) {
+            const float2 q = sum[w >> 2][w & 3][lane + 32 * v];
+            r += (double)q.x + (double)q.y;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
+        if (lane == 0) res[w >> 2][w & 3] = r;
+        __syncthreads();
+        if (threadIdx.x < CB && b < P.cnt) {
+            const double *f = res[body];
+            const uint32_t o = g.tsorted[P.s0 + b];
+            if (g.kick_dthf != 0.0 && g.nstep > 0) {
+                g.vx[o] = __dadd_rn(g.vx[o], __dmul_rn(__dsub_rn(f[0], g.oax[o]), g.kick_dthf));
+                g.vy[o] = __dadd_rn(g.vy[o], __dmul_rn(__dsub_rn(f[1], g.oay[o]), g.kick_dthf));
+                g.vz[o] = __dadd_rn(g.vz[o], __dmul_rn(__dsub_rn(f[2], g.oaz[o]), g.kick_dthf));
+            }
+            g.oax[o] = f[0];
+            g.oay[o] = f[1];
+            g.oaz[o] = f[2];
+            g.ophi[o] = f[3];
+            if (COUNT) {
+                for (int v = 1; v < CL; v++) {
+                    c.x += num[body][v].x;
+                    c.y += num[body][v].y;
+                }
+                g.cnt_b[o] = c.x;
+                g.cnt_c[o] = c.y;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 template <bool Q, bool C, int M, bool L = false>
 int configure(hc_ctx *c, int variant)
 {
     const size_t smem = walk_smem(M, C);
     HC_CUDA(cudaFuncSetAttribute(k_walk<Q, C, M, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if constexpr (M != 0 && !L)
+        HC_CUDA(cudaFuncSetAttribute(k_walk<Q, C, M, L, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int dev = 0, nsm = 0, per_sm = 0;
     HC_CUDA(cudaGetDevice(&dev));
     HC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1004,12 +1254,23 @@ template <bool Q, bool C, int M, bool L = false>
 int launch(hc_ctx *c, WalkArgs &a, int variant)
 {
     const size_t smem = walk_smem(M, C);
-    int64_t blocks = c->walk_blocks[variant];               // persistent: groups are fetched dynamically
-    int64_t need = ((a.ntarget + 31) / 32 + WARPS - 1) / WARPS;
+    const int64_t full = c->walk_blocks[variant];           // persistent: groups and tasks are fetched dynamically
+    int64_t blocks = full;
+    const int64_t need = ((a.ntarget + 31) / 32 + WARPS - 1) / WARPS;
     if (!a.use_table && blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
+    a.warps = (int)(full * WARPS);
+    a.phase = 0;
     k_walk<Q, C, M, L><<<(unsigned)blocks, WARPS * 32, smem, c->stream>>>(a);
     c->launches++;
+    if constexpr (M != 0 && !L) {
+        for (a.phase = 1; a.phase < 4; a.phase++) {
+            k_walk<Q, C, M, L, true><<<(unsigned)full, WARPS * 32, smem, c->stream>>>(a);
+            c->launches++;
+        }
+        k_walk_combine<C><<<(unsigned)full, CB * CL, 0, c->stream>>>(a);
+        c->launches++;
+    }
     return HC_OK;
 }
 
@@ -1058,7 +1319,7 @@ int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorte
     a.vy = c->vy;
     a.vz = c->vz;
     a.st = c->st;
-    a.group_counter = (unsigned *)(c->st + 1);
+    a.sp = c->split;
     a.pax = c->ax;
     a.pay = c->ay;
     a.paz = c->az;
@@ -1069,10 +1330,18 @@ int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorte
     // criterion), else 32 consecutive bodies (also the guard's fallback walk)
     const bool per_body = body_rule || c->criterion == HC_CRITERION_BODY;
     a.use_table = (self && (!per_body || (c->criterion == HC_CRITERION_BODY && c->group_kind == 1))) ? 1 : 0;
-    HC_CUDA(cudaMemsetAsync(a.group_counter, 0, sizeof(unsigned), c->stream));
+    HC_CUDA(cudaMemsetAsync(a.sp.ctl, 0, sizeof(hc_walk_ctl), c->stream));
     const bool count = c->prm.count_per_body && self && c->cnt_b;
     const int v = (c->prm.usequad ? 2 : 0) + (count ? 1 : 0);
     a.eps_acc = (float)c->group_theta;
+    {
+        // how long a group's walk is expected to be, relative to theta = 0.5
+        // (cells opened ~ theta^-3) or an error budget of 0.05 (~ budget^-3/5)
+        const bool budgeted = !per_body && (c->criterion == HC_CRITERION_ERROR || c->criterion == HC_CRITERION_LEARNED);
+        const double th = per_body ? c->prm.tol : c->group_theta;
+        const double f = budgeted ? pow(0.05 / std::max(th, 1e-9), 0.6) : pow(0.5 / std::max(fabs(th), 1e-3), 3.0);
+        a.split_scale = (float)std::min(std::max(f, 1.0), 1e6);
+    }
     const bool rc = c->criterion == HC_CRITERION_BH86 || c->criterion == HC_CRITERION_SW94 ||
                     c->criterion == HC_CRITERION_BARNES;
     if (!body_rule && (c->criterion == HC_CRITERION_GROUP || rc)) {
