@@ -63,13 +63,10 @@ int check_status(hc_ctx *c)
 void free_all(hc_ctx *c)
 {
     void *ptrs[] = {c->mass, c->px, c->py, c->pz, c->vx, c->vy, c->vz, c->ax, c->ay, c->az, c->phi, c->cnt_b,
-                    c->cnt_c, c->khi[0], c->khi[1], c->klo[0], c->klo[1], c->kval[0], c->kval[1], c->s_rank,
-                    c->leaf_of_sorted, c->tord, c->gstart, c->gcount, c->gcnt, c->goff, c->mhi, c->mlo, c->midx, c->mpos, c->dlcp, c->ccount, c->pre_info, c->pre_a, c->bfs_a,
-                    c->dkey[0], c->dkey[1], c->dval[0], c->dval[1], c->pre2bfs, c->parent, c->lastc, c->cperm, c->cbins,
-                    c->nodeA, c->nodeB, c->nodeQ, c->nodeC, c->nm, c->ncx, c->ncy, c->ncz, c->flags,
-                    c->scan_tmp, c->hist, c->cand, c->ncand, c->diag_part, c->st, c->box, c->tx, c->ty, c->tz,
-                    c->tax, c->tay, c->taz, c->tphi, c->tkhi[0], c->tkhi[1], c->tklo[0], c->tklo[1],
-                    c->tkval[0], c->tkval[1], c->thist};
+                    c->cnt_c, c->khi[0], c->khi[1], c->klo, c->kval[0], c->kval[1], c->body, c->gstart, c->gcount,
+                    c->bfs_a, c->bfs_link, c->bfs_d, c->cperm, c->nodeAB, c->nodeQ, c->nodeC, c->nodeD,
+                    c->hist, c->first2, c->cand, c->ncand, c->diag_part, c->st, c->box, c->tx, c->ty, c->tz,
+                    c->tax, c->tay, c->taz, c->tphi, c->tkhi[0], c->tkhi[1], c->tkval[0], c->tkval[1], c->thist};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     void *mptrs[] = {c->mlp_p, c->mlp_m, c->mlp_v, c->mlp_grad, c->mlp_loss, c->mlp_gpart, c->mlp_lpart,
@@ -99,47 +96,23 @@ int alloc_all(hc_ctx *c)
     HC_TRY(dalloc(c, &c->cnt_c, n));
     for (int i = 0; i < 2; i++) {
         HC_TRY(dalloc(c, &c->khi[i], n));
-        HC_TRY(dalloc(c, &c->klo[i], n));
         HC_TRY(dalloc(c, &c->kval[i], n));
     }
-    HC_TRY(dalloc(c, &c->s_rank, n));
-    HC_TRY(dalloc(c, &c->tord, n));
+    HC_TRY(dalloc(c, &c->klo, n));
+    HC_TRY(dalloc(c, &c->body, n));
     HC_TRY(dalloc(c, &c->gstart, n));
     HC_TRY(dalloc(c, &c->gcount, n));
-    HC_TRY(dalloc(c, &c->leaf_of_sorted, n));
-    HC_TRY(dalloc(c, &c->mhi, n));
-    HC_TRY(dalloc(c, &c->mlo, n));
-    HC_TRY(dalloc(c, &c->midx, n));
-    HC_TRY(dalloc(c, &c->mpos, n));
-    HC_TRY(dalloc(c, &c->dlcp, n));
-    HC_TRY(dalloc(c, &c->ccount, n + 1));
     const int64_t mn = c->maxnode;
-    HC_TRY(dalloc(c, &c->pre_info, mn));
-    HC_TRY(dalloc(c, &c->pre_a, mn));
     HC_TRY(dalloc(c, &c->bfs_a, mn));
-    for (int i = 0; i < 2; i++) {
-        HC_TRY(dalloc(c, &c->dkey[i], mn));
-        HC_TRY(dalloc(c, &c->dval[i], mn));
-    }
-    HC_TRY(dalloc(c, &c->pre2bfs, mn));
-    HC_TRY(dalloc(c, &c->parent, mn));
-    HC_TRY(dalloc(c, &c->lastc, mn));
+    HC_TRY(dalloc(c, &c->bfs_link, mn));
+    HC_TRY(dalloc(c, &c->bfs_d, mn));
     HC_TRY(dalloc(c, &c->cperm, mn));
-    HC_TRY(dalloc(c, &c->cbins, 520));
-    HC_TRY(dalloc(c, &c->gcnt, mn + 1));
-    HC_TRY(dalloc(c, &c->goff, mn + 1));
-    HC_TRY(dalloc(c, &c->nodeA, mn));
-    HC_TRY(dalloc(c, &c->nodeB, mn));
+    HC_TRY(dalloc(c, &c->nodeAB, 2 * mn));
     HC_TRY(dalloc(c, &c->nodeQ, 2 * mn));
     HC_TRY(dalloc(c, &c->nodeC, mn));
-    HC_TRY(dalloc(c, &c->nm, mn));
-    HC_TRY(dalloc(c, &c->ncx, mn));
-    HC_TRY(dalloc(c, &c->ncy, mn));
-    HC_TRY(dalloc(c, &c->ncz, mn));
-    HC_TRY(dalloc(c, &c->flags, 4 * n + 8));
-    const int64_t big = std::max<int64_t>(n, mn);
-    HC_TRY(dalloc(c, &c->scan_tmp, hc_scan_scratch_words(big + 1)));
-    HC_TRY(dalloc(c, &c->hist, hc_sort_scratch_words(big)));
+    HC_TRY(dalloc(c, &c->nodeD, mn));
+    HC_TRY(dalloc(c, &c->hist, hc_build_scratch_words(n, mn)));
+    HC_TRY(dalloc(c, &c->first2, (n + 4095) / 4096));
     HC_TRY(dalloc(c, &c->cand, n));
     HC_TRY(dalloc(c, &c->ncand, 4));
     HC_TRY(dalloc(c, &c->diag_part, 36 * 1024));
@@ -197,7 +170,7 @@ int ensure_test_capacity(hc_ctx *c, int64_t nt)
     c->tcap = 0;
     void **ptrs[] = {(void **)&c->tx, (void **)&c->ty, (void **)&c->tz, (void **)&c->tax, (void **)&c->tay,
                      (void **)&c->taz, (void **)&c->tphi, (void **)&c->tkhi[0], (void **)&c->tkhi[1],
-                     (void **)&c->tklo[0], (void **)&c->tklo[1], (void **)&c->tkval[0], (void **)&c->tkval[1],
+                     (void **)&c->tkval[0], (void **)&c->tkval[1],
                      (void **)&c->thist};
     for (void **p : ptrs) {
         if (*p) cudaFree(*p);
@@ -207,7 +180,6 @@ int ensure_test_capacity(hc_ctx *c, int64_t nt)
     for (double **p : dd) HC_TRY(dalloc(c, p, nt));
     for (int i = 0; i < 2; i++) {
         HC_TRY(dalloc(c, &c->tkhi[i], nt));
-        HC_TRY(dalloc(c, &c->tklo[i], nt));
         HC_TRY(dalloc(c, &c->tkval[i], nt));
     }
     HC_TRY(dalloc(c, &c->thist, hc_sort_scratch_words(nt)));
@@ -230,6 +202,14 @@ __global__ void k_unpack_phase(const double *phase, int64_t n, double *px, doubl
         vy[i] = q[4];
         vz[i] = q[5];
     }
+}
+
+__global__ void k_massless(const double *mass, int64_t n, int *any)
+{
+    bool z = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        z = z || !hc_nonzero(mass[i]);
+    if (__syncthreads_or(z) && threadIdx.x == 0) *any = 1;
 }
 
 __global__ void k_pack3(const double *x, const double *y, const double *z, int64_t n, double *out, int stride,
@@ -393,6 +373,27 @@ int hc_set_params(hc_ctx *c, const hc_params *p)
     return HC_OK;
 }
 
+// Synchronises the stream and notes whether every body has mass: the build
+// then takes the sorted bodies as they are, without a compaction.
+extern "C++" int hc_note_masses(hc_ctx *c)
+{
+    int *any = c->ncand + 1, *h_any = reinterpret_cast<int *>(c->h_box);
+    HC_CUDA(cudaMemsetAsync(any, 0, sizeof(int), c->stream));
+    k_massless<<<hc_grid(c->n, 256, 152 * 4), 256, 0, c->stream>>>(c->mass, c->n, any);
+    HC_CUDA(cudaMemcpyAsync(h_any, any, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    HC_CUDA(cudaStreamSynchronize(c->stream));
+    HC_CUDA(cudaGetLastError());
+    if (c->all_massive != (*h_any == 0)) {
+        c->all_massive = *h_any == 0;
+        for (auto &g : static_cast<hc_ctx_ext *>(c)->graphs)   // captured graphs bake the build's form
+            if (g.exec) {
+                cudaGraphExecDestroy(g.exec);
+                g.exec = nullptr;
+            }
+    }
+    return HC_OK;
+}
+
 int hc_upload(hc_ctx *ctx, const double *mass, const double *phase)
 {
     if (!ctx || !mass || !phase) return HC_ERR_ARG;
@@ -406,8 +407,7 @@ int hc_upload(hc_ctx *ctx, const double *mass, const double *phase)
     HC_CUDA(cudaMemsetAsync(c->ay, 0, sizeof(double) * n, c->stream));
     HC_CUDA(cudaMemsetAsync(c->az, 0, sizeof(double) * n, c->stream));
     HC_CUDA(cudaMemsetAsync(c->phi, 0, sizeof(double) * n, c->stream));
-    HC_CUDA(cudaStreamSynchronize(c->stream));
-    HC_CUDA(cudaGetLastError());
+    HC_TRY(hc_note_masses(c));
     c->have_tree = c->have_forces = false;
     return HC_OK;
 }
@@ -559,8 +559,9 @@ int hc_forces_at(hc_ctx *ctx, const double *test_pos, int64_t ntest, double *acc
     reset_status(c);
     HC_CUDA(cudaMemcpyAsync(c->stage.d, test_pos, sizeof(double) * 3 * ntest, cudaMemcpyHostToDevice, c->stream));
     k_unpack3<<<hc_grid(ntest, 256), 256, 0, c->stream>>>(c->stage.d, ntest, c->tx, c->ty, c->tz);
-    hc_keys_for_points(c, c->tx, c->ty, c->tz, ntest, c->tkhi[0], c->tklo[0], c->tkval[0]);
-    int sel = hc_radix_sort_keys(c, c->thist, c->tkhi, c->tklo, c->tkval, ntest, 0, 64, false);
+    HC_CUDA(cudaMemsetAsync(c->thist, 0, sizeof(uint32_t) * hc_sort_scratch_words(ntest), c->stream));
+    hc_keys_for_points(c, c->tx, c->ty, c->tz, ntest, c->tkhi[0], nullptr, nullptr, c->thist);
+    int sel = hc_radix_sort_keys(c, c->thist, c->tkhi, c->tkval, ntest, nullptr);
     HC_CUDA(cudaEventRecord(c->ev[2], c->stream));
     HC_TRY(hc_walk_launch(c, false, ntest, c->tkval[sel], c->tx, c->ty, c->tz, c->tax, c->tay, c->taz, c->tphi,
                           0.0, 0));
@@ -742,6 +743,10 @@ static int launch_evaluation(hc_ctx_ext *c, int slot, double kick_dthf, int64_t 
     }
     HC_CUDA(cudaGraphLaunch(g.exec, c->stream));
     c->launches = g.launches;
+    // what the replayed build makes (its configuration is the current one: every
+    // change drops the graphs)
+    c->table_gmax = hc_table_gmax(c);
+    c->have_groups = hc_build_makes_groups(c);
     return HC_OK;
 }
 

@@ -180,15 +180,15 @@ __global__ void k_ens_translate(int64_t n_tree, const int32_t *body_sys, const S
 
 // 4. root cell of each tree system: the cell at the system's depth that
 // holds its first body in key order
-__global__ void k_ens_roots(const hc_box *fbox, const int32_t *pre_depth, const int32_t *pre_a, const uint32_t *midx,
-                            const uint32_t *pre2bfs, const int32_t *body_sys, const int32_t *depth, int32_t *root)
+__global__ void k_ens_roots(const hc_box *fbox, const int2 *nodeC, const uint32_t *bfs_a, const uint32_t *midx,
+                            const int32_t *body_sys, const int32_t *depth, int32_t *root)
 {
     const int nn = fbox->nnode;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nn; p += gridDim.x * blockDim.x) {
-        const int a = pre_a[p];
-        if (a < 0) continue;                          // a body
-        const int s = body_sys[midx[a]];
-        if (pre_depth[p] == depth[s]) root[s] = (int32_t)pre2bfs[p];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+        const int2 C = nodeC[k];
+        if (C.x < 0) continue;                        // a body
+        const int s = body_sys[midx[bfs_a[k]]];
+        if (C.y >> 8 == depth[s]) root[s] = k;
     }
 }
 
@@ -414,7 +414,7 @@ int ens_enqueue(hc_ens *e, double kick_dthf, int64_t nstep, double dt, bool capt
             e->err = c->err;
             return r;
         }
-        k_ens_roots<<<hc_grid(c->maxnode, 256), 256, 0, s>>>(c->box, c->pre_info, c->pre_a, c->midx, c->pre2bfs,
+        k_ens_roots<<<hc_grid(c->maxnode, 256), 256, 0, s>>>(c->box, c->nodeC, c->bfs_a, c->xidx,
                                                              e->d_body_sys, e->d_depth, e->d_root);
         r = hc_walk_launch(c, true, c->n, c->tord, c->px, c->py, c->pz, c->ax, c->ay, c->az, c->phi, kick_dthf,
                            nstep);
@@ -544,6 +544,7 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
             *mine[k] = ens[k];
         }
         c->group_kind = HC_GROUPS_TREE;      // groups must not straddle systems
+        c->all_massive = true;               // hc_ens_upload takes no others
         c->walk_sys_root = e->d_root;
         c->walk_body_sys = e->d_body_sys;
         e->stream = c->stream;

@@ -305,7 +305,7 @@ extern "C" int hc_generate(hc_ctx *c, const char *model, uint64_t seed, const do
     }
     int nf = 0;
     HC_CUDA(cudaMemcpyAsync(&nf, fails, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    HC_CUDA(cudaStreamSynchronize(c->stream));
+    if (int r = hc_note_masses(c)) return r;
     HC_CUDA(cudaGetLastError());
     if (r != HC_OK) {
         if (c->err.empty()) c->err = "hc_generate: bad parameters for '" + nm + "'";

@@ -6,10 +6,10 @@
 //     interleaved, x most significant) + 27-bit low key + original index
 //   tree nodes (bodies and cells) in breadth-first order, children of a
 //     cell contiguous and in subindex order 0..7 (load.c:162-177):
-//       nodeA float4 (cm_hi.xyz, mass)   nodeB float4 (cm_lo.xyz, size^2)
+//       nodeAB 2 x float4 (cm_hi.xyz, mass | cm_lo.xyz, size^2)
 //       nodeC int2   (first child | -1-body slot, nchild | depth<<8)
 //       nodeQ 2 x float4 (Qxx Qxy Qxz Qyy | Qyz Qzz 0 0)
-//       FP64 mass / cm / quad per node for the upward pass and for exact
+//       nodeD 4 x double (cm.xyz, mass) for the upward pass and for exact
 //       re-evaluation of borderline opening decisions.
 #pragma once
 #include <cuda_runtime.h>
@@ -113,41 +113,33 @@ struct hc_ctx {
     double *mass, *px, *py, *pz, *vx, *vy, *vz, *ax, *ay, *az, *phi;
     int32_t *cnt_b, *cnt_c;   // per-body counts (optional)
 
-    // keys and sort (n entries, double-buffered)
+    // keys and sort (n entries; the low keys stay in body order)
     unsigned long long *khi[2];
-    uint32_t *klo[2];
+    uint32_t *klo;
     uint32_t *kval[2];
-    int sort_sel;             // which buffer holds the sorted result
-    uint32_t *sidx;           // sorted position -> original index (all bodies)
-    int32_t *s_rank;          // sorted position -> massive rank or -1
-    int32_t *leaf_of_sorted;  // sorted position -> BFS node of its leaf or -1
-    uint32_t *tord;           // walk target order: massive in key order, then massless
-    int32_t *gcnt, *goff;     // groups per node, their offsets (maxnode + 1)
+    double4_32a *body;        // bodies' (x, y, z, mass), body order
     int32_t *gstart, *gcount; // tree-aligned groups: first massive rank, count
     int group_kind;           // 0: 32 consecutive bodies, 1: tree-aligned groups
+    int table_gmax;           // largest tree-aligned group of the current tree
+    bool have_groups;         // the current tree has its group table
+    bool all_massive;         // every body of the last upload has mass
 
-    // massive bodies in key order
-    unsigned long long *mhi;
-    uint32_t *mlo;
-    uint32_t *midx;           // massive rank -> original index
-    uint32_t *mpos;           // massive rank -> sorted position
-    int32_t *dlcp;            // lcp in octal digits of adjacent massive keys
-    int32_t *ccount;          // cells starting at each massive rank (scan -> offsets)
+    // massive bodies in key order: views of the sort's buffers, set by the build
+    const unsigned long long *xhi;   // high keys
+    const uint32_t *xidx;     // massive rank -> original index
+    const uint32_t *tord;     // walk target order: massive in key order, then massless
 
     // nodes
     int64_t maxnode;
-    int32_t *pre_info;        // pre-order: level (cell) or -1 (body); bit 31 unused
-    int32_t *pre_a;           // pre-order: massive rank of first body
-    uint32_t *bfs_a;          // breadth-first order: pre_a of each node (the depth sort's payload)
-    unsigned long long *dkey[2]; // depth sort keys
-    uint32_t *dval[2];
-    uint32_t *bfs2pre, *pre2bfs;
-    int32_t *parent, *lastc;
+    // breadth-first order: first massive body (-1 - rank for a leaf), start of
+    // the children (or where they would be), depth
+    uint32_t *bfs_a;
+    int32_t *bfs_link;
+    uint8_t *bfs_d;
     int4 *cperm;              // upward pass: cells (index, first child, nodeC.y) grouped by depth, then child count
-    uint32_t *cbins;          // their group offsets [257] and placement cursors [256]
-    float4 *nodeA, *nodeB, *nodeQ;
+    float4 *nodeAB, *nodeQ;
     int2 *nodeC;
-    double *nm, *ncx, *ncy, *ncz;         // FP64 mass and centre of mass per node
+    double4_32a *nodeD;
     int cofm_grid;                        // co-resident blocks of the upward-pass kernel
     int walk_blocks[20];                  // resident blocks of each walk variant
     hc_walk_split split;                  // buffers of split walks
@@ -190,9 +182,8 @@ struct hc_ctx {
     double group_theta;                   // opening angle of the group criterion
 
     // scratch
-    int32_t *flags;           // n
-    uint32_t *scan_tmp;       // single-pass scan: tile counter and look-back words
-    uint32_t *hist;           // radix histograms
+    uint32_t *hist;           // sort and build: digit counts, tile counters, look-back words
+    int2 *first2;             // per tile of the box test: its first two massive bodies
     int32_t *cand;            // expandbox candidates (original indices)
     int32_t *ncand;
     double *diag_part;        // per-block diagnostics partials
@@ -205,28 +196,32 @@ struct hc_ctx {
     int64_t tcap;
     double *tx, *ty, *tz, *tax, *tay, *taz, *tphi;
     unsigned long long *tkhi[2];
-    uint32_t *tklo[2], *tkval[2];
+    uint32_t *tkval[2];
     uint32_t *thist;          // their radix sort's scratch (hist is baked into captured graphs)
 };
 
 // ---- host-side launchers implemented in the .cu files ----
-// scan / sort (hc_sort.cu)
-void hc_scan_exclusive_i32(hc_ctx *c, const int32_t *in, int32_t *out, int64_t n, int32_t *total_dev);
-int64_t hc_scan_scratch_words(int64_t n);
+// sort (hc_sort.cu)
 // 32-bit words of sort scratch for sorting n keys (n < 2^30)
 int64_t hc_sort_scratch_words(int64_t n);
 int hc_sort_setup(hc_ctx *c);
-// scratch: hc_sort_scratch_words(n) words (c->hist for the tree, c->thist for test points)
-int hc_radix_sort_keys(hc_ctx *c, uint32_t *scratch, unsigned long long *khi[2], uint32_t *klo[2],
-                       uint32_t *kval[2], int64_t n, int begin_bit, int end_bit, bool tie_fix,
-                       const int *n_dev = nullptr);
+// true: the sort of n keys needs no scratch and no digit counts
+bool hc_sort_counts_digits(int64_t n);
+// scratch: hc_sort_scratch_words(n) words, zeroed, then filled by hc_keys_for_points
+int hc_radix_sort_keys(hc_ctx *c, uint32_t *scratch, unsigned long long *khi[2], uint32_t *kval[2], int64_t n,
+                       const uint32_t *lo);
 // tree (hc_tree.cu)
 int hc_tree_build(hc_ctx *c);
 int hc_tree_setup(hc_ctx *c);
+int64_t hc_build_scratch_words(int64_t n, int64_t maxnode);
+bool hc_build_makes_groups(const hc_ctx *c);
+void hc_groups_launch(hc_ctx *c);
 int hc_tree_dump_impl(hc_ctx *c, int32_t *level, int32_t *corner, int32_t *count, double *mass,
                       double *cm, double *quad, int32_t *bparent);
 void hc_keys_for_points(hc_ctx *c, const double *x, const double *y, const double *z, int64_t n,
-                        unsigned long long *khi, uint32_t *klo, uint32_t *kval);
+                        unsigned long long *khi, uint32_t *klo, double4_32a *body, uint32_t *scratch);
+// synchronises and notes whether every body has mass (hc_api.cu)
+int hc_note_masses(hc_ctx *c);
 // walk (hc_walk.cu)
 int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorted,
                    const double *tx, const double *ty, const double *tz, double *oax, double *oay,

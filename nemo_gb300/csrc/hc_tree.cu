@@ -13,12 +13,16 @@
 //
 //   1. expandbox replay on the device (one block, FP64, body order),
 //   2. 90-bit keys: floor(2^30 (x - rmin) / rsize) per axis, Morton order,
-//   3. radix sort, compaction of the massive bodies,
+//   3. radix sort; compaction of the massive bodies where there are massless ones,
 //   4. d[a] = common octal digits of adjacent keys; cells starting at sorted
-//      body a have levels (d[a-1], d[a]], which lays cells and bodies out in
-//      DFS pre-order directly,
-//   5. stable sort of the pre-order by depth -> breadth-first layout with the
-//      children of each cell contiguous and in subindex order 0..7,
+//      body a have levels (d[a-1], d[a]]: the bodies in key order, each after
+//      the cells that start at it, are the nodes in DFS pre-order.  One pass
+//      counts the nodes of every depth; a second gives each node its
+//      breadth-first place (nodes of its depth before it in pre-order) and its
+//      first child's place (the nodes one deeper before it), so that the
+//      children of each cell are contiguous and in subindex order 0..7 and no
+//      node has to search for its parent or children,
+//   5. node records, cells grouped by depth and child count,
 //   6. level-synchronous upward pass (one cooperative kernel, a grid barrier
 //      per level): mass and centre of mass in FP64, children summed in the
 //      same order as hackcofm so they are bit-identical (they decide cell
@@ -26,7 +30,7 @@
 //      accumulated in FP32 from FP64 offsets.
 #include <cooperative_groups.h>
 #include <memory>
-#include "hc_internal.cuh"
+#include "hc_scan.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -97,66 +101,94 @@ __device__ __forceinline__ int2 warp_min2(int2 v)
     return v;
 }
 
-// Whether a massive body lies outside the box (intcoord's test,
-// load.c:135-156), and each block's first two massive bodies in body order
-// (the expansion replay needs the first two of all).  A body clearly inside
-// by an FP32 estimate with a margin far above its error skips the exact FP64
-// test (the FP64 pipe runs at a small fraction of the FP32 rate); the rest
-// take it.
-__global__ void __launch_bounds__(256) k_box_flags(const double *mass, const double *px, const double *py,
-                                                   const double *pz, int64_t n, const hc_box *box, int32_t *outside,
-                                                   int2 *first2)
+// The massive bodies outside the box (intcoord's test, load.c:135-156), in body
+// order, and each tile's first two massive bodies (the expansion replay needs
+// the first two of all).  A body clearly inside by an FP32 estimate with a
+// margin far above its error skips the exact FP64 test (the FP64 pipe runs at a
+// small fraction of the FP32 rate); the rest take it.  One pass: a tile's place
+// in the list comes from decoupled look-back (as three kernels -- flags, scan,
+// compaction -- this took 21 + 13 + 5 us at N = 2^20 and two more launches).
+constexpr int BOX_ITEMS = 16, BOX_TILE = 256 * BOX_ITEMS;
+__global__ void __launch_bounds__(256) k_box_outside(const double *mass, const double *px, const double *py,
+                                                     const double *pz, int64_t n, const hc_box *box, int32_t *cand,
+                                                     int32_t *ncand, int2 *first2, uint32_t *status, uint32_t *ctr,
+                                                     int *err)
 {
     __shared__ int2 wf[8];
+    __shared__ uint32_t wsum[8], s_tile, s_prefix;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ctr, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile, base = tile * BOX_TILE + wid * (BOX_TILE / 8);
     double rmin[3] = {box->rmin[0], box->rmin[1], box->rmin[2]};
     double rsize = box->rsize;
     const float lo[3] = {hc_d2f_rn(rmin[0]), hc_d2f_rn(rmin[1]), hc_d2f_rn(rmin[2])}, sz = hc_d2f_rn(rsize);
     int2 f2 = make_int2(INT_MAX, INT_MAX);     // this thread's first two massive bodies (ascending i)
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const bool m = hc_nonzero(mass[i]);
-        if (m && f2.y == INT_MAX) {
-            if (f2.x == INT_MAX) f2.x = (int)i;
-            else f2.y = (int)i;
-        }
-        const double x[3] = {px[i], py[i], pz[i]};
-        bool clear = true;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            float f;
-            if (!approx_f32(x[k], &f)) {
-                clear = false;
-                continue;
+    uint32_t out = 0, cnt = 0;                 // rounds in which this lane's body is outside; the warp's number
+#pragma unroll 4
+    for (int r = 0; r < BOX_ITEMS; r++) {
+        const int64_t i = base + r * 32 + lane;
+        bool o = false;
+        if (i < n) {
+            const bool m = hc_nonzero(mass[i]);
+            if (m && f2.y == INT_MAX) {
+                if (f2.x == INT_MAX) f2.x = (int)i;
+                else f2.y = (int)i;
             }
-            const float u = f - lo[k], margin = 0x1p-16f * sz + 0x1p-18f * fabsf(f);
-            clear = clear && u >= margin && u <= sz - margin;
+            const double x[3] = {px[i], py[i], pz[i]};
+            bool clear = true;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                float f;
+                if (!approx_f32(x[k], &f)) {
+                    clear = false;
+                    continue;
+                }
+                const float u = f - lo[k], margin = 0x1p-16f * sz + 0x1p-18f * fabsf(f);
+                clear = clear && u >= margin && u <= sz - margin;
+            }
+            o = m && !(clear || inbox(x[0], x[1], x[2], rmin, rsize));
         }
-        outside[i] = m && !(clear || inbox(x[0], x[1], x[2], rmin, rsize));
+        cnt += __popc(__ballot_sync(0xffffffffu, o));
+        out |= (uint32_t)o << r;
     }
     f2 = warp_min2(f2);
-    if ((threadIdx.x & 31) == 0) wf[threadIdx.x >> 5] = f2;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) f2 = min2(f2, wf[w]);
-        first2[blockIdx.x] = f2;
+    if (lane == 0) {
+        wf[wid] = f2;
+        wsum[wid] = cnt;
     }
-}
-
-__global__ void k_box_compact(const int32_t *outside, const int32_t *opos, int64_t n, int32_t *cand)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        if (outside[i]) cand[opos[i]] = (int32_t)i;
+    __syncthreads();
+    if (wid == 0) {
+        const uint32_t agg = __reduce_add_sync(0xffffffffu, lane < 8 ? wsum[lane] : 0u);
+        const uint32_t prefix = tile_prefix(status, tile, agg, err);
+        if (lane == 0) {
+            s_prefix = prefix;
+            if ((tile + 1) * BOX_TILE >= n) *ncand = (int32_t)(prefix + agg);     // the last tile
+            for (int w = 1; w < 8; w++) f2 = min2(f2, wf[w]);
+            first2[tile] = f2;
+        }
+    }
+    __syncthreads();
+    if (cnt == 0) return;                      // the whole warp
+    uint32_t pos = s_prefix;
+    for (int w = 0; w < wid; w++) pos += wsum[w];
+    for (int r = 0; r < BOX_ITEMS; r++) {
+        const unsigned b = __ballot_sync(0xffffffffu, (out >> r) & 1u);
+        if ((out >> r) & 1u) cand[pos + __popc(b & ((1u << lane) - 1u))] = (int32_t)(base + r * 32 + lane);
+        pos += __popc(b);
+    }
 }
 
 // One block replays expandbox over the bodies that were outside the box at
 // the start, in body order.  The box only grows, so a body inside stays
 // inside; each round finds the first remaining body outside, expands for
 // it, and continues after it.
-// The first two massive bodies come from k_box_flags' per-block pairs: the
+// The first two massive bodies come from k_box_outside's per-tile pairs: the
 // first one (original order) is where the expansion-chain cells hang, the
 // second is the body whose insertion may graft them.
 __global__ void __launch_bounds__(256) k_box_replay(const double *px, const double *py, const double *pz,
                                                     const int32_t *cand, const int32_t *ncand_p, const int2 *first2,
-                                                    int nblk, hc_box *box, hc_status *st)
+                                                    int nblk, hc_box *box, hc_status *st, int nmassive)
 {
     __shared__ int first;
     __shared__ double rmin[3], rsize;
@@ -173,6 +205,7 @@ __global__ void __launch_bounds__(256) k_box_replay(const double *px, const doub
         if (threadIdx.x == 0) {
             for (int w = 1; w < (int)(blockDim.x >> 5); w++) f2 = min2(f2, wf[w]);
             box->first_massive = f2.x == INT_MAX ? -1 : f2.x;
+            if (nmassive >= 0) box->nmassive = nmassive;       // every body has mass
             second_massive = f2.y == INT_MAX ? -1 : f2.y;
         }
     }
@@ -305,312 +338,368 @@ __device__ __forceinline__ int intcoord_pow2(double x, double rmin, int E)
     return s >= 64 ? 0 : (int)(sig >> s);
 }
 
-__global__ void k_keys(const double *x, const double *y, const double *z, int64_t n, const hc_box *box,
-                       unsigned long long *khi, uint32_t *klo, uint32_t *kval)
+// Keys of the bodies (or test points), the digit counts of the sort's eight
+// passes (counts: [8][256], null for the small sort), and with body the bodies'
+// positions and masses as one 32-byte record each: the leaf records gather one
+// sector per body from it instead of four.
+__global__ void __launch_bounds__(256) k_keys(const double *x, const double *y, const double *z, const double *mass,
+                                              int64_t n, const hc_box *box, unsigned long long *khi, uint32_t *klo,
+                                              double4_32a *body, uint32_t *counts)
 {
+    __shared__ uint32_t h[8][256];
+    if (counts) {
+        for (int p = 0; p < 8; p++) h[p][threadIdx.x] = 0;
+        __syncthreads();
+    }
     double r0 = box->rmin[0], r1 = box->rmin[1], r2 = box->rmin[2], rs = box->rsize;
     // rs = 2^E exactly when its significand bits are zero (a normal double)
     const uint64_t rb = hc_dbits(rs);
     const int ref = (int)((rb >> 52) & 0x7ff), E = ref - 1023;
     const bool pow2 = (rb & 0xfffffffffffffull) == 0 && ref > 0 && ref < 0x7ff && !(rb >> 63);
+#pragma unroll 2
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double xi = x[i], yi = y[i], zi = z[i];
         unsigned ix, iy, iz;
         if (pow2) {
-            ix = intcoord_pow2(x[i], r0, E);
-            iy = intcoord_pow2(y[i], r1, E);
-            iz = intcoord_pow2(z[i], r2, E);
+            ix = intcoord_pow2(xi, r0, E);
+            iy = intcoord_pow2(yi, r1, E);
+            iz = intcoord_pow2(zi, r2, E);
         } else {
-            ix = intcoord_clamped(x[i], r0, rs);
-            iy = intcoord_clamped(y[i], r1, rs);
-            iz = intcoord_clamped(z[i], r2, rs);
+            ix = intcoord_clamped(xi, r0, rs);
+            iy = intcoord_clamped(yi, r1, rs);
+            iz = intcoord_clamped(zi, r2, rs);
         }
-        khi[i] = (spread21(ix >> 9) << 2) | (spread21(iy >> 9) << 1) | spread21(iz >> 9);
-        klo[i] = (spread9(ix) << 2) | (spread9(iy) << 1) | spread9(iz);
-        kval[i] = (uint32_t)i;
+        const unsigned long long k = (spread21(ix >> 9) << 2) | (spread21(iy >> 9) << 1) | spread21(iz >> 9);
+        khi[i] = k;
+        if (klo) klo[i] = (spread9(ix) << 2) | (spread9(iy) << 1) | spread9(iz);
+        if (body) body[i] = make_double4_32a(xi, yi, zi, mass[i]);
+        if (counts)
+#pragma unroll
+            for (int p = 0; p < 8; p++) atomicAdd(&h[p][(k >> (8 * p)) & 255u], 1u);
+    }
+    if (counts) {
+        __syncthreads();
+        for (int p = 0; p < 8; p++)
+            if (h[p][threadIdx.x]) atomicAdd(&counts[p * 256 + threadIdx.x], h[p][threadIdx.x]);
     }
 }
 
 // ---------------- massive compaction and cell enumeration ----------------
 
-__global__ void k_sorted_massive(const uint32_t *sidx, const double *mass, int64_t n, int32_t *flag)
+// Massive bodies in key order (tree input) and the walk's target order: massive
+// bodies in key order, then massless ones in key order (their number is known
+// after the pass; k_target_tail appends them).  Only for systems that have
+// massless bodies: otherwise the sorted arrays are the massive ones.
+constexpr int MC_ITEMS = 8, MC_TILE = 256 * MC_ITEMS;
+__global__ void __launch_bounds__(256) k_massive(const uint32_t *sidx, const unsigned long long *khi, const double *mass,
+                                                 int64_t n, hc_box *box, unsigned long long *mhi, uint32_t *midx,
+                                                 uint32_t *massless, uint32_t *status, uint32_t *ctr, int *err)
 {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x)
-        flag[s] = hc_nonzero(mass[sidx[s]]);
-}
-
-// Massive bodies in key order (tree input) and the walk's target order:
-// massive bodies in key order, then massless ones in key order.
-__global__ void k_mcompact(const int32_t *flag, const int32_t *rank, int64_t n, const unsigned long long *khi,
-                           const uint32_t *klo, const uint32_t *sidx, const hc_box *box, unsigned long long *mhi,
-                           uint32_t *mlo, uint32_t *midx, uint32_t *mpos, int32_t *s_rank, int32_t *leaf_of_sorted,
-                           uint32_t *tord)
-{
-    const int M = box->nmassive;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-        leaf_of_sorted[s] = -1;
-        int r = rank[s];
-        if (flag[s]) {
-            mhi[r] = khi[s];
-            mlo[r] = klo[s];
-            midx[r] = sidx[s];
-            mpos[r] = (uint32_t)s;
-            s_rank[s] = r;
-            tord[r] = sidx[s];
-        } else {
-            s_rank[s] = -1;
-            tord[M + (s - r)] = sidx[s];
+    __shared__ uint32_t wsum[8], s_tile, s_prefix;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ctr, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile, base = tile * MC_TILE + wid * (MC_TILE / 8);
+    uint32_t idx[MC_ITEMS], bal[MC_ITEMS], cnt = 0;
+#pragma unroll
+    for (int r = 0; r < MC_ITEMS; r++) {
+        const int64_t s = base + r * 32 + lane;
+        idx[r] = s < n ? sidx[s] : 0u;
+        bal[r] = __ballot_sync(0xffffffffu, s < n && hc_nonzero(mass[idx[r]]));
+        cnt += __popc(bal[r]);
+    }
+    if (lane == 0) wsum[wid] = cnt;
+    __syncthreads();
+    if (wid == 0) {
+        const uint32_t agg = __reduce_add_sync(0xffffffffu, lane < 8 ? wsum[lane] : 0u);
+        const uint32_t prefix = tile_prefix(status, tile, agg, err);
+        if (lane == 0) {
+            s_prefix = prefix;
+            if ((tile + 1) * MC_TILE >= n) box->nmassive = (int)(prefix + agg);   // the last tile
         }
+    }
+    __syncthreads();
+    uint32_t rank = s_prefix;
+    for (int w = 0; w < wid; w++) rank += wsum[w];
+#pragma unroll
+    for (int r = 0; r < MC_ITEMS; r++) {
+        const int64_t s = base + r * 32 + lane;
+        const uint32_t mine = rank + __popc(bal[r] & ((1u << lane) - 1u));
+        if (s < n) {
+            if ((bal[r] >> lane) & 1u) {
+                mhi[mine] = khi[s];
+                midx[mine] = idx[r];
+            } else {
+                massless[s - mine] = idx[r];
+            }
+        }
+        rank += __popc(bal[r]);
     }
 }
 
-// common leading octal digits of two 90-bit keys (30 = identical)
-__device__ __forceinline__ int lcp_digits(unsigned long long ha, uint32_t la, unsigned long long hb, uint32_t lb)
+__global__ void k_target_tail(int64_t n, const hc_box *box, const uint32_t *massless, uint32_t *tord)
 {
-    unsigned long long x = ha ^ hb;
+    const int64_t M = box->nmassive;
+    for (int64_t i = M + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        tord[i] = massless[i - M];
+}
+
+// common leading octal digits of the keys of massive bodies a and b (30 =
+// identical); the low keys are in body order and only read where the high tie
+__device__ __forceinline__ int lcp_digits(unsigned long long ha, unsigned long long hb, const uint32_t *klo,
+                                          const uint32_t *midx, int a, int b)
+{
+    const unsigned long long x = ha ^ hb;
     if (x) return (__clzll(x) - 1) / 3;
-    uint32_t y = la ^ lb;
+    const uint32_t y = klo[midx[a]] ^ klo[midx[b]];
     if (y) return 21 + (__clz(y) - 5) / 3;
     return 30;
 }
 
-__device__ __forceinline__ int dprime(const int32_t *d, const uint32_t *midx, int a, const hc_box *box)
+// Levels of the cells that start at massive body a: (dp, dm], dp = lcp with the
+// body before, dm = lcp with the body after, deepened to the expansion chain's
+// lowest level at the first massive body.
+struct Levels {
+    int dp, dm;
+};
+
+__device__ __forceinline__ int chain_level(int dm, const uint32_t *midx, int a, int chain, int first_massive)
 {
-    int v = d[a];
-    if ((int)midx[a] == box->first_massive && box->chain_lmax > v) v = box->chain_lmax;
-    return v;
+    return chain > dm && (int)midx[a] == first_massive ? chain : dm;
 }
 
-__global__ void k_lcp(const unsigned long long *mhi, const uint32_t *mlo, const uint32_t *midx, hc_box *box,
-                      int32_t *d, hc_status *st)
+// Nodes of every depth: each body's cells and its leaf, counted in columns of
+// shared memory, one per lane (no conflicts, no atomics).
+__global__ void __launch_bounds__(256) k_depth_count(const unsigned long long *mhi, const uint32_t *klo,
+                                                     const uint32_t *midx, const hc_box *box, uint32_t *count,
+                                                     hc_status *st)
 {
-    const int M = box->nmassive;
+    __shared__ uint32_t h[8][32][32];
+    const int M = box->nmassive, chain = box->chain_lmax, fm = box->first_massive;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if ((int64_t)blockIdx.x * blockDim.x >= M) return;
+    for (int d = 0; d < 32; d++) h[wid][d][lane] = 0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < M; a += gridDim.x * blockDim.x) {
-        int v = -1;
+        const unsigned long long k = mhi[a];
+        const int dp = a > 0 ? min(lcp_digits(mhi[a - 1], k, klo, midx, a - 1, a), 29) : -1;
+        int dm = -1;
         if (a + 1 < M) {
-            v = lcp_digits(mhi[a], mlo[a], mhi[a + 1], mlo[a + 1]);
-            if (v >= 30) {                     // assert(l != 0), load.c:113
+            dm = lcp_digits(k, mhi[a + 1], klo, midx, a, a + 1);
+            if (dm >= 30) {                    // assert(l != 0), load.c:113
                 atomicCAS(&st->error, 0, HC_ERR_COINCIDENT);
                 st->info = (int)midx[a];
-                v = 29;
+                dm = 29;
             }
         }
-        d[a] = v;
-    }
-}
-
-__global__ void k_ccount(const int32_t *d, const uint32_t *midx, const hc_box *box, int32_t *ccount)
-{
-    const int M = box->nmassive;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < M; a += gridDim.x * blockDim.x) {
-        int dp = a > 0 ? d[a - 1] : -1;
-        int dm = dprime(d, midx, a, box);
-        ccount[a] = dm > dp ? dm - dp : 0;
-    }
-}
-
-__global__ void k_post_count(int32_t *cstart, hc_box *box, int64_t maxcell, hc_status *st)
-{
-    const int M = box->nmassive;
-    int ncell = cstart[M];
-    box->ncell = ncell;
-    box->nnode = M + ncell;
-    if (ncell > maxcell) {                      // makecell, load.c:237-239
-        atomicCAS(&st->error, 0, HC_ERR_CELLS);
-        st->info = (int)maxcell;
-        box->nnode = 0;                         // later kernels see an empty tree
-        box->ncell = 0;
-    }
-}
-
-// Pre-order layout: for each sorted massive body a, the cells that start
-// at a (levels dprev+1 .. d'[a], outermost first), then body a itself.
-__global__ void k_emit_preorder(const int32_t *d, const uint32_t *midx, const int32_t *cstart, const hc_box *box,
-                                int64_t maxnode, int32_t *pre_depth, int32_t *pre_a,
-                                unsigned long long *dkey, uint32_t *dval)
-{
-    const int M = box->nmassive;
-    if (box->nnode > maxnode || box->nnode == 0) return;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < M; a += gridDim.x * blockDim.x) {
-        int dp = a > 0 ? d[a - 1] : -1;
-        int dm = dprime(d, midx, a, box);
-        int base = a + cstart[a];
-        int p = base;
-        for (int L = dp + 1; L <= dm; L++, p++) {
-            pre_depth[p] = L;
-            pre_a[p] = a;
-            dkey[p] = (unsigned long long)L;
-            dval[p] = (uint32_t)p;
-        }
-        int depth = (dp > dm ? dp : dm) + 1;    // parent is the deepest cell holding a
-        p = a + cstart[a + 1];
-        pre_depth[p] = depth;
-        pre_a[p] = -1 - a;
-        dkey[p] = (unsigned long long)depth;
-        dval[p] = (uint32_t)p;
-    }
-}
-
-__global__ void k_levels(const uint32_t *offs, hc_box *box)
-{
-    // offs: the depth sort's digit offsets (exclusive scan of its depth counts)
-    int D = threadIdx.x;
-    if (D <= HC_MAXLEVEL + 1) {
-        int v = D <= HC_MAXLEVEL ? (int)offs[D] : box->nnode;
-        if (v > box->nnode) v = box->nnode;
-        box->level_start[D] = v;
+        dm = chain_level(dm, midx, a, chain, fm);
+        for (int L = dp + 1; L <= dm; L++) h[wid][L][lane]++;
+        h[wid][max(dp, dm) + 1][lane]++;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int md = 0;
-        for (int l = 0; l <= HC_MAXLEVEL; l++)
-            if (box->level_start[l + 1] > box->level_start[l]) md = l;
-        box->max_depth = md;
+    // warp w sums depths w, w + 8, ... over all warps' columns
+    for (int d = wid; d < 32; d += 8) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) v += h[w][d][lane];
+        v = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0 && v) atomicAdd(&count[d], v);
     }
 }
 
-__global__ void k_pre2bfs(const uint32_t *bfs2pre, const hc_box *box, uint32_t *pre2bfs)
+// The nodes in breadth-first order.  A tile holds TB consecutive massive
+// bodies, TI per thread; a thread's nodes are counted per depth, the counts
+// scanned over the threads and (look-back, one depth per lane) over the tiles.
+// A node's place is its depth's start + the nodes of its depth before it in
+// pre-order; link = the start of the next depth + the nodes of that depth
+// before it: a cell's first child, and the next node's link is the end of its
+// children.
+constexpr int TI = 8, TB = 256 * TI;
+__global__ void __launch_bounds__(256) k_emit_nodes(const unsigned long long *mhi, const uint32_t *klo,
+                                                    const uint32_t *midx, hc_box *box, int64_t maxcell,
+                                                    const uint32_t *count, uint32_t *bfs_a, int32_t *bfs_link,
+                                                    uint8_t *bfs_d, uint32_t *status, uint32_t *ctr, hc_status *st)
 {
-    const int nn = box->nnode;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x)
-        pre2bfs[bfs2pre[k]] = (uint32_t)k;
-}
-
-// parent = the node one level up with the largest pre-order index below ours
-// (bdep: each node's depth in breadth-first order, the depth sort's keys)
-__global__ void k_parent(const uint32_t *bfs2pre, const unsigned long long *bdep, const hc_box *box, int32_t *parent)
-{
-    const int nn = box->nnode;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-        uint32_t p = bfs2pre[k];
-        int D = (int)bdep[k];
-        if (D == 0) {
-            parent[k] = -1;
-            continue;
-        }
-        int lo = box->level_start[D - 1], hi = box->level_start[D] - 1;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (bfs2pre[mid] < p) lo = mid;
-            else hi = mid - 1;
-        }
-        parent[k] = lo;
+    __shared__ unsigned long long sk[TB + 2];      // keys of bodies base - 1 .. base + TB
+    __shared__ uint16_t cnt[32][256];
+    __shared__ int start[33], place[33];
+    __shared__ uint32_t s_tile;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (tid == 0) s_tile = atomicAdd(ctr, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile, base = tile * TB;
+    const int M = box->nmassive, chain = box->chain_lmax, fm = box->first_massive;
+    if (base >= M && tile > 0) return;
+    if (wid == 0) {
+        const uint32_t c = count[lane], incl = warp_inclusive_scan(c);
+        start[lane] = (int)(incl - c);
+        if (lane == 31) start[32] = (int)incl;
     }
-}
-
-__global__ void k_children(const int32_t *parent, const unsigned long long *bdep, const hc_box *box, int2 *nodeC,
-                           int32_t *lastc)
-{
-    const int nn = box->nnode;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-        int p = parent[k];
-        if (p < 0) continue;
-        int D = (int)bdep[k];
-        int ls = box->level_start[D], le = box->level_start[D + 1];
-        if (k == ls || parent[k - 1] != p) nodeC[p].x = k;
-        if (k + 1 == le || parent[k + 1] != p) lastc[p] = k;
+    __syncthreads();
+    const int total = start[32], ncell = total - M;
+    const bool fits = ncell <= maxcell;            // makecell, load.c:237-239
+    if (tile == 0) {
+        if (tid < 33) box->level_start[tid] = fits ? start[tid] : 0;
+        if (tid == 0) {
+            int md = 0;
+            for (int l = 0; l < 32; l++)
+                if (fits && start[l + 1] > start[l]) md = l;
+            box->max_depth = md;
+            box->ncell = fits ? ncell : 0;         // else later kernels see an empty tree
+            box->nnode = fits ? total : 0;
+            if (!fits) {
+                atomicCAS(&st->error, 0, HC_ERR_CELLS);
+                st->info = (int)maxcell;
+            }
+        }
+    }
+    if (!fits || base >= M) return;                // the whole tile, and every other
+    const int tn = (int)(M - base < TB ? M - base : TB);
+    for (int j = tid; j < tn + 2; j += 256) {
+        const int64_t a = base + j - 1;
+        sk[j] = a >= 0 && a < M ? mhi[a] : 0ull;
+    }
+    for (int d = 0; d < 32; d++) cnt[d][tid] = 0;
+    __syncthreads();
+    int8_t lev[TI + 1];                            // lcp of bodies a - 1, a for the thread's a and one more
+#pragma unroll
+    for (int j = 0; j <= TI; j++) {
+        const int e = tid * TI + j;
+        const int64_t a = base + e;
+        lev[j] = e <= tn && a > 0 && a < M
+                     ? (int8_t)min(lcp_digits(sk[e], sk[e + 1], klo, midx, (int)a - 1, (int)a), 29)
+                     : (int8_t)-1;
+    }
+#pragma unroll
+    for (int j = 0; j < TI; j++) {
+        const int e = tid * TI + j;
+        if (e >= tn) continue;
+        const int dp = lev[j], dm = chain_level(lev[j + 1], midx, (int)base + e, chain, fm);
+        for (int L = dp + 1; L <= dm; L++) cnt[L][tid]++;
+        cnt[max(dp, dm) + 1][tid]++;
+    }
+    __syncthreads();
+    // warp w scans depths 4 w .. 4 w + 3 over the threads (eight per lane)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int d = wid * 4 + q;
+        uint4 v = *reinterpret_cast<const uint4 *>(&cnt[d][lane * 8]);
+        uint32_t w[4] = {v.x, v.y, v.z, v.w}, sum = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t lo = w[i] & 0xffffu, hi = w[i] >> 16;
+            w[i] = sum | (sum + lo) << 16;
+            sum += lo + hi;
+        }
+        const uint32_t incl = warp_inclusive_scan(sum), ex = incl - sum;
+        *reinterpret_cast<uint4 *>(&cnt[d][lane * 8]) =
+            make_uint4(w[0] + ex * 0x10001u, w[1] + ex * 0x10001u, w[2] + ex * 0x10001u, w[3] + ex * 0x10001u);
+        if (lane == 31) place[d] = (int)incl;      // the tile's count of depth d
+    }
+    __syncthreads();
+    if (wid == 0) {
+        const uint32_t before = digit_prefix(status, tile, 32, lane, (uint32_t)place[lane], &st->error);
+        __syncwarp();
+        place[lane] = start[lane] + (int)before;
+        if (lane == 0) place[32] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < TI; j++) {
+        const int e = tid * TI + j;
+        if (e >= tn) continue;
+        const int a = (int)base + e, dp = lev[j], dm = chain_level(lev[j + 1], midx, a, chain, fm);
+        const int leaf = max(dp, dm) + 1;          // its parent is the deepest cell holding the body
+        for (int L = dp + 1; L <= leaf; L++) {
+            if (L > dm) L = leaf;
+            const int k = place[L] + cnt[L][tid]++;
+            bfs_a[k] = L == leaf ? (uint32_t)(-1 - a) : (uint32_t)a;
+            bfs_link[k] = L < 31 ? place[L + 1] + cnt[L + 1][tid] : start[32];
+            bfs_d[k] = (uint8_t)L;
+        }
     }
 }
 
 // hi = RN_f32(v), lo = RN_f32(v - hi), on the double's bits (no FP64 pipe)
 __device__ __forceinline__ void split_hilo(double v, float *hi, float *lo) { hc_split_hilo(v, hi, lo); }
 
-// Node fields that do not need the upward pass: body leaves (mass and
-// position from the body arrays) and the child range of every cell.  bdep,
-// ba: each node's depth and first massive body (-1 - rank for a body leaf)
-// in breadth-first order, carried through the depth sort.
-__global__ void k_node_init(const unsigned long long *bdep, const uint32_t *ba, const uint32_t *midx, const uint32_t *mpos, const double *mass, const double *px,
-                            const double *py, const double *pz, const hc_box *box, int2 *nodeC,
-                            const int32_t *lastc, float4 *nodeA, float4 *nodeB, float4 *nodeQ, double *nm,
-                            double *ncx, double *ncy, double *ncz, int32_t *leaf_of_sorted,
-                            hc_status *st)
-{
-    const int nn = box->nnode;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-        int D = (int)bdep[k], a = (int)ba[k];
-        if (a < 0) {
-            a = -1 - a;
-            uint32_t o = midx[a], s = mpos[a];
-            double m = mass[o], x = px[o], y = py[o], z = pz[o];
-            nm[k] = m;
-            ncx[k] = x;
-            ncy[k] = y;
-            ncz[k] = z;
-            float4 A, B;
-            split_hilo(x, &A.x, &B.x);
-            split_hilo(y, &A.y, &B.y);
-            split_hilo(z, &A.z, &B.z);
-            A.w = hc_d2f_rn(m);
-            B.w = -1.0f;
-            nodeA[k] = A;
-            nodeB[k] = B;
-            nodeQ[2 * (int64_t)k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            nodeQ[2 * (int64_t)k + 1] = make_float4(0.f, 0.f, 1.f, 0.f);   // no quadrupole, one body, bmax 0
-            nodeC[k] = make_int2(-1 - a, D << 8);      // body leaf: -1 - massive rank
-            leaf_of_sorted[s] = k;
-        } else {
-            int fc = nodeC[k].x, nc = lastc[k] - fc + 1;
-            if (fc <= k || nc < 1 || nc > 8 || fc + nc > nn) {   // children follow their parent
-                atomicCAS(&st->error, 0, HC_ERR_STATE);
-                st->info = k;
-                fc = k + 1;
-                nc = 0;
-            }
-            nodeC[k] = make_int2(fc, nc | (D << 8));
-        }
-    }
-}
-
-// hackcofm (load.c:183-226), all levels, deepest first, one grid barrier
-// per level.  Children are summed in subindex order exactly as hackcofm does.
 // The upward pass takes each level's cells only, grouped by child count: the
 // cells of a warp then run the same number of FP64 child steps and no lane
 // idles on a body leaf (the levels interleave cells and leaves in key order).
 // Group of a cell: depth * 8 + (children - 1); order inside a group is free.
 __device__ __forceinline__ int cell_group(int2 C) { return min((C.y >> 8), 31) * 8 + (C.y & 255) - 1; }
 
-__global__ void k_cell_count(const int2 *nodeC, const hc_box *box, uint32_t *cnt)
+// Node records that do not need the upward pass: body leaves (from the bodies'
+// 32-byte records) and the child range of every cell; counts the cells of each
+// group.  Bound by the gather of the leaves' records and the stores: with the
+// four FP64 arrays gathered apart (four 32-byte sectors a leaf instead of one)
+// it took 56 us at N = 2^20, 380 at 2^22 and 1960 at 2^24.
+__global__ void __launch_bounds__(256) k_node_init(const uint8_t *bdep, const uint32_t *ba, const int32_t *blink,
+                                                   const uint32_t *midx, const double4_32a *body, const hc_box *box,
+                                                   int2 *nodeC, float4 *nodeAB, float4 *nodeQ, double4_32a *nodeD,
+                                                   uint32_t *gcount, hc_status *st)
 {
     __shared__ uint32_t h[256];
+    const int nn = box->nnode;
+    if ((int64_t)blockIdx.x * blockDim.x >= nn) return;
     h[threadIdx.x] = 0;
     __syncthreads();
-    const int nn = box->nnode;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-        const int2 C = nodeC[k];
-        if (C.x >= 0 && (C.y & 255) >= 1) atomicAdd(&h[cell_group(C)], 1u);
+        const int D = (int)bdep[k];
+        int a = (int)ba[k];
+        if (a < 0) {
+            a = -1 - a;
+            const double4_32a b = body[midx[a]];
+            nodeD[k] = b;
+            float4 A, B;
+            split_hilo(b.x, &A.x, &B.x);
+            split_hilo(b.y, &A.y, &B.y);
+            split_hilo(b.z, &A.z, &B.z);
+            A.w = hc_d2f_rn(b.w);
+            B.w = -1.0f;
+            nodeAB[2 * (int64_t)k] = A;
+            nodeAB[2 * (int64_t)k + 1] = B;
+            nodeQ[2 * (int64_t)k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            nodeQ[2 * (int64_t)k + 1] = make_float4(0.f, 0.f, 1.f, 0.f);   // no quadrupole, one body, bmax 0
+            nodeC[k] = make_int2(-1 - a, D << 8);      // body leaf: -1 - massive rank
+        } else {
+            // the children end where those of the next node of the depth begin
+            int fc = blink[k];
+            const int end = k + 1 < box->level_start[D + 1] ? blink[k + 1] : box->level_start[D + 2];
+            int nc = end - fc;
+            if (fc <= k || nc < 1 || nc > 8 || fc + nc > nn) {   // children follow their parent
+                atomicCAS(&st->error, 0, HC_ERR_STATE);
+                st->info = k;
+                fc = k + 1;
+                nc = 0;
+            }
+            const int2 C = make_int2(fc, nc | (D << 8));
+            nodeC[k] = C;
+            if (nc >= 1) atomicAdd(&h[cell_group(C)], 1u);
+        }
     }
     __syncthreads();
-    if (h[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], h[threadIdx.x]);
+    if (h[threadIdx.x]) atomicAdd(&gcount[threadIdx.x], h[threadIdx.x]);
 }
 
-// group offsets off[0..256] (exclusive scan of the 256 counts) and placement
-// cursors cur[0..255]; one block of 256 threads: warp scans, then the warp sums
-__global__ void k_cell_offsets(uint32_t *off, uint32_t *cur)
+// Places each block's cells: the group offsets are the exclusive scan of the 256
+// counts (every block makes its own; block 0 leaves them in off[0..256] for
+// the upward pass), then one reservation per group per block and slots handed
+// out inside the reservation.
+__global__ void __launch_bounds__(256) k_cell_place(const int2 *nodeC, const hc_box *box, const uint32_t *count,
+                                                    uint32_t *cur, uint32_t *off, int4 *perm)
 {
-    __shared__ uint32_t wsum[8];
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const uint32_t v = off[t];
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    uint32_t before = 0;
-    for (int i = 0; i < w; i++) before += wsum[i];
-    const uint32_t ex = before + x - v;
-    off[t] = ex;
-    cur[t] = ex;
-    if (t == 255) off[256] = ex + v;
-}
-
-// places each block's cells: one reservation per group per block, then slots
-// handed out inside the reservation
-__global__ void k_cell_place(const int2 *nodeC, const hc_box *box, uint32_t *cur, int4 *perm)
-{
-    __shared__ uint32_t h[256], base[256];
+    __shared__ uint32_t h[256], base[256], first[256], sh[32];
     const int nn = box->nnode;
+    if (blockIdx.x > 0 && (int64_t)blockIdx.x * blockDim.x >= nn) return;
+    {
+        const uint32_t v = count[threadIdx.x];
+        uint32_t total;
+        first[threadIdx.x] = block_exclusive_scan<uint32_t>(v, sh, &total);
+        if (blockIdx.x == 0) {
+            off[threadIdx.x] = first[threadIdx.x];
+            if (threadIdx.x == 0) off[256] = total;
+        }
+    }
     for (int k0 = blockIdx.x * blockDim.x; k0 < nn; k0 += gridDim.x * blockDim.x) {
         const int k = k0 + threadIdx.x;
         h[threadIdx.x] = 0;
@@ -625,7 +714,7 @@ __global__ void k_cell_place(const int2 *nodeC, const hc_box *box, uint32_t *cur
             }
         }
         __syncthreads();
-        if (h[threadIdx.x]) base[threadIdx.x] = atomicAdd(&cur[threadIdx.x], h[threadIdx.x]);
+        if (h[threadIdx.x]) base[threadIdx.x] = first[threadIdx.x] + atomicAdd(&cur[threadIdx.x], h[threadIdx.x]);
         __syncthreads();
         if (grp >= 0) perm[base[grp] + slot] = make_int4(k, C.x, C.y, 0);   // the cell and its child links
         __syncthreads();
@@ -637,10 +726,10 @@ __device__ __forceinline__ void prefetch_l1(const void *p)
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-__global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *box, const int2 *nodeC, double *nm,
-                                                     double *ncx, double *ncy, double *ncz, float4 *nodeA,
-                                                     float4 *nodeB, float4 *nodeQ, const int4 *cperm,
-                                                     const uint32_t *coff)
+// hackcofm (load.c:183-226), all levels, deepest first, one grid barrier
+// per level.  Children are summed in subindex order exactly as hackcofm does.
+__global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *box, double4_32a *nodeD, float4 *nodeAB,
+                                                     float4 *nodeQ, const int4 *cperm, const uint32_t *coff)
 {
     cg::grid_group grid = cg::this_grid();
     const int maxd = box->nnode > 0 ? box->max_depth : -1;
@@ -662,10 +751,8 @@ __global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *
             const int k = P.x, fc = P.y, nc = P.z & 255;
             // the children's FP32 node data are needed after the FP64 sums: start
             // bringing their lines into L1 now, beside the FP64 loads
-            prefetch_l1(nodeA + fc);
-            prefetch_l1(nodeA + fc + nc - 1);
-            prefetch_l1(nodeB + fc);
-            prefetch_l1(nodeB + fc + nc - 1);
+            prefetch_l1(nodeAB + 2 * (int64_t)fc);
+            prefetch_l1(nodeAB + 2 * (int64_t)(fc + nc) - 1);
             prefetch_l1(nodeQ + 2 * (int64_t)fc);
             prefetch_l1(nodeQ + 2 * (int64_t)(fc + nc) - 1);
             // The children's loads are issued together (predicated on the
@@ -674,23 +761,17 @@ __global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *
             double m = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
 #pragma unroll
             for (int h = 0; h < 8; h += 4) {
-                double cm[4], px[4], py[4], pz[4];
+                double4_32a c[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (h + i < nc) c[i] = nodeD[fc + h + i];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     if (h + i < nc) {
-                        cm[i] = nm[fc + h + i];
-                        px[i] = ncx[fc + h + i];
-                        py[i] = ncy[fc + h + i];
-                        pz[i] = ncz[fc + h + i];
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (h + i < nc) {
-                        m = dadd(m, cm[i]);
-                        cx = dadd(cx, dmul(px[i], cm[i]));
-                        cy = dadd(cy, dmul(py[i], cm[i]));
-                        cz = dadd(cz, dmul(pz[i], cm[i]));
+                        m = dadd(m, c[i].w);
+                        cx = dadd(cx, dmul(c[i].x, c[i].w));
+                        cy = dadd(cy, dmul(c[i].y, c[i].w));
+                        cz = dadd(cz, dmul(c[i].z, c[i].w));
                     }
                 }
             }
@@ -713,12 +794,12 @@ __global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *
                 float4 ca[4], cb[4], q0[4], q1[4];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const int ch = fc + h + i;
+                    const int64_t ch = 2 * (int64_t)(fc + h + i);
                     if (h + i < nc) {
-                        ca[i] = nodeA[ch];
-                        cb[i] = nodeB[ch];
-                        q1[i] = nodeQ[2 * (int64_t)ch + 1];
-                        if (usequad) q0[i] = nodeQ[2 * (int64_t)ch];
+                        ca[i] = nodeAB[ch];
+                        cb[i] = nodeAB[ch + 1];
+                        q1[i] = nodeQ[ch + 1];
+                        if (usequad) q0[i] = nodeQ[ch];
                     }
                 }
 #pragma unroll
@@ -740,32 +821,17 @@ __global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *
                     }
                 }
             }
-            nm[k] = m;
-            ncx[k] = cx;
-            ncy[k] = cy;
-            ncz[k] = cz;
+            nodeD[k] = make_double4_32a(cx, cy, cz, m);
             A.w = hc_d2f_rn(m);
             B.w = dsqf;
-            nodeA[k] = A;
-            nodeB[k] = B;
+            nodeAB[2 * (int64_t)k] = A;
+            nodeAB[2 * (int64_t)k + 1] = B;
             nodeQ[2 * (int64_t)k] = make_float4(Q[0], Q[1], Q[2], Q[3]);
             nodeQ[2 * (int64_t)k + 1] = make_float4(Q[4], Q[5], nbody, bmax);
         }
         grid.sync();
     }
 }
-
-// clear the child links of the nodes of this build
-__global__ void k_clear_links(const hc_box *box, int64_t maxnode, int2 *nodeC, int32_t *lastc)
-{
-    const int64_t nn = box->nnode < maxnode ? box->nnode : maxnode;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x) {
-        nodeC[k] = make_int2(-1, -1);
-        lastc[k] = -1;
-    }
-}
-
-__global__ void k_set_nmassive(const int32_t *total, hc_box *box) { box->nmassive = *total; }
 
 // ---------------- walk groups aligned with the tree ----------------
 // A group is a run of massive bodies (in key order) that lie in one cell of
@@ -786,63 +852,85 @@ __device__ __forceinline__ int node_count(const uint32_t *ba, const float4 *node
     return (int)fminf(nodeQ[2 * (int64_t)k + 1].z, 2.0e9f);
 }
 
-template <bool EMIT>
-__global__ void k_groups(const uint32_t *ba, const float4 *nodeQ, const int32_t *parent,
-                         const int2 *nodeC, const hc_box *box, int64_t maxnode, int gmax, int32_t *ng,
-                         const int32_t *goff, int32_t *gstart, int32_t *gcount)
+// Packs of node k's children into groups (for the root also itself, when it is
+// small): calls f(first body, bodies) for each and returns their number.
+template <typename F>
+__device__ __forceinline__ int node_packs(const uint32_t *ba, const float4 *nodeQ, const int2 *nodeC, int k, int gmax,
+                                          F f)
 {
-    const int nn = box->nnode;
-    for (int64_t kk = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; kk < maxnode;
-         kk += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)kk;
-        if (k >= nn) {
-            if (!EMIT) ng[k] = 0;
-            continue;
+    int first, packs = 0;
+    const int cnt = node_count(ba, nodeQ, k, &first);
+    if (cnt <= gmax) {                         // only the root can be a small group on its own here
+        if (k == 0) {
+            f(first, cnt);
+            packs = 1;
         }
-        int first;
-        const int cnt = node_count(ba, nodeQ, k, &first);
-        int out = EMIT ? goff[k] : 0, packs = 0;
-        if (cnt <= gmax) {                         // only the root can be a small group on its own here
-            if (parent[k] < 0) {
-                if (EMIT) {
-                    gstart[out] = first;
-                    gcount[out] = cnt;
-                }
-                packs = 1;
-            }
-        } else {
-            const int fc = nodeC[k].x, nc = nodeC[k].y & 255;
-            int cur = 0, cur_first = 0;
-            for (int i = 0; i < nc; i++) {
-                int f;
-                const int cc = node_count(ba, nodeQ, fc + i, &f);
-                if (cc > gmax || cur + cc > gmax) {
-                    if (cur > 0) {
-                        if (EMIT) {
-                            gstart[out + packs] = cur_first;
-                            gcount[out + packs] = cur;
-                        }
-                        packs++;
-                        cur = 0;
-                    }
-                    if (cc > gmax) continue;
-                }
-                if (cur == 0) cur_first = f;
-                cur += cc;
-            }
-            if (cur > 0) {
-                if (EMIT) {
-                    gstart[out + packs] = cur_first;
-                    gcount[out + packs] = cur;
-                }
-                packs++;
-            }
-        }
-        if (!EMIT) ng[k] = packs;
+        return packs;
     }
+    const int fc = nodeC[k].x, nc = nodeC[k].y & 255;
+    int cur = 0, cur_first = 0;
+    for (int i = 0; i < nc; i++) {
+        int g;
+        const int cc = node_count(ba, nodeQ, fc + i, &g);
+        if (cc > gmax || cur + cc > gmax) {
+            if (cur > 0) {
+                f(cur_first, cur);
+                packs++;
+                cur = 0;
+            }
+            if (cc > gmax) continue;
+        }
+        if (cur == 0) cur_first = g;
+        cur += cc;
+    }
+    if (cur > 0) {
+        f(cur_first, cur);
+        packs++;
+    }
+    return packs;
 }
 
-__global__ void k_set_ngroups(const int32_t *goff, int64_t maxnode, hc_box *box) { box->ngroups = goff[maxnode]; }
+// The group table in node order, in one pass (decoupled look-back over tiles of
+// four nodes per thread).
+constexpr int GI = 4, GTILE = 256 * GI;
+__global__ void __launch_bounds__(256) k_groups(const uint32_t *ba, const float4 *nodeQ, const int2 *nodeC, hc_box *box,
+                                                int gmax, int32_t *gstart, int32_t *gcount, uint32_t *status,
+                                                uint32_t *ctr, int *err)
+{
+    __shared__ uint32_t s_tile, s_prefix, sh[32];
+    if (threadIdx.x == 0) s_tile = atomicAdd(ctr, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile, base = tile * GTILE + threadIdx.x * GI;
+    const int nn = box->nnode;
+    if (tile * GTILE >= nn) {
+        if (tile == 0 && threadIdx.x == 0) box->ngroups = 0;
+        return;
+    }
+    uint32_t n = 0;
+#pragma unroll
+    for (int i = 0; i < GI; i++)
+        if (base + i < nn) n += node_packs(ba, nodeQ, nodeC, (int)base + i, gmax, [](int, int) {});
+    uint32_t agg;
+    const uint32_t ex = block_exclusive_scan<uint32_t>(n, sh, &agg);
+    if (threadIdx.x < 32) {
+        const uint32_t prefix = tile_prefix(status, tile, agg, err);
+        if (threadIdx.x == 0) {
+            s_prefix = prefix;
+            if ((tile + 1) * GTILE >= nn) box->ngroups = (int)(prefix + agg);    // the last tile
+        }
+    }
+    __syncthreads();
+    if (n == 0) return;
+    uint32_t out = s_prefix + ex;
+#pragma unroll
+    for (int i = 0; i < GI; i++)
+        if (base + i < nn)
+            node_packs(ba, nodeQ, nodeC, (int)base + i, gmax, [&](int first, int cnt) {
+                gstart[out] = first;
+                gcount[out] = cnt;
+                out++;
+            });
+}
 
 // ---------------- treecode1 critical radii ----------------
 // setrcrit (treecode1/treeload.c:232-252) for every cell: the cell's centre
@@ -853,7 +941,7 @@ __global__ void k_set_ngroups(const int32_t *goff, int64_t maxnode, hc_box *box)
 //   theta = 0: (2 rsize)^2 (always open).
 __global__ void k_rcrit(int kind, double theta, const hc_box *box, const uint32_t *ba,
                         const uint32_t *midx, const double *px, const double *py, const double *pz, const int2 *nodeC,
-                        const double *ncx, const double *ncy, const double *ncz, float *rcrit2)
+                        const double4_32a *nodeD, float *rcrit2)
 {
     const int nn = box->nnode;
     const double rsize = box->rsize;
@@ -862,7 +950,8 @@ __global__ void k_rcrit(int kind, double theta, const hc_box *box, const uint32_
         if (C.x < 0) continue;                           // body leaf
         const int D = C.y >> 8;
         const uint32_t o = midx[ba[k]];
-        const double p[3] = {px[o], py[o], pz[o]}, cm[3] = {ncx[k], ncy[k], ncz[k]};
+        const double4_32a nd = nodeD[k];
+        const double p[3] = {px[o], py[o], pz[o]}, cm[3] = {nd.x, nd.y, nd.z};
         const double size = ldexp(rsize, -D), unit = ldexp(rsize, -30);
         const int shift = 30 - D;
         double off2 = 0.0, bmax2 = 0.0;
@@ -892,18 +981,69 @@ __global__ void k_rcrit(int kind, double theta, const hc_box *box, const uint32_
 
 void hc_rcrit_launch(hc_ctx *c, int kind, double theta)
 {
-    k_rcrit<<<hc_grid(c->maxnode, 256), 256, 0, c->stream>>>(kind, theta, c->box, c->bfs_a, c->midx,
-                                                              c->px, c->py, c->pz, c->nodeC, c->ncx, c->ncy, c->ncz,
-                                                              c->rcrit2);
+    k_rcrit<<<hc_grid(c->maxnode, 256), 256, 0, c->stream>>>(kind, theta, c->box, c->bfs_a, c->xidx,
+                                                              c->px, c->py, c->pz, c->nodeC, c->nodeD, c->rcrit2);
     c->launches++;
 }
 
 void hc_keys_for_points(hc_ctx *c, const double *x, const double *y, const double *z, int64_t n,
-                        unsigned long long *khi, uint32_t *klo, uint32_t *kval)
+                        unsigned long long *khi, uint32_t *klo, double4_32a *body, uint32_t *scratch)
 {
-    k_keys<<<hc_grid(n, 256), 256, 0, c->stream>>>(x, y, z, n, c->box, khi, klo, kval);
+    const bool counts = !hc_sort_counts_digits(n);
+    // enough blocks to hide the loads; each adds up to 2048 digit counts
+    k_keys<<<hc_grid(n, 256, counts ? 152 * 4 : 152 * 16), 256, 0, c->stream>>>(x, y, z, c->mass, n, c->box, khi, klo, body,
+                                                                               counts ? scratch : nullptr);
     c->launches++;
 }
+
+// The build's own scratch after the sort's: look-back words and counters, all
+// zeroed together at the start of a build.
+namespace {
+struct BuildScratch {
+    uint32_t *ctr;                       // tile counters of box, massive, emit, groups
+    uint32_t *depth, *gcount, *gcur, *goff;
+    uint32_t *box, *massive, *emit, *groups;
+    int64_t words;                       // of all, sort included
+};
+
+BuildScratch build_scratch(uint32_t *p, int64_t n, int64_t maxnode)
+{
+    BuildScratch b;
+    int64_t w = hc_sort_scratch_words(n);
+    auto take = [&](int64_t count) {
+        uint32_t *q = p ? p + w : nullptr;
+        w += (count + 31) / 32 * 32;
+        return q;
+    };
+    b.ctr = take(32);
+    b.depth = take(32);
+    b.gcount = take(256);
+    b.gcur = take(256);
+    b.goff = take(257);
+    b.box = take((n + BOX_TILE - 1) / BOX_TILE);
+    b.massive = take((n + MC_TILE - 1) / MC_TILE);
+    b.emit = take((n + TB - 1) / TB * 32);
+    b.groups = take((maxnode + GTILE - 1) / GTILE);
+    b.words = w;
+    return b;
+}
+}  // namespace
+
+int64_t hc_build_scratch_words(int64_t n, int64_t maxnode) { return build_scratch(nullptr, n, maxnode).words; }
+
+// Walk groups aligned with the tree (for c->table_gmax, fixed by the build).
+void hc_groups_launch(hc_ctx *c)
+{
+    const BuildScratch b = build_scratch(c->hist, c->n, c->maxnode);
+    k_groups<<<(unsigned)((c->maxnode + GTILE - 1) / GTILE), 256, 0, c->stream>>>(
+        c->bfs_a, c->nodeQ, c->nodeC, c->box, c->table_gmax, c->gstart, c->gcount, b.groups, b.ctr + 3, &c->st->error);
+    c->launches++;
+}
+
+// Whether a build of this configuration makes the group table: the per-body
+// rule over consecutive bodies does not use it.  A walk that needs the table of
+// a tree built without it makes it first (hc_walk_launch).
+bool hc_build_makes_groups(const hc_ctx *c) { return c->criterion != HC_CRITERION_BODY || c->group_kind == 1; }
 
 // Launch the whole build on the context stream without host synchronisation
 // (graph-capturable); errors land in the device status word.
@@ -912,81 +1052,58 @@ int hc_tree_build(hc_ctx *c)
     const int64_t n = c->n;
     cudaStream_t s = c->stream;
     const int B = 256;
-    const int G = hc_grid(n, B);
-    int32_t *outside = c->flags;
-    int32_t *opos = c->flags + 2 * n;
-    int2 *first2 = reinterpret_cast<int2 *>(c->flags + 3 * n + (n & 1));   // [G], 8-byte aligned
+    const BuildScratch b = build_scratch(c->hist, n, c->maxnode);
+    HC_CUDA(cudaMemsetAsync(c->hist, 0, sizeof(uint32_t) * b.words, s));
 
     // 1. expandbox replay
-    k_box_flags<<<G, B, 0, s>>>(c->mass, c->px, c->py, c->pz, n, c->box, outside, first2);
-    hc_scan_exclusive_i32(c, outside, opos, n, c->ncand);
-    k_box_compact<<<G, B, 0, s>>>(outside, opos, n, c->cand);
-    k_box_replay<<<1, 256, 0, s>>>(c->px, c->py, c->pz, c->cand, c->ncand, first2, G, c->box, c->st);
-    c->launches += 3;
+    const int boxtiles = (int)((n + BOX_TILE - 1) / BOX_TILE);
+    k_box_outside<<<boxtiles, B, 0, s>>>(c->mass, c->px, c->py, c->pz, n, c->box, c->cand, c->ncand, c->first2, b.box,
+                                         b.ctr, &c->st->error);
+    k_box_replay<<<1, 256, 0, s>>>(c->px, c->py, c->pz, c->cand, c->ncand, c->first2, boxtiles, c->box, c->st,
+                                   c->all_massive ? (int)n : -1);
+    c->launches += 2;
 
     // 2-3. keys, sort, massive compaction
-    hc_keys_for_points(c, c->px, c->py, c->pz, n, c->khi[0], c->klo[0], c->kval[0]);
-    int sel = hc_radix_sort_keys(c, c->hist, c->khi, c->klo, c->kval, n, 0, 64, true);
-    c->sort_sel = sel;
-    c->sidx = c->kval[sel];
-    int32_t *sflag = c->flags;            // reuse (outside no longer needed)
-    int32_t *srank = c->flags + n;
-    k_sorted_massive<<<G, B, 0, s>>>(c->sidx, c->mass, n, sflag);
-    hc_scan_exclusive_i32(c, sflag, srank, n, c->flags + 2 * n);
-    k_set_nmassive<<<1, 1, 0, s>>>(c->flags + 2 * n, c->box);
-    k_mcompact<<<G, B, 0, s>>>(sflag, srank, n, c->khi[sel], c->klo[sel], c->sidx, c->box, c->mhi, c->mlo,
-                               c->midx, c->mpos, c->s_rank, c->leaf_of_sorted, c->tord);
-    c->launches += 3;
-
-    // 4. cells in pre-order
-    k_lcp<<<G, B, 0, s>>>(c->mhi, c->mlo, c->midx, c->box, c->dlcp, c->st);
-    int32_t *cstart = c->flags + n;       // [n+1]
-    HC_CUDA(cudaMemsetAsync(c->ccount, 0, sizeof(int32_t) * (n + 1), s));
-    k_ccount<<<G, B, 0, s>>>(c->dlcp, c->midx, c->box, c->ccount);
-    hc_scan_exclusive_i32(c, c->ccount, cstart, n + 1, nullptr);
-    k_post_count<<<1, 1, 0, s>>>(cstart, c->box, c->maxcell, c->st);
-    const int Gn = hc_grid(c->maxnode, B);
-    k_emit_preorder<<<G, B, 0, s>>>(c->dlcp, c->midx, cstart, c->box, c->maxnode, c->pre_info, c->pre_a,
-                                    c->dkey[0], c->dval[0]);
-    c->launches += 5;
-
-    // 5. breadth-first layout: stable sort of the pre-order by depth (count on the device)
-    // the pre-order's first bodies ride along as the sort's low words, so the
-    // later kernels read depth and first body in breadth-first order
-    uint32_t *alo[2] = {reinterpret_cast<uint32_t *>(c->pre_a), c->bfs_a};
-    int dsel = hc_radix_sort_keys(c, c->hist, c->dkey, alo, c->dval, c->maxnode, 0, 8, false, &c->box->nnode);
-    if (dsel != 1) {          // one 8-bit pass: the result is in the second buffers
-        c->err = "depth sort: unexpected pass count";
-        return HC_ERR_STATE;
+    hc_keys_for_points(c, c->px, c->py, c->pz, n, c->khi[0], c->klo, c->body, c->hist);
+    const int sel = hc_radix_sort_keys(c, c->hist, c->khi, c->kval, n, c->klo);
+    if (c->all_massive) {
+        c->xhi = c->khi[sel];
+        c->xidx = c->tord = c->kval[sel];
+    } else {
+        // the other buffers of the sort are free again
+        c->xhi = c->khi[sel ^ 1];
+        c->xidx = c->tord = c->kval[sel ^ 1];
+        uint32_t *massless = reinterpret_cast<uint32_t *>(c->cand);
+        k_massive<<<(unsigned)((n + MC_TILE - 1) / MC_TILE), B, 0, s>>>(c->kval[sel], c->khi[sel], c->mass, n, c->box,
+                                                                        c->khi[sel ^ 1], c->kval[sel ^ 1], massless,
+                                                                        b.massive, b.ctr + 1, &c->st->error);
+        k_target_tail<<<hc_grid(n, B), B, 0, s>>>(n, c->box, massless, c->kval[sel ^ 1]);
+        c->launches += 2;
     }
-    c->bfs2pre = c->dval[dsel];
-    const unsigned long long *bdep = c->dkey[dsel];
-    k_levels<<<1, 64, 0, s>>>(c->hist, c->box);      // the sort leaves its digit offsets at hist[0..255]
-    k_pre2bfs<<<Gn, B, 0, s>>>(c->bfs2pre, c->box, c->pre2bfs);
-    k_parent<<<Gn, B, 0, s>>>(c->bfs2pre, bdep, c->box, c->parent);
-    k_clear_links<<<Gn, B, 0, s>>>(c->box, c->maxnode, c->nodeC, c->lastc);
-    k_children<<<Gn, B, 0, s>>>(c->parent, bdep, c->box, c->nodeC, c->lastc);
-    k_node_init<<<Gn, B, 0, s>>>(bdep, c->bfs_a, c->midx, c->mpos, c->mass, c->px, c->py,
-                                 c->pz, c->box, c->nodeC, c->lastc, c->nodeA, c->nodeB, c->nodeQ, c->nm, c->ncx,
-                                 c->ncy, c->ncz, c->leaf_of_sorted, c->st);
-    c->launches += 7;
 
-    // 6. upward pass, deepest level first, one cooperative launch, over the
-    // cells grouped by depth and child count.  Work forked onto the side
-    // stream joins here: nothing else runs beside the cooperative launch.
+    // 4. the nodes in breadth-first order
+    k_depth_count<<<hc_grid(n, B, 152 * 4), B, 0, s>>>(c->xhi, c->klo, c->xidx, c->box, b.depth, c->st);
+    k_emit_nodes<<<(unsigned)((n + TB - 1) / TB), B, 0, s>>>(c->xhi, c->klo, c->xidx, c->box, c->maxcell, b.depth, c->bfs_a,
+                                                           c->bfs_link, c->bfs_d, b.emit, b.ctr + 2, c->st);
+
+    // 5. node records; cells grouped by depth and child count
+    const int Gn = hc_grid(c->maxnode, B);
+    k_node_init<<<Gn, B, 0, s>>>(c->bfs_d, c->bfs_a, c->bfs_link, c->xidx, c->body, c->box, c->nodeC, c->nodeAB, c->nodeQ,
+                                 c->nodeD, b.gcount, c->st);
+    k_cell_place<<<Gn, B, 0, s>>>(c->nodeC, c->box, b.gcount, b.gcur, b.goff, c->cperm);
+    c->launches += 4;
+
+    // 6. upward pass, deepest level first, one cooperative launch.  Work forked
+    // onto the side stream joins here: nothing else runs beside the
+    // cooperative launch.
     if (c->join_pending) {
         c->join_pending = false;
         HC_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
     }
-    HC_CUDA(cudaMemsetAsync(c->cbins, 0, sizeof(uint32_t) * 520, s));
-    k_cell_count<<<Gn, B, 0, s>>>(c->nodeC, c->box, c->cbins);
-    k_cell_offsets<<<1, 256, 0, s>>>(c->cbins, c->cbins + 260);
-    k_cell_place<<<Gn, B, 0, s>>>(c->nodeC, c->box, c->cbins + 260, c->cperm);
-    c->launches += 3;
     {
         int usequad = c->prm.usequad;
-        void *args[] = {&usequad, &c->box, &c->nodeC, &c->nm, &c->ncx, &c->ncy, &c->ncz, &c->nodeA, &c->nodeB,
-                        &c->nodeQ, &c->cperm, &c->cbins};
+        uint32_t *goff = b.goff;
+        void *args[] = {&usequad, &c->box, &c->nodeD, &c->nodeAB, &c->nodeQ, &c->cperm, &goff};
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(c->cofm_grid);
         cfg.blockDim = dim3(256);
@@ -1001,14 +1118,9 @@ int hc_tree_build(hc_ctx *c)
     }
 
     // 7. walk groups aligned with the tree
-    const int gmax = hc_table_gmax(c);
-    k_groups<false><<<Gn, B, 0, s>>>(c->bfs_a, c->nodeQ, c->parent, c->nodeC,
-                                     c->box, c->maxnode, gmax, c->gcnt, nullptr, nullptr, nullptr);
-    hc_scan_exclusive_i32(c, c->gcnt, c->goff, c->maxnode + 1, nullptr);
-    k_set_ngroups<<<1, 1, 0, s>>>(c->goff, c->maxnode, c->box);
-    k_groups<true><<<Gn, B, 0, s>>>(c->bfs_a, c->nodeQ, c->parent, c->nodeC, c->box, c->maxnode,
-                                    gmax, nullptr, c->goff, c->gstart, c->gcount);
-    c->launches += 3;
+    c->table_gmax = hc_table_gmax(c);
+    c->have_groups = hc_build_makes_groups(c);
+    if (c->have_groups) hc_groups_launch(c);
     return HC_OK;
 }
 
@@ -1034,40 +1146,31 @@ int hc_tree_dump_impl(hc_ctx *c, int32_t *level, int32_t *corner, int32_t *count
     for (int64_t i = 0; i < c->n && bparent; i++) bparent[i] = -1;
     if (nn <= 0) return 0;
     auto H = [&](size_t bytes) { return std::unique_ptr<char[]>(new char[bytes > 0 ? bytes : 1]); };
-    auto hb = H(sizeof(uint32_t) * nn), hd = H(sizeof(int32_t) * nn), ha = H(sizeof(int32_t) * nn),
-         hbb = H(sizeof(int32_t) * nn), hmhi = H(sizeof(unsigned long long) * M), hmlo = H(sizeof(uint32_t) * M),
-         hmidx = H(sizeof(uint32_t) * M), hnm = H(sizeof(double) * nn), hx = H(sizeof(double) * nn),
-         hy = H(sizeof(double) * nn), hz = H(sizeof(double) * nn), hq = H(sizeof(float4) * 2 * nn);
-    uint32_t *bfs2pre = (uint32_t *)hb.get();
-    int32_t *pd = (int32_t *)hd.get(), *pa = (int32_t *)ha.get(), *pb = (int32_t *)hbb.get();
+    auto hl = H(sizeof(uint32_t) * c->n), ha = H(sizeof(int32_t) * nn), hbb = H(sizeof(int32_t) * nn),
+         hmhi = H(sizeof(unsigned long long) * M), hmidx = H(sizeof(uint32_t) * M), hd = H(sizeof(double) * 4 * nn),
+         hq = H(sizeof(float4) * 2 * nn);
+    int32_t *pa = (int32_t *)ha.get(), *pb = (int32_t *)hbb.get();
     unsigned long long *mhi = (unsigned long long *)hmhi.get();
-    uint32_t *mlo = (uint32_t *)hmlo.get(), *midx = (uint32_t *)hmidx.get();
-    double *nm = (double *)hnm.get(), *nx = (double *)hx.get(), *ny = (double *)hy.get(), *nz = (double *)hz.get();
+    uint32_t *klo = (uint32_t *)hl.get(), *midx = (uint32_t *)hmidx.get();
+    double *nd = (double *)hd.get();
     float *nq = (float *)hq.get();
-    HC_CUDA(cudaMemcpy(bfs2pre, c->bfs2pre, sizeof(uint32_t) * nn, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(pd, c->pre_info, sizeof(int32_t) * nn, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(pa, c->pre_a, sizeof(int32_t) * nn, cudaMemcpyDeviceToHost));
+    std::unique_ptr<int2[]> C(new int2[nn]);
+    HC_CUDA(cudaMemcpy(C.get(), c->nodeC, sizeof(int2) * nn, cudaMemcpyDeviceToHost));
+    HC_CUDA(cudaMemcpy(pa, c->bfs_a, sizeof(int32_t) * nn, cudaMemcpyDeviceToHost));
     // bodies per node, summed up the children links (breadth-first: children
     // follow their parent, so one pass from the back)
-    {
-        std::unique_ptr<int2[]> C(new int2[nn]);
-        HC_CUDA(cudaMemcpy(C.get(), c->nodeC, sizeof(int2) * nn, cudaMemcpyDeviceToHost));
-        for (int k = nn - 1; k >= 0; k--) {
-            int cnt = 1;
-            if (C[k].x >= 0) {
-                cnt = 0;
-                for (int i = 0; i < (C[k].y & 255); i++) cnt += pb[C[k].x + i];
-            }
-            pb[k] = cnt;
+    for (int k = nn - 1; k >= 0; k--) {
+        int cnt = 1;
+        if (C[k].x >= 0) {
+            cnt = 0;
+            for (int i = 0; i < (C[k].y & 255); i++) cnt += pb[C[k].x + i];
         }
+        pb[k] = cnt;
     }
-    HC_CUDA(cudaMemcpy(mhi, c->mhi, sizeof(unsigned long long) * M, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(mlo, c->mlo, sizeof(uint32_t) * M, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(midx, c->midx, sizeof(uint32_t) * M, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(nm, c->nm, sizeof(double) * nn, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(nx, c->ncx, sizeof(double) * nn, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(ny, c->ncy, sizeof(double) * nn, cudaMemcpyDeviceToHost));
-    HC_CUDA(cudaMemcpy(nz, c->ncz, sizeof(double) * nn, cudaMemcpyDeviceToHost));
+    HC_CUDA(cudaMemcpy(mhi, c->xhi, sizeof(unsigned long long) * M, cudaMemcpyDeviceToHost));
+    HC_CUDA(cudaMemcpy(klo, c->klo, sizeof(uint32_t) * c->n, cudaMemcpyDeviceToHost));
+    HC_CUDA(cudaMemcpy(midx, c->xidx, sizeof(uint32_t) * M, cudaMemcpyDeviceToHost));
+    HC_CUDA(cudaMemcpy(nd, c->nodeD, sizeof(double) * 4 * nn, cudaMemcpyDeviceToHost));
     HC_CUDA(cudaMemcpy(nq, c->nodeQ, sizeof(float4) * 2 * nn, cudaMemcpyDeviceToHost));
     auto unspread = [](unsigned long long hi, uint32_t lo, int axis) {
         // axis 0 = x (bit 2 of each digit), 1 = y, 2 = z
@@ -1079,8 +1182,7 @@ int hc_tree_dump_impl(hc_ctx *c, int32_t *level, int32_t *corner, int32_t *count
     };
     int ci = 0;
     for (int k = 0; k < nn; k++) {
-        uint32_t p = bfs2pre[k];
-        int D = pd[p], a = pa[p];
+        const int D = C[k].y >> 8, a = pa[k];
         if (a < 0) {
             if (bparent) bparent[midx[-1 - a]] = D - 1;
             continue;
@@ -1088,18 +1190,15 @@ int hc_tree_dump_impl(hc_ctx *c, int32_t *level, int32_t *corner, int32_t *count
         if (level) level[ci] = D;
         if (corner) {
             for (int ax = 0; ax < 3; ax++) {
-                unsigned v = unspread(mhi[a], mlo[a], ax);
+                unsigned v = unspread(mhi[a], klo[midx[a]], ax);
                 unsigned mask = D >= 30 ? 0xffffffffu : ~((1u << (30 - D)) - 1u);
                 corner[3 * ci + ax] = (int32_t)(v & mask);
             }
         }
         if (count) count[ci] = pb[k];
-        if (mass) mass[ci] = nm[k];
-        if (cm) {
-            cm[3 * ci] = nx[k];
-            cm[3 * ci + 1] = ny[k];
-            cm[3 * ci + 2] = nz[k];
-        }
+        if (mass) mass[ci] = nd[4 * (int64_t)k + 3];
+        if (cm)
+            for (int ax = 0; ax < 3; ax++) cm[3 * ci + ax] = nd[4 * (int64_t)k + ax];
         if (quad)
             for (int q = 0; q < 6; q++) quad[6 * ci + q] = nq[(int64_t)8 * k + q];
         ci++;

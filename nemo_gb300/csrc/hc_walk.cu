@@ -90,9 +90,9 @@ __host__ __device__ constexpr size_t walk_smem(int mode, bool count)
 }
 
 struct WalkArgs {
-    const float4 *nodeA, *nodeB, *nodeQ;
+    const float4 *nodeAB, *nodeQ;
     const int2 *nodeC;
-    const double *ncx, *ncy, *ncz;
+    const double4_32a *nodeD;
     const hc_box *box;
     int64_t ntarget;
     const uint32_t *tsorted;              // sorted slot -> target index
@@ -801,8 +801,8 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             constexpr bool QEARLY = QUAD && MODE == 2;
             float4 Q0 = A, Q1 = A;
             if (have) {
-                A = g.nodeA[my_node];
-                B = g.nodeB[my_node];
+                A = g.nodeAB[2 * (int64_t)my_node];
+                B = g.nodeAB[2 * (int64_t)my_node + 1];
                 C = g.nodeC[my_node];
                 if (QEARLY) {
                     Q0 = g.nodeQ[2 * (int64_t)my_node];
@@ -962,8 +962,8 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
                         // borderline: decide exactly as subdivp does, in FP64
                         const int jn = __shfl_sync(FULL, my_node, j), jdepth = __shfl_sync(FULL, C.y, j) >> 8;
                         if (edge) {
-                            op = open_exact(g.ncx[jn], g.ncy[jn], g.ncz[jn], xd[0], yd[0], zd[0], g.tol2d,
-                                            g.box->dsq[jdepth]);
+                            const double4_32a nd = g.nodeD[jn];
+                            op = open_exact(nd.x, nd.y, nd.z, xd[0], yd[0], zd[0], g.tol2d, g.box->dsq[jdepth]);
                             nborder++;
                         }
                     }
@@ -1290,13 +1290,10 @@ int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorte
     }
     a.sys_root = self ? c->walk_sys_root : nullptr;
     a.body_sys = c->walk_body_sys;
-    a.nodeA = c->nodeA;
-    a.nodeB = c->nodeB;
+    a.nodeAB = c->nodeAB;
     a.nodeQ = c->nodeQ;
     a.nodeC = c->nodeC;
-    a.ncx = c->ncx;
-    a.ncy = c->ncy;
-    a.ncz = c->ncz;
+    a.nodeD = c->nodeD;
     a.box = c->box;
     a.ntarget = ntarget;
     a.tsorted = tsorted;
@@ -1330,6 +1327,12 @@ int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorte
     // criterion), else 32 consecutive bodies (also the guard's fallback walk)
     const bool per_body = body_rule || c->criterion == HC_CRITERION_BODY;
     a.use_table = (self && (!per_body || (c->criterion == HC_CRITERION_BODY && c->group_kind == 1))) ? 1 : 0;
+    if (a.use_table && !c->have_groups) {
+        // the tree was built for a walk without tree groups; inside a build's
+        // capture this cannot happen (the build makes what its walk uses)
+        hc_groups_launch(c);
+        c->have_groups = true;
+    }
     HC_CUDA(cudaMemsetAsync(a.sp.ctl, 0, sizeof(hc_walk_ctl), c->stream));
     const bool count = c->prm.count_per_body && self && c->cnt_b;
     const int v = (c->prm.usequad ? 2 : 0) + (count ? 1 : 0);
@@ -1490,7 +1493,7 @@ __global__ void __launch_bounds__(128) k_label(WalkArgs g, const int *gstart, co
                 gmaxz = wmax(mxz);
     const float eps2 = g.eps2f;
     auto rel_pos = [&](int k, float &cx, float &cy, float &cz) {
-        const float4 A = g.nodeA[k], B = g.nodeB[k];
+        const float4 A = g.nodeAB[2 * (int64_t)k], B = g.nodeAB[2 * (int64_t)k + 1];
         cx = (A.x - ghx) + (B.x - glx);
         cy = (A.y - ghy) + (B.y - gly);
         cz = (A.z - ghz) + (B.z - glz);
@@ -1583,8 +1586,7 @@ int hc_label_launch(hc_ctx *c, int nsample, float eps_label)
     if (nsample <= 0) return HC_OK;
     WalkArgs a;
     memset(&a, 0, sizeof a);
-    a.nodeA = c->nodeA;
-    a.nodeB = c->nodeB;
+    a.nodeAB = c->nodeAB;
     a.nodeQ = c->nodeQ;
     a.nodeC = c->nodeC;
     a.eps2f = (float)(c->prm.eps * c->prm.eps);

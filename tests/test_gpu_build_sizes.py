@@ -1,0 +1,103 @@
+"""GPU tests of the octree build at the sizes and mixtures where its kernels
+change form: the one-block sort's capacities, tile edges of the sort, the box
+test, the compaction and the node emission, systems with massless bodies (the
+compaction pass) and with many ties of the 63-bit high keys.  The tree is the
+oracle's bit for bit, and a walk on tree groups made after the build gives the
+same counts as one made with it."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hc():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from nemo_gb300 import build as B
+    B.build()
+    from nemo_gb300 import hackcode
+    return hackcode
+
+
+@pytest.fixture(scope="module")
+def O():
+    from oracle import oracle
+    oracle.build(ref=None)
+    return oracle
+
+
+def _bodies(n, kind, seed):
+    rng = np.random.default_rng([seed, n])
+    pos = rng.normal(0.0, 0.7, (n, 3))
+    m = rng.uniform(0.5, 1.5, n) / n
+    if kind == "massless":
+        m[rng.random(n) < 0.3] = 0.0
+        if n > 3:
+            m[:2] = 0.0                          # the first massive body is not the first body
+    elif kind == "ties":                         # pairs and triples far closer than the high keys resolve
+        k = n // 3
+        pos[k:2 * k] = pos[:k] + rng.normal(0.0, 1e-6, (k, 3))
+        pos[2 * k:3 * k] = pos[:k] + rng.normal(0.0, 1e-6, (k, 3))
+    elif kind == "far":                          # many bodies outside the first box
+        pos *= rng.uniform(0.1, 9.0, (n, 1)) ** 2
+    return m, pos
+
+
+def _canon(d):
+    k = np.lexsort((d["corner"][:, 2], d["corner"][:, 1], d["corner"][:, 0], d["level"]))
+    return {f: d[f][k] for f in ("level", "corner", "count", "mass", "cm")}
+
+
+# sort: 1024, 2048, 4096, 8192 per form, 4096 per tile; box 4096, compaction and emission 2048 per tile
+SIZES = [1, 2, 3, 31, 33, 1023, 1024, 1025, 2049, 4096, 4097, 8191, 8192, 8193, 20481]
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("kind", ["plain", "massless", "ties", "far"])
+def test_tree_matches_oracle(hc, O, n, kind):
+    m, pos = _bodies(n, kind, 3)
+    ph = np.zeros((n, 2, 3))
+    ph[:, 0] = pos
+    T = O.Tree(n, 12.0)
+    assert T.build(m, pos, True) == 0
+    ref = T.dump()
+    with hc.Context(n, tol=0.6, eps=0.02, fcells=12.0, usequad=True, count_per_body=True) as ctx:
+        ctx.upload(m, ph)
+        ctx.build_tree()
+        rmin, rsize = ctx.box()
+        assert np.array_equal(rmin, T.box()[0]) and rsize == T.box()[1]
+        c, r = _canon(ctx.dump_tree()), _canon(ref)
+        for f in c:
+            assert np.array_equal(c[f], r[f]), f
+        assert ctx.tree_info().nbody_massive == int((m != 0).sum())
+        _, _, rb, rc = T.forces(0.6, 0.02, True)
+        ctx.forces()
+        b, cc = ctx.body_counts()
+        assert np.array_equal(b, rb) and np.array_equal(cc, rc)
+        ctx.set_grouping("tree")                 # the table is made by the walk: the build had no use for it
+        ctx.forces()
+        b, cc = ctx.body_counts()
+        assert np.array_equal(b, rb) and np.array_equal(cc, rc)
+        ctx.evaluate()                           # made with the build
+        b, cc = ctx.body_counts()
+        assert np.array_equal(b, rb) and np.array_equal(cc, rc)
+
+
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 8192, 8193])
+def test_points_of_any_number(hc, O, n):
+    """Forces at n test points (the sort's forms without ties) equal the oracle's."""
+    m, pos = _bodies(500, "plain", 4)
+    pts = np.random.default_rng(n).normal(0.0, 1.5, (n, 3))
+    ph = np.zeros((500, 2, 3))
+    ph[:, 0] = pos
+    T = O.Tree(500, 2.0)
+    assert T.build(m, pos, True) == 0
+    ra, rp = T.forces(0.6, 0.02, True, test_pos=pts, skip_self=False)[:2]
+    with hc.Context(500, tol=0.6, eps=0.02, usequad=True) as ctx:
+        ctx.upload(m, ph)
+        ctx.build_tree()
+        a, p = ctx.forces_at(pts)
+    assert (np.linalg.norm(a - ra, axis=1) <= 1e-5 * np.linalg.norm(ra, axis=1)).mean() >= 0.999
+    assert (np.abs(p - rp) <= 1e-5 * np.abs(rp)).mean() >= 0.999
