@@ -112,7 +112,7 @@ int alloc_all(hc_ctx *c)
     HC_TRY(dalloc(c, &c->nodeC, mn));
     HC_TRY(dalloc(c, &c->nodeD, mn));
     HC_TRY(dalloc(c, &c->hist, hc_build_scratch_words(n, mn)));
-    HC_TRY(dalloc(c, &c->first2, (n + 4095) / 4096));
+    HC_TRY(dalloc(c, &c->first2, (n + 1023) / 1024));
     HC_TRY(dalloc(c, &c->cand, n));
     HC_TRY(dalloc(c, &c->ncand, 4));
     HC_TRY(dalloc(c, &c->diag_part, 36 * 1024));

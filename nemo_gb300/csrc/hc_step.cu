@@ -11,7 +11,7 @@
 namespace {
 
 constexpr int DIAG_BLOCKS = 304;
-constexpr int DIAG_THREADS = 256;
+constexpr int DIAG_THREADS = 256, DIAG_THREADS_SMALL = 64;
 constexpr int NDIAG = 36;   // KE, PE, keten[9], peten[9], amten_raw[9], m x[3], m v[3], mtot
 
 // v1/2 = v + a dt/2; x += v1/2 dt; v = v1/2 + a dt/2   (code.c:182-188)
@@ -108,7 +108,8 @@ __device__ __forceinline__ double wsum(double v)
 }
 
 // Per-block partial sums in a fixed order (deterministic for a given launch shape).
-__global__ void __launch_bounds__(DIAG_THREADS) k_diag_part(int64_t n, const double *mass, const double *px,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_diag_part(int64_t n, const double *mass, const double *px,
                                                             const double *py, const double *pz, const double *vx,
                                                             const double *vy, const double *vz, const double *ax,
                                                             const double *ay, const double *az, const double *phi,
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag_part(int64_t n, const dou
         // counts the external part once more (hackcode3/code_io.c:180-186)
         hc_diag_body(acc, mass[i], x, v, a, phi_ext ? __dadd_rn(phi[i], phi_ext[i]) : phi[i]);
     }
-    __shared__ double sh[DIAG_THREADS / 32][NDIAG];
+    __shared__ double sh[THREADS / 32][NDIAG];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < NDIAG; q++) {
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag_part(int64_t n, const dou
     __syncthreads();
     if (threadIdx.x < NDIAG) {
         double s = 0.0;
-        for (int w = 0; w < DIAG_THREADS / 32; w++) s += sh[w][threadIdx.x];
+        for (int w = 0; w < THREADS / 32; w++) s += sh[w][threadIdx.x];
         part[(int64_t)blockIdx.x * NDIAG + threadIdx.x] = s;
     }
 }
@@ -257,11 +258,16 @@ void hc_extpot_launch(hc_ctx *c, double kick_dthf, int64_t nstep)
 // out36 (device): KE, PE, keten, peten, amten(raw), sum m x, sum m v, mtot
 void hc_diag_launch(hc_ctx *c, double *out36)
 {
-    int nb = (int)std::min<int64_t>(DIAG_BLOCKS, (c->n + DIAG_THREADS - 1) / DIAG_THREADS);
+    // Small systems: a body per thread in blocks of two warps, on as many SMs as
+    // possible: each warp's 36 FP64 reductions hold its SM's FP64 pipe for
+    // 3000 cycles (4096 bodies: 23 us with blocks of eight warps).
+    const bool small = c->n <= DIAG_BLOCKS * DIAG_THREADS_SMALL;
+    const int threads = small ? DIAG_THREADS_SMALL : DIAG_THREADS;
+    int nb = (int)std::min<int64_t>(DIAG_BLOCKS, (c->n + threads - 1) / threads);
     if (nb < 1) nb = 1;
-    k_diag_part<<<nb, DIAG_THREADS, 0, c->stream>>>(c->n, c->mass, c->px, c->py, c->pz, c->vx, c->vy, c->vz, c->ax,
-                                                    c->ay, c->az, c->phi, c->extpot ? c->phi_ext : nullptr,
-                                                    c->diag_part);
+    auto *part = small ? k_diag_part<DIAG_THREADS_SMALL> : k_diag_part<DIAG_THREADS>;
+    part<<<nb, threads, 0, c->stream>>>(c->n, c->mass, c->px, c->py, c->pz, c->vx, c->vy, c->vz, c->ax, c->ay, c->az,
+                                        c->phi, c->extpot ? c->phi_ext : nullptr, c->diag_part);
     k_diag_final<<<1, 64, 0, c->stream>>>(c->diag_part, nb, out36);
     c->launches += 2;
 }

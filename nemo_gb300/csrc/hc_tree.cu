@@ -108,12 +108,17 @@ __device__ __forceinline__ int2 warp_min2(int2 v)
 // small fraction of the FP32 rate); the rest take it.  One pass: a tile's place
 // in the list comes from decoupled look-back (as three kernels -- flags, scan,
 // compaction -- this took 21 + 13 + 5 us at N = 2^20 and two more launches).
-constexpr int BOX_ITEMS = 16, BOX_TILE = 256 * BOX_ITEMS;
+// Tiles of 1024 bodies up to 2^18, of 4096 above (4096 bodies: 15 -> 8 us; at
+// 2^20 the larger tile is 4 us faster).
+constexpr int BOX_SMALL = 1 << 18;
+static inline int box_items(int64_t n) { return n <= BOX_SMALL ? 4 : 16; }
+template <int BOX_ITEMS>
 __global__ void __launch_bounds__(256) k_box_outside(const double *mass, const double *px, const double *py,
                                                      const double *pz, int64_t n, const hc_box *box, int32_t *cand,
                                                      int32_t *ncand, int2 *first2, uint32_t *status, uint32_t *ctr,
                                                      int *err)
 {
+    constexpr int BOX_TILE = 256 * BOX_ITEMS;
     __shared__ int2 wf[8];
     __shared__ uint32_t wsum[8], s_tile, s_prefix;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -721,115 +726,187 @@ __global__ void __launch_bounds__(256) k_cell_place(const int2 *nodeC, const hc_
     }
 }
 
-__device__ __forceinline__ void prefetch_l1(const void *p)
+// hackcofm (load.c:183-226), deepest level first.  Children are summed in
+// subindex order exactly as hackcofm does.
+//
+// Bound by the dependent chain of a cell (children's loads, FP64 sums,
+// divisions, records) at every level, and by the FP64 pipe at levels of 10^5
+// cells.  So the two halves of the work run beside each other on warps of their
+// own: in one step the FP64 half (mass and centre of mass) of level D, and the
+// FP32 half (quadrupole, extent, body count) of level D + 1, which reads what
+// the step before wrote.  Levels with few cells give each cell four lanes (x,
+// y, z, mass), so that its three divisions run at once; with many cells one
+// lane a cell does a third less work on the FP64 pipe.  One warp doing both
+// halves of a cell one after the other took 119 us at 50,021 bodies (now 78),
+// 243 at 2^20 (206) and 543 at 2^22 (537, bound by the FP64 pipe).  Four lanes
+// a cell in the FP32 half too, or fewer children in flight, were slower.
+
+// mass and centre of mass, one lane per cell; load.c:193-224, bit-exact
+__device__ __forceinline__ void cofm_mass(int4 P, float dsqf, double4_32a *nodeD, float4 *nodeAB)
 {
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+    const int k = P.x, fc = P.y, nc = P.z & 255;
+    double m = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+        // the children's loads are issued together (predicated on the child
+        // count), not one dependent round trip per child
+        double4_32a c[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (h + i < nc) c[i] = nodeD[fc + h + i];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (h + i < nc) {
+                m = dadd(m, c[i].w);
+                cx = dadd(cx, dmul(c[i].x, c[i].w));
+                cy = dadd(cy, dmul(c[i].y, c[i].w));
+                cz = dadd(cz, dmul(c[i].z, c[i].w));
+            }
+        }
+    }
+    cx = ddiv(cx, m);
+    cy = ddiv(cy, m);
+    cz = ddiv(cz, m);
+    float4 A, B;
+    split_hilo(cx, &A.x, &B.x);
+    split_hilo(cy, &A.y, &B.y);
+    split_hilo(cz, &A.z, &B.z);
+    A.w = hc_d2f_rn(m);
+    B.w = dsqf;
+    nodeD[k] = make_double4_32a(cx, cy, cz, m);
+    nodeAB[2 * (int64_t)k] = A;
+    nodeAB[2 * (int64_t)k + 1] = B;
 }
 
-// hackcofm (load.c:183-226), all levels, deepest first, one grid barrier
-// per level.  Children are summed in subindex order exactly as hackcofm does.
+// the same with four lanes per cell: lane q = 0, 1, 2 the coordinates, 3 the mass
+__device__ __forceinline__ void cofm_mass4(int4 P, int q, float dsqf, double *nodeD, float *nodeAB)
+{
+    const int64_t k = P.x;
+    const int nc = P.z & 255;
+    const double *c = nodeD + 4 * (int64_t)P.y;
+    double cm[8], cq[8], m = 0.0, v = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        if (i < nc) {
+            cm[i] = c[4 * i + 3];
+            cq[i] = c[4 * i + q];
+        }
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        if (i < nc) {
+            m = dadd(m, cm[i]);
+            v = dadd(v, dmul(cq[i], cm[i]));
+        }
+    float hi, lo;
+    if (q < 3) {
+        v = ddiv(v, m);
+        split_hilo(v, &hi, &lo);
+    } else {
+        v = m;
+        hi = hc_d2f_rn(m);
+        lo = dsqf;
+    }
+    nodeD[4 * k + q] = v;
+    nodeAB[8 * k + q] = hi;
+    nodeAB[8 * k + 4 + q] = lo;
+}
+
+// Quadrupole, extent and body count of a cell.  Children's offsets from the
+// centre of mass in FP32, from the hi + lo positions ((hi - hi) + (lo - lo)):
+// no FP64 work per child.  bmax: children's extents shifted to the new centre;
+// Q = sum_child [ m (3 dr dr^T - |dr|^2 I) + Q_child ], dr = x_child - x_cm.
+__device__ __forceinline__ void cofm_quad(int4 P, int usequad, const float4 *nodeAB, float4 *nodeQ)
+{
+    const int k = P.x, fc = P.y, nc = P.z & 255;
+    const float4 A = nodeAB[2 * (int64_t)k], B = nodeAB[2 * (int64_t)k + 1];
+    float bmax = 0.f, nbody = 0.f;
+    float Q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+        float4 ca[4], cb[4], q0[4], q1[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t ch = 2 * (int64_t)(fc + h + i);
+            if (h + i < nc) {
+                ca[i] = nodeAB[ch];
+                cb[i] = nodeAB[ch + 1];
+                q1[i] = nodeQ[ch + 1];
+                if (usequad) q0[i] = nodeQ[ch];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (h + i >= nc) continue;
+            const float dx = (ca[i].x - A.x) + (cb[i].x - B.x), dy = (ca[i].y - A.y) + (cb[i].y - B.y),
+                        dz = (ca[i].z - A.z) + (cb[i].z - B.z);
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            bmax = fmaxf(bmax, sqrtf(r2) + q1[i].w);
+            nbody += q1[i].z;                // bodies in the cell (exact below 2^24)
+            if (usequad) {
+                const float mr = ca[i].w;
+                Q[0] += mr * (3.f * dx * dx - r2) + q0[i].x;
+                Q[1] += mr * (3.f * dx * dy) + q0[i].y;
+                Q[2] += mr * (3.f * dx * dz) + q0[i].z;
+                Q[3] += mr * (3.f * dy * dy - r2) + q0[i].w;
+                Q[4] += mr * (3.f * dy * dz) + q1[i].x;
+                Q[5] += mr * (3.f * dz * dz - r2) + q1[i].y;
+            }
+        }
+    }
+    nodeQ[2 * (int64_t)k] = make_float4(Q[0], Q[1], Q[2], Q[3]);
+    nodeQ[2 * (int64_t)k + 1] = make_float4(Q[4], Q[5], nbody, bmax);
+}
+
+// One step: w of nw warps works on its half's level (mass: level D, else D + 1).
+// Consecutive 32-cell chunks go to consecutive warps, which the callers number
+// so that they sit on different SMs.
+__device__ __forceinline__ void cofm_step(bool mass, int D, int maxd, int w, int nw, int usequad, const hc_box *box,
+                                          double4_32a *nodeD, float4 *nodeAB, float4 *nodeQ, const int4 *cperm,
+                                          const uint32_t *coff)
+{
+    const int L = mass ? D : D + 1, lane = (int)(threadIdx.x & 31);
+    if (L < 0 || L > maxd) return;
+    // the level's cells only, grouped by child count (coff: group offsets)
+    const int ls = (int)coff[L * 8], le = (int)coff[L * 8 + 8];
+    const float dsqf = hc_d2f_rn(box->dsq[L]);
+    if (!mass) {
+        for (int j = ls + w * 32 + lane; j < le; j += nw * 32) cofm_quad(cperm[j], usequad, nodeAB, nodeQ);
+    } else if (le - ls <= nw * 8) {
+        const int j = ls + w * 8 + (lane >> 2);
+        if (j < le) cofm_mass4(cperm[j], lane & 3, dsqf, reinterpret_cast<double *>(nodeD), reinterpret_cast<float *>(nodeAB));
+    } else {
+        for (int j = ls + w * 32 + lane; j < le; j += nw * 32) cofm_mass(cperm[j], dsqf, nodeD, nodeAB);
+    }
+}
+
 __global__ void __launch_bounds__(256, 2) k_cofm_all(int usequad, const hc_box *box, double4_32a *nodeD, float4 *nodeAB,
                                                      float4 *nodeQ, const int4 *cperm, const uint32_t *coff)
 {
     cg::grid_group grid = cg::this_grid();
-    const int maxd = box->nnode > 0 ? box->max_depth : -1;
-    // A warp takes 32 consecutive cells of a level (one child-count group,
-    // so its FP64 child loop is uniform); consecutive 32-cell chunks go to
-    // consecutive blocks, which sit on different SMs.  A level of a few
-    // thousand cells then spreads over the whole GPU instead of crowding
-    // the FP64 units of the first few SMs.
-    const int nwarps = (int)(grid.size() >> 5);
-    const int wrank = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
-    const int lane = (int)(threadIdx.x & 31);
-    for (int D = maxd; D >= 0; D--) {
-        // the level's cells only, grouped by child count (coff: group offsets)
-        const int ls = (int)coff[D * 8], le = (int)coff[D * 8 + 8];
-        const float dsqf = __double2float_rn(box->dsq[D]);
-        for (int j = ls + wrank * 32 + lane; j < le; j += nwarps * 32) {
-            // the cell with its child links in one load (one dependent round trip less)
-            const int4 P = cperm[j];
-            const int k = P.x, fc = P.y, nc = P.z & 255;
-            // the children's FP32 node data are needed after the FP64 sums: start
-            // bringing their lines into L1 now, beside the FP64 loads
-            prefetch_l1(nodeAB + 2 * (int64_t)fc);
-            prefetch_l1(nodeAB + 2 * (int64_t)(fc + nc) - 1);
-            prefetch_l1(nodeQ + 2 * (int64_t)fc);
-            prefetch_l1(nodeQ + 2 * (int64_t)(fc + nc) - 1);
-            // The children's loads are issued together (predicated on the
-            // child count), not one dependent round trip per child.  FP64 mass
-            // and first moments in hackcofm's order (load.c:193-224; bit-exact).
-            double m = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
-#pragma unroll
-            for (int h = 0; h < 8; h += 4) {
-                double4_32a c[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (h + i < nc) c[i] = nodeD[fc + h + i];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (h + i < nc) {
-                        m = dadd(m, c[i].w);
-                        cx = dadd(cx, dmul(c[i].x, c[i].w));
-                        cy = dadd(cy, dmul(c[i].y, c[i].w));
-                        cz = dadd(cz, dmul(c[i].z, c[i].w));
-                    }
-                }
-            }
-            cx = ddiv(cx, m);
-            cy = ddiv(cy, m);
-            cz = ddiv(cz, m);
-            float4 A, B;
-            split_hilo(cx, &A.x, &B.x);
-            split_hilo(cy, &A.y, &B.y);
-            split_hilo(cz, &A.z, &B.z);
-            // children's offsets from the centre of mass in FP32, from the
-            // hi + lo positions ((hi - hi) + (lo - lo)): no FP64 work per child.
-            // bmax: children's extents shifted to the new centre; Q = sum_child
-            // [ m (3 dr dr^T - |dr|^2 I) + Q_child ], dr = x_child - x_cm.
-            // Four children at a time, their loads in flight together.
-            float bmax = 0.f, nbody = 0.f;
-            float Q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int h = 0; h < 8; h += 4) {
-                float4 ca[4], cb[4], q0[4], q1[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int64_t ch = 2 * (int64_t)(fc + h + i);
-                    if (h + i < nc) {
-                        ca[i] = nodeAB[ch];
-                        cb[i] = nodeAB[ch + 1];
-                        q1[i] = nodeQ[ch + 1];
-                        if (usequad) q0[i] = nodeQ[ch];
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (h + i >= nc) continue;
-                    const float dx = (ca[i].x - A.x) + (cb[i].x - B.x), dy = (ca[i].y - A.y) + (cb[i].y - B.y),
-                                dz = (ca[i].z - A.z) + (cb[i].z - B.z);
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    bmax = fmaxf(bmax, sqrtf(r2) + q1[i].w);
-                    nbody += q1[i].z;                // bodies in the cell (exact below 2^24)
-                    if (usequad) {
-                        const float mr = ca[i].w;
-                        Q[0] += mr * (3.f * dx * dx - r2) + q0[i].x;
-                        Q[1] += mr * (3.f * dx * dy) + q0[i].y;
-                        Q[2] += mr * (3.f * dx * dz) + q0[i].z;
-                        Q[3] += mr * (3.f * dy * dy - r2) + q0[i].w;
-                        Q[4] += mr * (3.f * dy * dz) + q1[i].x;
-                        Q[5] += mr * (3.f * dz * dz - r2) + q1[i].y;
-                    }
-                }
-            }
-            nodeD[k] = make_double4_32a(cx, cy, cz, m);
-            A.w = hc_d2f_rn(m);
-            B.w = dsqf;
-            nodeAB[2 * (int64_t)k] = A;
-            nodeAB[2 * (int64_t)k + 1] = B;
-            nodeQ[2 * (int64_t)k] = make_float4(Q[0], Q[1], Q[2], Q[3]);
-            nodeQ[2 * (int64_t)k + 1] = make_float4(Q[4], Q[5], nbody, bmax);
-        }
-        grid.sync();
+    const int maxd = box->nnode > 0 ? box->max_depth : -1, wid = (int)(threadIdx.x >> 5);
+    const int w = (wid >> 1) * (int)gridDim.x + (int)blockIdx.x, nw = (int)(blockDim.x >> 6) * (int)gridDim.x;
+    for (int D = maxd; D >= -1; D--) {
+        cofm_step(!(wid & 1), D, maxd, w, nw, usequad, box, nodeD, nodeAB, nodeQ, cperm, coff);
+        if (D >= 0) grid.sync();
+    }
+}
+
+// The same for small systems in one cluster of eight blocks: a cluster barrier
+// per level instead of the grid's, and registers for all of a cell's loads
+// (128 bodies: 68 -> 33 us, 4096: 103 -> 61).  Above COFM_SMALL eight SMs' FP64
+// pipes would take longer than the grid's barriers cost.
+constexpr int COFM_CLUSTER = 8, COFM_SMALL = 16384, COFM_THREADS = 256;
+__global__ void __cluster_dims__(COFM_CLUSTER, 1, 1) __launch_bounds__(COFM_THREADS, 1)
+    k_cofm_small(int usequad, const hc_box *box, double4_32a *nodeD, float4 *nodeAB, float4 *nodeQ, const int4 *cperm,
+                 const uint32_t *coff)
+{
+    cg::cluster_group cluster = cg::this_cluster();
+    const int maxd = box->nnode > 0 ? box->max_depth : -1, wid = (int)(threadIdx.x >> 5);
+    const int w = (wid >> 1) * COFM_CLUSTER + (int)blockIdx.x;
+    for (int D = maxd; D >= -1; D--) {
+        cofm_step(!(wid & 1), D, maxd, w, COFM_THREADS / 64 * COFM_CLUSTER, usequad, box, nodeD, nodeAB, nodeQ, cperm,
+                  coff);
+        if (D >= 0) cluster.sync();
     }
 }
 
@@ -891,45 +968,57 @@ __device__ __forceinline__ int node_packs(const uint32_t *ba, const float4 *node
 }
 
 // The group table in node order, in one pass (decoupled look-back over tiles of
-// four nodes per thread).
+// GI rounds of 256 consecutive nodes).
 constexpr int GI = 4, GTILE = 256 * GI;
 __global__ void __launch_bounds__(256) k_groups(const uint32_t *ba, const float4 *nodeQ, const int2 *nodeC, hc_box *box,
                                                 int gmax, int32_t *gstart, int32_t *gcount, uint32_t *status,
                                                 uint32_t *ctr, int *err)
 {
-    __shared__ uint32_t s_tile, s_prefix, sh[32];
+    __shared__ uint32_t s_tile, s_prefix, wsum[GI][8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_tile = atomicAdd(ctr, 1u);
     __syncthreads();
-    const int64_t tile = s_tile, base = tile * GTILE + threadIdx.x * GI;
+    const int64_t tile = s_tile, base = tile * GTILE + threadIdx.x;
     const int nn = box->nnode;
     if (tile * GTILE >= nn) {
         if (tile == 0 && threadIdx.x == 0) box->ngroups = 0;
         return;
     }
-    uint32_t n = 0;
+    uint32_t n[GI], ex[GI];
 #pragma unroll
-    for (int i = 0; i < GI; i++)
-        if (base + i < nn) n += node_packs(ba, nodeQ, nodeC, (int)base + i, gmax, [](int, int) {});
-    uint32_t agg;
-    const uint32_t ex = block_exclusive_scan<uint32_t>(n, sh, &agg);
-    if (threadIdx.x < 32) {
+    for (int r = 0; r < GI; r++) {
+        const int64_t k = base + r * 256;
+        n[r] = k < nn ? (uint32_t)node_packs(ba, nodeQ, nodeC, (int)k, gmax, [](int, int) {}) : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < GI; r++) {
+        const uint32_t incl = warp_inclusive_scan(n[r]);
+        ex[r] = incl - n[r];
+        if (lane == 31) wsum[r][wid] = incl;
+    }
+    __syncthreads();
+    if (wid == 0) {                            // GI * 8 sums, one per lane, in node order
+        static_assert(GI * 8 == 32, "one warp scans the warps' sums");
+        const uint32_t v = (&wsum[0][0])[lane], incl = warp_inclusive_scan(v);
+        const uint32_t agg = __shfl_sync(0xffffffffu, incl, 31);
+        (&wsum[0][0])[lane] = incl - v;
         const uint32_t prefix = tile_prefix(status, tile, agg, err);
-        if (threadIdx.x == 0) {
+        if (lane == 0) {
             s_prefix = prefix;
             if ((tile + 1) * GTILE >= nn) box->ngroups = (int)(prefix + agg);    // the last tile
         }
     }
     __syncthreads();
-    if (n == 0) return;
-    uint32_t out = s_prefix + ex;
 #pragma unroll
-    for (int i = 0; i < GI; i++)
-        if (base + i < nn)
-            node_packs(ba, nodeQ, nodeC, (int)base + i, gmax, [&](int first, int cnt) {
-                gstart[out] = first;
-                gcount[out] = cnt;
-                out++;
-            });
+    for (int r = 0; r < GI; r++) {
+        if (n[r] == 0) continue;
+        uint32_t out = s_prefix + wsum[r][wid] + ex[r];
+        node_packs(ba, nodeQ, nodeC, (int)(base + r * 256), gmax, [&](int first, int cnt) {
+            gstart[out] = first;
+            gcount[out] = cnt;
+            out++;
+        });
+    }
 }
 
 // ---------------- treecode1 critical radii ----------------
@@ -1020,7 +1109,7 @@ BuildScratch build_scratch(uint32_t *p, int64_t n, int64_t maxnode)
     b.gcount = take(256);
     b.gcur = take(256);
     b.goff = take(257);
-    b.box = take((n + BOX_TILE - 1) / BOX_TILE);
+    b.box = take((n + 1023) / 1024);
     b.massive = take((n + MC_TILE - 1) / MC_TILE);
     b.emit = take((n + TB - 1) / TB * 32);
     b.groups = take((maxnode + GTILE - 1) / GTILE);
@@ -1056,8 +1145,9 @@ int hc_tree_build(hc_ctx *c)
     HC_CUDA(cudaMemsetAsync(c->hist, 0, sizeof(uint32_t) * b.words, s));
 
     // 1. expandbox replay
-    const int boxtiles = (int)((n + BOX_TILE - 1) / BOX_TILE);
-    k_box_outside<<<boxtiles, B, 0, s>>>(c->mass, c->px, c->py, c->pz, n, c->box, c->cand, c->ncand, c->first2, b.box,
+    const int boxtile = 256 * box_items(n), boxtiles = (int)((n + boxtile - 1) / boxtile);
+    auto *box_outside = box_items(n) == 4 ? k_box_outside<4> : k_box_outside<16>;
+    box_outside<<<boxtiles, B, 0, s>>>(c->mass, c->px, c->py, c->pz, n, c->box, c->cand, c->ncand, c->first2, b.box,
                                          b.ctr, &c->st->error);
     k_box_replay<<<1, 256, 0, s>>>(c->px, c->py, c->pz, c->cand, c->ncand, c->first2, boxtiles, c->box, c->st,
                                    c->all_massive ? (int)n : -1);
@@ -1100,7 +1190,10 @@ int hc_tree_build(hc_ctx *c)
         c->join_pending = false;
         HC_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
     }
-    {
+    if (n <= COFM_SMALL) {
+        k_cofm_small<<<COFM_CLUSTER, COFM_THREADS, 0, s>>>(c->prm.usequad, c->box, c->nodeD, c->nodeAB, c->nodeQ, c->cperm, b.goff);
+        c->launches++;
+    } else {
         int usequad = c->prm.usequad;
         uint32_t *goff = b.goff;
         void *args[] = {&usequad, &c->box, &c->nodeD, &c->nodeAB, &c->nodeQ, &c->cperm, &goff};
