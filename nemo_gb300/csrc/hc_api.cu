@@ -35,11 +35,9 @@ int dalloc(hc_ctx *c, T **p, int64_t count)
         if (r_ != HC_OK) return r_; \
     } while (0)
 
-int check_status(hc_ctx *c)
+// The device status already copied to c->h_st (the stream is synchronised).
+int status_result(hc_ctx *c)
 {
-    HC_CUDA(cudaMemcpyAsync(c->h_st, c->st, sizeof(hc_status), cudaMemcpyDeviceToHost, c->stream));
-    HC_CUDA(cudaStreamSynchronize(c->stream));
-    HC_CUDA(cudaGetLastError());
     const hc_status &s = *c->h_st;
     if (s.error == 0) return HC_OK;
     char buf[256];
@@ -58,6 +56,14 @@ int check_status(hc_ctx *c)
     }
     c->err = buf;
     return s.error;
+}
+
+int check_status(hc_ctx *c)
+{
+    HC_CUDA(cudaMemcpyAsync(c->h_st, c->st, sizeof(hc_status), cudaMemcpyDeviceToHost, c->stream));
+    HC_CUDA(cudaStreamSynchronize(c->stream));
+    HC_CUDA(cudaGetLastError());
+    return status_result(c);
 }
 
 void free_all(hc_ctx *c)
@@ -132,32 +138,38 @@ int alloc_all(hc_ctx *c)
         HC_CUDA(cudaMemset(pk, 0, sizeof(MlpSmem)));
     }
     HC_TRY(dalloc(c, &c->sample_count, 2));
-    {
-        // split walks (outlying groups only): sized for some 10^4 parts, less for small systems
-        hc_walk_split &w = c->split;
-        const int64_t small = std::max<int64_t>(64, n);
-        w.out_cap = (int)small;
-        w.slot_cap[0] = (int)std::min<int64_t>(4096, small);
-        w.slot_cap[1] = (int)std::min<int64_t>(16384, small);
-        w.entry_cap[0] = (int)std::min<int64_t>(65536, 16 * small);
-        w.entry_cap[1] = (int)std::min<int64_t>(262144, 16 * small);
-        w.slot0[0] = 0;
-        w.slot0[1] = w.slot_cap[0];
-        const int64_t slots = w.slot_cap[0] + (int64_t)w.slot_cap[1];
-        HC_TRY(dalloc(c, &w.ctl, 1));
-        HC_TRY(dalloc(c, &w.out, w.out_cap));
-        for (int k = 0; k < 2; k++) {
-            HC_TRY(dalloc(c, &w.task[k], w.slot_cap[k]));
-            HC_TRY(dalloc(c, &w.entry[k], w.entry_cap[k]));
-        }
-        HC_TRY(dalloc(c, &w.group, w.slot_cap[0]));
-        HC_TRY(dalloc(c, &w.sub, w.slot_cap[0]));
-        HC_TRY(dalloc(c, &w.part, 2 * slots * HC_GROUP2));
-        HC_TRY(dalloc(c, &w.part_cnt, slots * HC_GROUP2));
-    }
+    HC_TRY(dalloc(c, &c->split.ctl, 1));
     HC_TRY(dalloc(c, &c->box, 1));
     HC_CUDA(cudaMallocHost((void **)&c->h_st, sizeof(hc_status)));
     HC_CUDA(cudaMallocHost((void **)&c->h_box, sizeof(hc_box)));
+    return HC_OK;
+}
+
+// Buffers of split walks (outlying groups under the group criteria), once per
+// context: sized for some 10^4 parts, less for small systems.
+int ensure_split(hc_ctx *c)
+{
+    hc_walk_split &w = c->split;
+    if (w.out_cap > 0) return HC_OK;
+    const int64_t small = std::max<int64_t>(64, c->n);
+    w.slot_cap[0] = (int)std::min<int64_t>(4096, small);
+    w.slot_cap[1] = (int)std::min<int64_t>(16384, small);
+    w.entry_cap[0] = (int)std::min<int64_t>(65536, 16 * small);
+    w.entry_cap[1] = (int)std::min<int64_t>(262144, 16 * small);
+    w.slot0[0] = 0;
+    w.slot0[1] = w.slot_cap[0];
+    const int64_t slots = w.slot_cap[0] + (int64_t)w.slot_cap[1];
+    auto once = [&](auto **p, int64_t count) { return *p ? HC_OK : dalloc(c, p, count); };   // after a failure
+    HC_TRY(once(&w.out, small));
+    for (int k = 0; k < 2; k++) {
+        HC_TRY(once(&w.task[k], w.slot_cap[k]));
+        HC_TRY(once(&w.entry[k], w.entry_cap[k]));
+    }
+    HC_TRY(once(&w.group, w.slot_cap[0]));
+    HC_TRY(once(&w.sub, w.slot_cap[0]));
+    HC_TRY(once(&w.part, 2 * slots * HC_GROUP2));
+    HC_TRY(once(&w.part_cnt, slots * HC_GROUP2));
+    w.out_cap = (int)small;              // from here on walks may split
     return HC_OK;
 }
 
@@ -222,6 +234,31 @@ __global__ void k_pack3(const double *x, const double *y, const double *z, int64
     }
 }
 
+// [n][2][3] positions and velocities, [n][3] accelerations and [n] potentials,
+// whichever are asked for, in one pass into one buffer
+__global__ void k_pack_state(int64_t n, const double *px, const double *py, const double *pz, const double *vx,
+                             const double *vy, const double *vz, const double *ax, const double *ay, const double *az,
+                             const double *phi, double *ophase, double *oacc, double *ophi)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (ophase) {
+            double *q = ophase + 6 * i;
+            q[0] = px[i];
+            q[1] = py[i];
+            q[2] = pz[i];
+            q[3] = vx[i];
+            q[4] = vy[i];
+            q[5] = vz[i];
+        }
+        if (oacc) {
+            oacc[3 * i] = ax[i];
+            oacc[3 * i + 1] = ay[i];
+            oacc[3 * i + 2] = az[i];
+        }
+        if (ophi) ophi[i] = phi[i];
+    }
+}
+
 __global__ void k_unpack3(const double *in, int64_t n, double *x, double *y, double *z)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -256,6 +293,11 @@ struct GraphSlot {
     int64_t launches = 0;
 };
 
+// Downloads of at most this many doubles (1 MB) go through a page-locked buffer
+// of the context: one copy over the link instead of one through the driver's
+// staging per array.
+constexpr int64_t HC_SMALL_COPY = 1 << 17;
+
 struct hc_ctx_ext : hc_ctx {
     Staging stage;
     Staging stage_acc;            // hc_evaluate_host: previous accelerations
@@ -266,6 +308,7 @@ struct hc_ctx_ext : hc_ctx {
     cudaEvent_t ev_acc = nullptr;
     bool use_graphs = true;
     double *h_diag = nullptr;     // pinned
+    double *h_small = nullptr;    // pinned, up to HC_SMALL_COPY doubles after h_diag: small downloads
     double *d_diag = nullptr;
     int64_t *d_idx = nullptr;
     int64_t idx_cap = 0;
@@ -323,7 +366,8 @@ int hc_create(hc_ctx **out, int64_t nbody, const hc_params *params)
     b.chain_lmax = b.chain_lmin = -1;
     HC_CUDA(cudaMemcpy(c->box, &b, sizeof b, cudaMemcpyHostToDevice));
     HC_CUDA(cudaMemset(c->st, 0, 2 * sizeof(hc_status)));
-    HC_CUDA(cudaMallocHost((void **)&c->h_diag, 64 * sizeof(double)));
+    HC_CUDA(cudaMallocHost((void **)&c->h_diag, (64 + std::min<int64_t>(10 * c->n, HC_SMALL_COPY)) * sizeof(double)));
+    c->h_small = c->h_diag + 64;
     HC_TRY(hc_guard_setup(c));
     int r2 = hc_tree_setup(c);
     return r2 != HC_OK ? r2 : hc_walk_setup(c);
@@ -574,26 +618,44 @@ int hc_forces_at(hc_ctx *ctx, const double *test_pos, int64_t ntest, double *acc
     return HC_OK;
 }
 
+// The state packed on the device and its copies to the host, enqueued; when
+// they have been waited for, finish_download hands small ones on.
+static int enqueue_download(hc_ctx_ext *c, double *phase, double *acc, double *phi)
+{
+    const int64_t n = c->n, np = phase ? 6 * n : 0, na = acc ? 3 * n : 0, nf = phi ? n : 0, total = np + na + nf;
+    if (total == 0) return HC_OK;
+    HC_TRY(staging(c, c->stage, total));
+    double *d = c->stage.d;
+    k_pack_state<<<hc_grid(n, 256), 256, 0, c->stream>>>(n, c->px, c->py, c->pz, c->vx, c->vy, c->vz, c->ax, c->ay, c->az,
+                                                         c->phi, phase ? d : nullptr, acc ? d + np : nullptr,
+                                                         phi ? d + np + na : nullptr);
+    if (total <= HC_SMALL_COPY) {
+        HC_CUDA(cudaMemcpyAsync(c->h_small, d, sizeof(double) * total, cudaMemcpyDeviceToHost, c->stream));
+        return HC_OK;
+    }
+    if (phase) HC_CUDA(cudaMemcpyAsync(phase, d, sizeof(double) * np, cudaMemcpyDeviceToHost, c->stream));
+    if (acc) HC_CUDA(cudaMemcpyAsync(acc, d + np, sizeof(double) * na, cudaMemcpyDeviceToHost, c->stream));
+    if (phi) HC_CUDA(cudaMemcpyAsync(phi, d + np + na, sizeof(double) * nf, cudaMemcpyDeviceToHost, c->stream));
+    return HC_OK;
+}
+
+static void finish_download(hc_ctx_ext *c, double *phase, double *acc, double *phi)
+{
+    const int64_t n = c->n, np = phase ? 6 * n : 0, na = acc ? 3 * n : 0, nf = phi ? n : 0;
+    if (np + na + nf > HC_SMALL_COPY) return;
+    if (phase) std::memcpy(phase, c->h_small, sizeof(double) * np);
+    if (acc) std::memcpy(acc, c->h_small + np, sizeof(double) * na);
+    if (phi) std::memcpy(phi, c->h_small + np + na, sizeof(double) * nf);
+}
+
 int hc_download(hc_ctx *ctx, double *phase, double *acc, double *phi)
 {
     if (!ctx) return HC_ERR_ARG;
     hc_ctx_ext *c = static_cast<hc_ctx_ext *>(ctx);
-    const int64_t n = c->n;
-    HC_TRY(staging(c, c->stage, 6 * n));
-    if (phase) {
-        k_pack3<<<hc_grid(n, 256), 256, 0, c->stream>>>(c->px, c->py, c->pz, n, c->stage.d, 6, 0);
-        k_pack3<<<hc_grid(n, 256), 256, 0, c->stream>>>(c->vx, c->vy, c->vz, n, c->stage.d, 6, 3);
-        HC_CUDA(cudaMemcpyAsync(phase, c->stage.d, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, c->stream));
-        HC_CUDA(cudaStreamSynchronize(c->stream));
-    }
-    if (acc) {
-        k_pack3<<<hc_grid(n, 256), 256, 0, c->stream>>>(c->ax, c->ay, c->az, n, c->stage.d, 3, 0);
-        HC_CUDA(cudaMemcpyAsync(acc, c->stage.d, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream));
-        HC_CUDA(cudaStreamSynchronize(c->stream));
-    }
-    if (phi) HC_CUDA(cudaMemcpyAsync(phi, c->phi, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+    HC_TRY(enqueue_download(c, phase, acc, phi));
     HC_CUDA(cudaStreamSynchronize(c->stream));
     HC_CUDA(cudaGetLastError());
+    finish_download(c, phase, acc, phi);
     return HC_OK;
 }
 
@@ -694,9 +756,10 @@ static int enqueue_evaluation(hc_ctx_ext *c, double kick_dthf, int64_t nstep, bo
 
 static int finish_evaluation(hc_ctx_ext *c)
 {
+    // the evaluation's last node copied the status word
     HC_CUDA(cudaStreamSynchronize(c->stream));
     HC_CUDA(cudaGetLastError());
-    int r = check_status(c);
+    int r = status_result(c);
     if (r != HC_OK) return r;
     HC_CUDA(cudaEventElapsedTime(&c->build_ms, c->ev[0], c->ev[1]));
     HC_CUDA(cudaEventElapsedTime(&c->walk_ms, c->ev[2], c->ev[3]));
@@ -826,11 +889,13 @@ int hc_step(hc_ctx *ctx, double dt, int64_t nstep, hc_diag *diag, double *snap_p
         HC_TRY(finish_evaluation(c));
     }
     if (diag) unpack_diag(c, c->h_diag, diag);
-    if (snap_phase || snap_acc || snap_phi) HC_TRY(hc_download(c, snap_phase, snap_acc, snap_phi));
+    // the snapshot is packed before the drift; both are waited for together
+    HC_TRY(enqueue_download(c, snap_phase, snap_acc, snap_phi));
     hc_kick_drift(c, dt);
     c->launches++;
     HC_CUDA(cudaStreamSynchronize(c->stream));
     HC_CUDA(cudaGetLastError());
+    finish_download(c, snap_phase, snap_acc, snap_phi);
     c->have_tree = false;
     return HC_OK;
 }
@@ -870,6 +935,7 @@ int hc_set_criterion(hc_ctx *ctx, int criterion, double theta)
     if (criterion != HC_CRITERION_BODY && !(theta >= 0.0)) return HC_ERR_ARG;
     hc_ctx_ext *c = static_cast<hc_ctx_ext *>(ctx);
     if (criterion >= HC_CRITERION_BH86 && !c->rcrit2) HC_TRY(dalloc(c, &c->rcrit2, c->maxnode));
+    if (criterion != HC_CRITERION_BODY) HC_TRY(ensure_split(c));
     c->criterion = criterion;
     c->group_theta = theta;
     for (auto &g : c->graphs)        // captured graphs bake the walk variant

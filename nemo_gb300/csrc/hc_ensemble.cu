@@ -331,6 +331,35 @@ __global__ void k_unpack_sys(const double *phase, int64_t n, double *px, double 
     }
 }
 
+// State of all bodies in the caller's order, packed: [n][2][3] positions and
+// velocities, [n][3] accelerations, [n] potentials, whichever are asked for.
+// user0: a system's first body in the caller's order.
+__global__ void k_pack_user(int64_t n, const int32_t *body_sys, const int64_t *off, const int64_t *user0,
+                            const double *px, const double *py, const double *pz, const double *vx, const double *vy,
+                            const double *vz, const double *ax, const double *ay, const double *az, const double *phi,
+                            double *ophase, double *oacc, double *ophi)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int s = body_sys[i];
+        const int64_t u = user0[s] + (i - off[s]);
+        if (ophase) {
+            double *q = ophase + 6 * u;
+            q[0] = px[i];
+            q[1] = py[i];
+            q[2] = pz[i];
+            q[3] = vx[i];
+            q[4] = vy[i];
+            q[5] = vz[i];
+        }
+        if (oacc) {
+            oacc[3 * u] = ax[i];
+            oacc[3 * u + 1] = ay[i];
+            oacc[3 * u + 2] = az[i];
+        }
+        if (ophi) ophi[u] = phi[i];
+    }
+}
+
 __global__ void k_init_boxes(int n, SysBox *box)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
@@ -370,7 +399,9 @@ struct hc_ens {
     int32_t *d_body_sys = nullptr, *d_user_of = nullptr, *d_dsys = nullptr;
     int32_t *d_root = nullptr, *d_depth = nullptr;
     SysBox *d_box = nullptr;
+    int64_t *d_user0 = nullptr;                  // [internal slot] first body in the caller's order
     double *d_origin = nullptr, *d_energy = nullptr, *h_energy = nullptr, *d_stage = nullptr;
+    bool uploaded = false;
     int max_direct_n = 0;
     int direct_threads = 256;                    // block size of the direct sum (tuned)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -509,6 +540,7 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
     HC_TRY(ens_alloc(e->err, &e->d_off, nsys + 1));
     HC_TRY(ens_alloc(e->err, &e->d_body_sys, n));
     HC_TRY(ens_alloc(e->err, &e->d_user_of, nsys));
+    HC_TRY(ens_alloc(e->err, &e->d_user0, nsys));
     HC_TRY(ens_alloc(e->err, &e->d_dsys, std::max(1, e->nsys_direct)));
     HC_TRY(ens_alloc(e->err, &e->d_root, std::max(1, e->nsys_tree)));
     HC_TRY(ens_alloc(e->err, &e->d_depth, std::max(1, e->nsys_tree)));
@@ -523,6 +555,9 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
             for (int64_t i = e->int_off[k]; i < e->int_off[k + 1]; i++) body_sys[i] = k;
             if (k >= e->nsys_tree) dsys[k - e->nsys_tree] = k;
         }
+        std::vector<int64_t> user0(nsys);
+        for (int k = 0; k < nsys; k++) user0[k] = e->user_off[e->order[k]];
+        EC(cudaMemcpy(e->d_user0, user0.data(), sizeof(int64_t) * nsys, cudaMemcpyHostToDevice));
         EC(cudaMemcpy(e->d_off, e->int_off.data(), sizeof(int64_t) * (nsys + 1), cudaMemcpyHostToDevice));
         EC(cudaMemcpy(e->d_body_sys, body_sys.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
         EC(cudaMemcpy(e->d_user_of, user_of.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice));
@@ -577,7 +612,7 @@ void hc_ens_destroy(hc_ens *e)
     }
     void *ptrs[] = {e->mass, e->px, e->py, e->pz, e->vx, e->vy, e->vz, e->ax, e->ay, e->az, e->phi, e->d_off,
                     e->d_body_sys, e->d_user_of, e->d_dsys, e->d_root, e->d_depth, e->d_box, e->d_origin,
-                    e->d_energy, e->d_stage};
+                    e->d_energy, e->d_stage, e->d_user0};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (e->h_energy) cudaFreeHost(e->h_energy);
@@ -606,7 +641,9 @@ int hc_ens_upload(hc_ens *e, const double *mass, const double *phase)
             e->err = "ensemble bodies need positive, finite masses";
             return HC_ERR_ARG;
         }
-    if (!e->d_stage) HC_TRY(ens_alloc(e->err, &e->d_stage, 6 * n));
+    if (!e->d_stage) {
+        HC_TRY(ens_alloc(e->err, &e->d_stage, 10 * n));      // the largest download too
+    }
     EC(cudaMemcpyAsync(e->mass, m.data(), sizeof(double) * n, cudaMemcpyHostToDevice, e->stream));
     EC(cudaMemcpyAsync(e->d_stage, ph.data(), sizeof(double) * 6 * n, cudaMemcpyHostToDevice, e->stream));
     k_unpack_sys<<<hc_grid(n, 256), 256, 0, e->stream>>>(e->d_stage, n, e->px, e->py, e->pz, e->vx, e->vy, e->vz);
@@ -616,6 +653,7 @@ int hc_ens_upload(hc_ens *e, const double *mass, const double *phase)
         k_init_boxes<<<hc_grid(e->nsys_tree, 256), 256, 0, e->stream>>>(e->nsys_tree, e->d_box);
     EC(cudaStreamSynchronize(e->stream));
     EC(cudaGetLastError());
+    e->uploaded = true;
     return HC_OK;
 }
 
@@ -709,7 +747,7 @@ int hc_ens_get_tuning(hc_ens *e, hc_ens_tuning *t)
 int hc_ens_autotune(hc_ens *e, hc_ens_tuning *best)
 {
     if (!e) return HC_ERR_ARG;
-    if (!e->d_stage) {
+    if (!e->uploaded) {
         e->err = "hc_ens_autotune: upload the bodies first";
         return HC_ERR_STATE;
     }
@@ -789,41 +827,26 @@ int hc_ens_download(hc_ens *e, double *phase, double *acc, double *phi)
 {
     if (!e) return HC_ERR_ARG;
     const int64_t n = e->ntot;
-    EC(cudaStreamSynchronize(e->stream));
-    auto fetch = [&](const double *d, std::vector<double> &h) -> int {
-        h.resize(n);
-        EC(cudaMemcpy(h.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    const int64_t np = phase ? 6 * n : 0, na = acc ? 3 * n : 0, nf = phi ? n : 0;
+    if (np + na + nf == 0) {
+        EC(cudaStreamSynchronize(e->stream));
         return HC_OK;
-    };
-    std::vector<double> a, b, c2;
-    if (phase) {
-        const double *src[6] = {e->px, e->py, e->pz, e->vx, e->vy, e->vz};
-        for (int q = 0; q < 6; q++) {
-            HC_TRY(fetch(src[q], a));
-            for (int k = 0; k < e->nsys; k++) {
-                const int u = e->order[k];
-                for (int64_t i = 0; i < e->user_count[u]; i++) phase[6 * (e->user_off[u] + i) + q] = a[e->int_off[k] + i];
-            }
-        }
     }
-    if (acc) {
-        const double *src[3] = {e->ax, e->ay, e->az};
-        for (int q = 0; q < 3; q++) {
-            HC_TRY(fetch(src[q], a));
-            for (int k = 0; k < e->nsys; k++) {
-                const int u = e->order[k];
-                for (int64_t i = 0; i < e->user_count[u]; i++) acc[3 * (e->user_off[u] + i) + q] = a[e->int_off[k] + i];
-            }
-        }
+    // Packed in the caller's order on the device, then one copy per array.  (Each
+    // of the ten components fetched apart and spread over the caller's arrays by
+    // the host took 4.4 ms of a 6.7 ms step and download of 320,000 bodies.)
+    if (!e->d_stage) {
+        HC_TRY(ens_alloc(e->err, &e->d_stage, 10 * n));
     }
-    if (phi) {
-        HC_TRY(fetch(e->phi, b));
-        for (int k = 0; k < e->nsys; k++) {
-            const int u = e->order[k];
-            std::memcpy(phi + e->user_off[u], &b[e->int_off[k]], sizeof(double) * e->user_count[u]);
-        }
-    }
-    (void)c2;
+    double *d = e->d_stage;
+    k_pack_user<<<hc_grid(n, 256), 256, 0, e->stream>>>(n, e->d_body_sys, e->d_off, e->d_user0, e->px, e->py, e->pz, e->vx,
+                                                        e->vy, e->vz, e->ax, e->ay, e->az, e->phi, phase ? d : nullptr,
+                                                        acc ? d + np : nullptr, phi ? d + np + na : nullptr);
+    if (phase) EC(cudaMemcpyAsync(phase, d, sizeof(double) * np, cudaMemcpyDeviceToHost, e->stream));
+    if (acc) EC(cudaMemcpyAsync(acc, d + np, sizeof(double) * na, cudaMemcpyDeviceToHost, e->stream));
+    if (phi) EC(cudaMemcpyAsync(phi, d + np + na, sizeof(double) * nf, cudaMemcpyDeviceToHost, e->stream));
+    EC(cudaStreamSynchronize(e->stream));
+    EC(cudaGetLastError());
     return HC_OK;
 }
 
