@@ -11,7 +11,7 @@
 // One step, all of it captured in one CUDA graph:
 //   1. per tree system, hackcode1's expandbox replay (load.c:68-95) on its
 //      own persistent root box, which starts at (-2,-2,-2), 4 (code.c:119-120)
-//      and only grows -- one warp per system, bodies in order;
+//      and only grows -- one block per system, bodies in order;
 //   2. slot layout: every system box is placed in its own slot of one forest
 //      box (slots of the largest system's size on a G^3 grid, G a power of
 //      two), so that the system box is exactly a forest cell; positions are
@@ -22,7 +22,7 @@
 //   4. the walk of each group starts at its system's root cell (found from
 //      the pre-order cells), so no system sees another;
 //   5. systems of at most direct_max bodies: FP32 direct sum, one block per
-//      system, positions split hi + lo relative to the system's first body;
+//      64 bodies, positions split hi + lo relative to the system's first body;
 //   6. closing half-kick inside 3-5 (code.c:175-179), per-system energies,
 //      then kick-drift of every body (code.c:182-188).
 //
@@ -31,6 +31,7 @@
 // that are reported as coincident), and the one-body cells that hackcode1
 // grafts when its second body expands the box twice or more are not formed.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -63,35 +64,69 @@ __device__ __forceinline__ bool inbox_d(double x, double y, double z, const doub
     return true;
 }
 
-// 1. expandbox replay, one warp per tree system.  The box only grows, so a
-// body found inside stays inside: each pass finds the first body of the
-// remaining range outside the current box and expands for it.
-__global__ void k_ens_replay(int nsys_tree, const int64_t *off, const double *mass, const double *px,
-                             const double *py, const double *pz, SysBox *box, hc_status *st)
+// 1. expandbox replay, one block per tree system.  The box only grows, so a
+// body found inside stays inside: each round finds the first body of the
+// remaining range outside the current box and expands for it.  A body clearly
+// inside by an FP32 estimate skips the exact test (as in k_box_outside): with
+// the exact test's three FP64 divisions for every body, one warp per system
+// took 1.26 ms for systems of up to 16,384 bodies.
+__global__ void __launch_bounds__(256) k_ens_replay(const int64_t *off, const double *mass, const double *px,
+                                                    const double *py, const double *pz, SysBox *box, hc_status *st)
 {
-    const int lane = threadIdx.x & 31;
-    const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (s >= nsys_tree) return;
-    double rmin[3] = {box[s].rmin[0], box[s].rmin[1], box[s].rmin[2]};
-    double rsize = box[s].rsize;
-    const int64_t b0 = off[s], b1 = off[s + 1];
-    for (int64_t base = b0; base < b1; base += 32) {
-        const int64_t i = base + lane;
-        bool out = false;
-        if (i < b1 && mass[i] != 0.0) out = !inbox_d(px[i], py[i], pz[i], rmin, rsize);
-        unsigned m = __ballot_sync(0xffffffffu, out);
-        while (m) {
-            const int f = __ffs(m) - 1;
-            const int64_t j = base + f;
-            const double x[3] = {px[j], py[j], pz[j]};
-            int k = 0;
-            while (!inbox_d(x[0], x[1], x[2], rmin, rsize)) {     // load.c:74-93 (same on every lane)
-                if (++k > 1100) {                                  // non-finite position
-                    if (lane == 0) {
-                        atomicCAS(&st->error, 0, HC_ERR_ARG);
-                        st->info = (int)j;
+    constexpr int CHUNK = 256 * 8;              // bodies between two looks for an early end
+    __shared__ double rmin[3], rsize;
+    __shared__ int first, bad;
+    const int s = blockIdx.x, tid = threadIdx.x;
+    const int64_t b0 = off[s];
+    const int n = (int)(off[s + 1] - b0);
+    if (tid == 0) {
+        for (int d = 0; d < 3; d++) rmin[d] = box[s].rmin[d];
+        rsize = box[s].rsize;
+        first = INT_MAX;
+        bad = 0;
+    }
+    __syncthreads();
+    int pos = 0;
+    while (true) {
+        const float lo[3] = {hc_d2f_rn(rmin[0]), hc_d2f_rn(rmin[1]), hc_d2f_rn(rmin[2])}, sz = hc_d2f_rn(rsize);
+        for (int base = pos; base < n; base += CHUNK) {
+            int mine = INT_MAX;
+#pragma unroll
+            for (int r = 0; r < CHUNK / 256; r++) {
+                const int i = base + r * 256 + tid;
+                if (i >= n) continue;
+                const double x[3] = {px[b0 + i], py[b0 + i], pz[b0 + i]};
+                bool clear = true;
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    float f;
+                    if (!hc_approx_f32(x[d], &f)) {
+                        clear = false;
+                        continue;
                     }
-                    return;
+                    const float u = f - lo[d], margin = 0x1p-16f * sz + 0x1p-18f * fabsf(f);
+                    clear = clear && u >= margin && u <= sz - margin;
+                }
+                if (!clear && hc_nonzero(mass[b0 + i]) && !inbox_d(x[0], x[1], x[2], rmin, rsize)) mine = min(mine, i);
+            }
+            if (__syncthreads_or(mine != INT_MAX)) {
+                if (mine != INT_MAX) atomicMin(&first, mine);
+                __syncthreads();
+                break;
+            }
+        }
+        const int f = first;
+        __syncthreads();
+        if (f == INT_MAX) break;
+        if (tid == 0) {
+            const double x[3] = {px[b0 + f], py[b0 + f], pz[b0 + f]};
+            int k = 0;
+            while (!inbox_d(x[0], x[1], x[2], rmin, rsize)) {         // load.c:74-93
+                if (++k > 1100) {                                      // non-finite position
+                    atomicCAS(&st->error, 0, HC_ERR_ARG);
+                    st->info = (int)(b0 + f);
+                    bad = 1;
+                    break;
                 }
                 double rmid[3];
                 for (int d = 0; d < 3; d++) rmid[d] = __dadd_rn(rmin[d], __dmul_rn(0.5, rsize));
@@ -99,13 +134,13 @@ __global__ void k_ens_replay(int nsys_tree, const int64_t *off, const double *ma
                     if (x[d] < rmid[d]) rmin[d] = __dsub_rn(rmin[d], rsize);
                 rsize = __dmul_rn(2.0, rsize);
             }
-            // bodies after f in this chunk: test again against the grown box
-            out = false;
-            if (lane > f && i < b1 && mass[i] != 0.0) out = !inbox_d(px[i], py[i], pz[i], rmin, rsize);
-            m = __ballot_sync(0xffffffffu, out);
+            first = INT_MAX;
         }
+        __syncthreads();
+        if (bad) return;
+        pos = f + 1;
     }
-    if (lane == 0) box[s] = SysBox{{rmin[0], rmin[1], rmin[2]}, rsize};
+    if (tid == 0) box[s] = SysBox{{rmin[0], rmin[1], rmin[2]}, rsize};
 }
 
 // 2a. slot layout (one block): slot size = largest system box, G^3 slots;
@@ -200,79 +235,112 @@ __device__ __forceinline__ void kahan(float &sum, float &comp, float x)
     sum = t;
 }
 
-// 5. direct sum of one small system per block (FP32, hi + lo positions
-// relative to the system's first body; Kahan over 64-body partials); any
-// block size up to 512 threads
-__global__ void __launch_bounds__(512) k_ens_direct(const int32_t *dsys, const int64_t *off, const double *mass,
-                                                         const double *px, const double *py, const double *pz,
-                                                         float eps2, double kick_dthf, int64_t nstep, double *vx,
-                                                         double *vy, double *vz, double *ax, double *ay, double *az,
-                                                         double *phi)
+// 5. direct sum of the small systems (FP32, hi + lo positions relative to the
+// system's first body; Kahan over 64-body partials).  A block takes 64 bodies
+// of one system (work: system, first body) and the whole system as sources,
+// staged in pairs: both bodies' values of one quantity adjacent, the operands
+// of one packed FP32x2 instruction.  Its T / 64 slices of warps take a slice of
+// the sources each, added at the end in slice order.  (One block per whole
+// system with scalar arithmetic: 253 us for 53 systems of up to 1024 bodies.)
+constexpr int DROWS = 64;
+static size_t ens_direct_smem(int n, int threads)
+{
+    return sizeof(float4) * (4 * (size_t)((n + 1) / 2) + 2 * (size_t)threads);
+}
+__global__ void __launch_bounds__(512) k_ens_direct(const int2 *work, const int64_t *off, const double *mass,
+                                                    const double *px, const double *py, const double *pz,
+                                                    float eps2, double kick_dthf, int64_t nstep, double *vx,
+                                                    double *vy, double *vz, double *ax, double *ay, double *az,
+                                                    double *phi)
 {
     extern __shared__ float4 sm[];
-    const int s = dsys[blockIdx.x];
+    const int s = work[blockIdx.x].x, row = work[blockIdx.x].y + threadIdx.x % DROWS;
+    const int slice = threadIdx.x / DROWS, nslice = blockDim.x / DROWS;
     const int64_t b0 = off[s];
-    const int n = (int)(off[s + 1] - b0);
-    float4 *H = sm, *L = sm + n;
+    const int n = (int)(off[s + 1] - b0), np = (n + 1) / 2;
+    float4(*const pair)[4] = reinterpret_cast<float4(*)[4]>(sm);   // (hx hy) (hz m) (lx ly) (lz -), for two bodies
+    float4 *const part = sm + 4 * np;
     const double cx = px[b0], cy = py[b0], cz = pz[b0];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double dx = px[b0 + j] - cx, dy = py[b0 + j] - cy, dz = pz[b0 + j] - cz;
-        float4 h, l;
-        hc_split_hilo(dx, &h.x, &l.x);          // on the doubles' bits (no FP64-pipe conversions)
-        hc_split_hilo(dy, &h.y, &l.y);
-        hc_split_hilo(dz, &h.z, &l.z);
-        h.w = hc_d2f_rn(mass[b0 + j]);
-        l.w = 0.f;
-        H[j] = h;
-        L[j] = l;
+    for (int j = threadIdx.x; j < 2 * np; j += blockDim.x) {
+        float *f = reinterpret_cast<float *>(pair[j >> 1]) + (j & 1);
+        if (j < n) {
+            hc_split_hilo(px[b0 + j] - cx, &f[0], &f[8]);          // on the doubles' bits (no FP64-pipe conversions)
+            hc_split_hilo(py[b0 + j] - cy, &f[2], &f[10]);
+            hc_split_hilo(pz[b0 + j] - cz, &f[4], &f[12]);
+            f[6] = hc_d2f_rn(mass[b0 + j]);
+        } else {                                                    // pad: massless, far away
+            f[0] = f[2] = f[4] = 1.0e4f;
+            f[6] = f[8] = f[10] = f[12] = 0.f;
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const float4 Hi = H[i], Li = L[i];
-        float sx = 0.f, sy = 0.f, sz = 0.f, sp = 0.f, cxs = 0.f, cys = 0.f, czs = 0.f, cps = 0.f;
-        for (int j0 = 0; j0 < n; j0 += 64) {
-            const int j1 = j0 + 64 < n ? j0 + 64 : n;
-            float qx = 0.f, qy = 0.f, qz = 0.f, qp = 0.f;
-            for (int j = j0; j < j1; j++) {
-                const float4 Hj = H[j], Lj = L[j];
-                const float dx = (Hj.x - Hi.x) + (Lj.x - Li.x), dy = (Hj.y - Hi.y) + (Lj.y - Li.y),
-                            dz = (Hj.z - Hi.z) + (Lj.z - Li.z);
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-                const float rinv = rsqrtf(r2);
-                const float mr = j == i ? 0.f : Hj.w * rinv;
-                const float mr3 = mr * rinv * rinv;
-                qp -= mr;
-                qx = fmaf(mr3, dx, qx);
-                qy = fmaf(mr3, dy, qy);
-                qz = fmaf(mr3, dz, qz);
+    float4 S = make_float4(0.f, 0.f, 0.f, 0.f), C = S;              // Kahan sums x, y, z, -phi
+    if (row < n) {
+        const float *f = reinterpret_cast<const float *>(pair[row >> 1]) + (row & 1);
+        const float2 bx = splat2(-f[0]), by = splat2(-f[2]), bz = splat2(-f[4]), blx = splat2(-f[8]), bly = splat2(-f[10]),
+                     blz = splat2(-f[12]), e2 = splat2(eps2);
+        const int p1 = (int)((int64_t)np * (slice + 1) / nslice);
+        for (int p0 = (int)((int64_t)np * slice / nslice); p0 < p1; p0 += 32) {
+            float2 qx = splat2(0.f), qy = qx, qz = qx, qp = qx;
+            const int pe = p0 + 32 < p1 ? p0 + 32 : p1;
+#pragma unroll 4
+            for (int p = p0; p < pe; p++) {
+                const float4 H0 = pair[p][0], H1 = pair[p][1], L0 = pair[p][2], L1 = pair[p][3];
+                const float2 dx = __fadd2_rn(__fadd2_rn(lo2(H0), bx), __fadd2_rn(lo2(L0), blx));
+                const float2 dy = __fadd2_rn(__fadd2_rn(hi2(H0), by), __fadd2_rn(hi2(L0), bly));
+                const float2 dz = __fadd2_rn(__fadd2_rn(lo2(H1), bz), __fadd2_rn(lo2(L1), blz));
+                const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+                const float2 w = make_float2(2 * p != row ? rsqrtf(r2.x) : 0.f, 2 * p + 1 != row ? rsqrtf(r2.y) : 0.f);
+                const float2 mr = __fmul2_rn(hi2(H1), w);
+                const float2 mr3 = __fmul2_rn(mr, __fmul2_rn(w, w));
+                qp = __fadd2_rn(qp, mr);
+                qx = __ffma2_rn(mr3, dx, qx);
+                qy = __ffma2_rn(mr3, dy, qy);
+                qz = __ffma2_rn(mr3, dz, qz);
             }
-            kahan(sx, cxs, qx);
-            kahan(sy, cys, qy);
-            kahan(sz, czs, qz);
-            kahan(sp, cps, qp);
+            kahan(S.x, C.x, qx.x + qx.y);
+            kahan(S.y, C.y, qy.x + qy.y);
+            kahan(S.z, C.z, qz.x + qz.y);
+            kahan(S.w, C.w, qp.x + qp.y);
         }
-        const int64_t o = b0 + i;
-        const double rx = (double)sx - (double)cxs, ry = (double)sy - (double)cys, rz = (double)sz - (double)czs;
-        if (kick_dthf != 0.0 && nstep > 0) {          // closing half kick (code.c:175-179)
-            vx[o] = __dadd_rn(vx[o], __dmul_rn(__dsub_rn(rx, ax[o]), kick_dthf));
-            vy[o] = __dadd_rn(vy[o], __dmul_rn(__dsub_rn(ry, ay[o]), kick_dthf));
-            vz[o] = __dadd_rn(vz[o], __dmul_rn(__dsub_rn(rz, az[o]), kick_dthf));
-        }
-        ax[o] = rx;
-        ay[o] = ry;
-        az[o] = rz;
-        phi[o] = (double)sp - (double)cps;
     }
+    part[2 * threadIdx.x] = S;
+    part[2 * threadIdx.x + 1] = C;
+    __syncthreads();
+    if (slice > 0 || row >= n) return;
+    double r[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int q = 0; q < nslice; q++) {
+        const float4 a = part[2 * (threadIdx.x + q * DROWS)], c = part[2 * (threadIdx.x + q * DROWS) + 1];
+        r[0] += (double)a.x - (double)c.x;
+        r[1] += (double)a.y - (double)c.y;
+        r[2] += (double)a.z - (double)c.z;
+        r[3] += (double)a.w - (double)c.w;
+    }
+    const int64_t o = b0 + row;
+    if (kick_dthf != 0.0 && nstep > 0) {          // closing half kick (code.c:175-179)
+        vx[o] = __dadd_rn(vx[o], __dmul_rn(__dsub_rn(r[0], ax[o]), kick_dthf));
+        vy[o] = __dadd_rn(vy[o], __dmul_rn(__dsub_rn(r[1], ay[o]), kick_dthf));
+        vz[o] = __dadd_rn(vz[o], __dmul_rn(__dsub_rn(r[2], az[o]), kick_dthf));
+    }
+    ax[o] = r[0];
+    ay[o] = r[1];
+    az[o] = r[2];
+    phi[o] = -r[3];
 }
 
-// 6a. kinetic and potential energy of each system (code_io.c:160-197)
-__global__ void __launch_bounds__(DTHREADS) k_ens_energy(const int64_t *off, const int32_t *user_of, const double *mass,
+// 6a. kinetic and potential energy of each system (code_io.c:160-197): a block
+// per chunk of ECHUNK bodies (work: system, first body), then each system's
+// chunks in order.  (One block per system held one SM's FP64 pipe for 54 us at
+// 16,384 bodies.)
+constexpr int ECHUNK = 1024;
+__global__ void __launch_bounds__(DTHREADS) k_ens_energy(const int2 *work, const int64_t *off, const double *mass,
                                                          const double *vx, const double *vy, const double *vz,
-                                                         const double *phi, double *out)
+                                                         const double *phi, double2 *part)
 {
-    const int s = blockIdx.x;
+    const int64_t i0 = off[work[blockIdx.x].x] + work[blockIdx.x].y, end = off[work[blockIdx.x].x + 1];
+    const int64_t i1 = i0 + ECHUNK < end ? i0 + ECHUNK : end;
     double ke = 0.0, pe = 0.0;
-    for (int64_t i = off[s] + threadIdx.x; i < off[s + 1]; i += DTHREADS) {
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += DTHREADS) {
         const double hm = __dmul_rn(0.5, mass[i]);
         double v2 = __dmul_rn(vx[i], vx[i]);
         v2 = __dadd_rn(v2, __dmul_rn(vy[i], vy[i]));
@@ -291,12 +359,22 @@ __global__ void __launch_bounds__(DTHREADS) k_ens_energy(const int64_t *off, con
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const int u = user_of[s];
-        out[3 * u + 0] = rk[0];
-        out[3 * u + 1] = rp[0];
-        out[3 * u + 2] = rk[0] + rp[0];
+    if (threadIdx.x == 0) part[blockIdx.x] = make_double2(rk[0], rp[0]);
+}
+
+__global__ void k_ens_energy_sum(int nsys, const int32_t *chunk0, const int32_t *user_of, const double2 *part, double *out)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nsys) return;
+    double ke = 0.0, pe = 0.0;
+    for (int c = chunk0[s]; c < chunk0[s + 1]; c++) {
+        ke += part[c].x;
+        pe += part[c].y;
     }
+    const int u = user_of[s];
+    out[3 * u + 0] = ke;
+    out[3 * u + 1] = pe;
+    out[3 * u + 2] = ke + pe;
 }
 
 // 6b. v += a dt/2; x += v dt; v += a dt/2  (code.c:182-188)
@@ -396,7 +474,11 @@ struct hc_ens {
     double *mass = nullptr, *px = nullptr, *py = nullptr, *pz = nullptr, *vx = nullptr, *vy = nullptr,
            *vz = nullptr, *ax = nullptr, *ay = nullptr, *az = nullptr, *phi = nullptr;
     int64_t *d_off = nullptr;
-    int32_t *d_body_sys = nullptr, *d_user_of = nullptr, *d_dsys = nullptr;
+    int32_t *d_body_sys = nullptr, *d_user_of = nullptr;
+    int2 *d_dwork = nullptr, *d_ework = nullptr; // (system, first body) of the direct sum's and the energies' blocks
+    int32_t *d_echunk0 = nullptr;                // [nsys + 1] first energy chunk of each system
+    double2 *d_epart = nullptr;
+    int ndwork = 0, nework = 0;
     int32_t *d_root = nullptr, *d_depth = nullptr;
     SysBox *d_box = nullptr;
     int64_t *d_user0 = nullptr;                  // [internal slot] first body in the caller's order
@@ -432,8 +514,7 @@ int ens_enqueue(hc_ens *e, double kick_dthf, int64_t nstep, double dt, bool capt
     if (e->forest) {
         hc_ctx *c = e->forest;
         EC(cudaMemsetAsync(c->st, 0, sizeof(hc_status), s));
-        k_ens_replay<<<(e->nsys_tree + 3) / 4, 128, 0, s>>>(e->nsys_tree, e->d_off, e->mass, e->px, e->py, e->pz,
-                                                          e->d_box, c->st);
+        k_ens_replay<<<e->nsys_tree, 256, 0, s>>>(e->d_off, e->mass, e->px, e->py, e->pz, e->d_box, c->st);
         k_ens_layout<<<1, 256, 0, s>>>(e->nsys_tree, e->gbits, e->d_box, e->d_origin, e->d_depth, e->d_root, c->box,
                                        c->st);
         k_ens_translate<<<hc_grid(e->n_tree, 256), 256, 0, s>>>(e->n_tree, e->d_body_sys, e->d_box, e->d_origin,
@@ -457,19 +538,18 @@ int ens_enqueue(hc_ens *e, double kick_dthf, int64_t nstep, double dt, bool capt
     }
     EC(cudaEventRecordWithFlags(e->ev[1], s, rflags));
     if (e->nsys_direct > 0) {
-        const size_t smem = sizeof(float4) * 2 * (size_t)e->max_direct_n;
-        k_ens_direct<<<e->nsys_direct, e->direct_threads, smem, s>>>(e->d_dsys, e->d_off, e->mass, e->px, e->py, e->pz,
-                                                             (float)(e->prm.eps * e->prm.eps), kick_dthf, nstep,
-                                                             e->vx, e->vy, e->vz, e->ax, e->ay, e->az, e->phi);
+        k_ens_direct<<<e->ndwork, e->direct_threads, ens_direct_smem(e->max_direct_n, e->direct_threads), s>>>(
+            e->d_dwork, e->d_off, e->mass, e->px, e->py, e->pz, (float)(e->prm.eps * e->prm.eps), kick_dthf, nstep,
+            e->vx, e->vy, e->vz, e->ax, e->ay, e->az, e->phi);
         e->launches++;
     }
     EC(cudaEventRecordWithFlags(e->ev[2], s, rflags));
     if (!advance) return HC_OK;          // forces only (the autotuner's evaluations)
-    k_ens_energy<<<e->nsys, DTHREADS, 0, s>>>(e->d_off, e->d_user_of, e->mass, e->vx, e->vy, e->vz, e->phi,
-                                              e->d_energy);
+    k_ens_energy<<<e->nework, DTHREADS, 0, s>>>(e->d_ework, e->d_off, e->mass, e->vx, e->vy, e->vz, e->phi, e->d_epart);
+    k_ens_energy_sum<<<(e->nsys + 127) / 128, 128, 0, s>>>(e->nsys, e->d_echunk0, e->d_user_of, e->d_epart, e->d_energy);
     k_ens_kick_drift<<<hc_grid(e->ntot, 256), 256, 0, s>>>(e->ntot, dt, e->px, e->py, e->pz, e->vx, e->vy, e->vz,
                                                            e->ax, e->ay, e->az);
-    e->launches += 2;
+    e->launches += 3;
     EC(cudaMemcpyAsync(e->h_energy, e->d_energy, sizeof(double) * 3 * e->nsys, cudaMemcpyDeviceToHost, s));
     if (e->forest) EC(cudaMemcpyAsync(e->forest->h_st, e->forest->st, sizeof(hc_status), cudaMemcpyDeviceToHost, s));
     return HC_OK;
@@ -541,7 +621,21 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
     HC_TRY(ens_alloc(e->err, &e->d_body_sys, n));
     HC_TRY(ens_alloc(e->err, &e->d_user_of, nsys));
     HC_TRY(ens_alloc(e->err, &e->d_user0, nsys));
-    HC_TRY(ens_alloc(e->err, &e->d_dsys, std::max(1, e->nsys_direct)));
+    std::vector<int2> dwork, ework;
+    std::vector<int32_t> echunk0(nsys + 1, 0);
+    for (int k = 0; k < nsys; k++) {
+        const int cnt = (int)(e->int_off[k + 1] - e->int_off[k]);
+        if (k >= e->nsys_tree)
+            for (int r = 0; r < cnt; r += DROWS) dwork.push_back(make_int2(k, r));
+        for (int r = 0; r < cnt; r += ECHUNK) ework.push_back(make_int2(k, r));
+        echunk0[k + 1] = (int32_t)ework.size();
+    }
+    e->ndwork = (int)dwork.size();
+    e->nework = (int)ework.size();
+    HC_TRY(ens_alloc(e->err, &e->d_dwork, std::max(1, e->ndwork)));
+    HC_TRY(ens_alloc(e->err, &e->d_ework, e->nework));
+    HC_TRY(ens_alloc(e->err, &e->d_epart, e->nework));
+    HC_TRY(ens_alloc(e->err, &e->d_echunk0, nsys + 1));
     HC_TRY(ens_alloc(e->err, &e->d_root, std::max(1, e->nsys_tree)));
     HC_TRY(ens_alloc(e->err, &e->d_depth, std::max(1, e->nsys_tree)));
     HC_TRY(ens_alloc(e->err, &e->d_box, std::max(1, e->nsys_tree)));
@@ -549,11 +643,10 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
     HC_TRY(ens_alloc(e->err, &e->d_energy, 3 * nsys));
     EC(cudaMallocHost((void **)&e->h_energy, sizeof(double) * 3 * nsys));
     {
-        std::vector<int32_t> body_sys(n), user_of(nsys), dsys(std::max(1, e->nsys_direct));
+        std::vector<int32_t> body_sys(n), user_of(nsys);
         for (int k = 0; k < nsys; k++) {
             user_of[k] = e->order[k];
             for (int64_t i = e->int_off[k]; i < e->int_off[k + 1]; i++) body_sys[i] = k;
-            if (k >= e->nsys_tree) dsys[k - e->nsys_tree] = k;
         }
         std::vector<int64_t> user0(nsys);
         for (int k = 0; k < nsys; k++) user0[k] = e->user_off[e->order[k]];
@@ -561,7 +654,9 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
         EC(cudaMemcpy(e->d_off, e->int_off.data(), sizeof(int64_t) * (nsys + 1), cudaMemcpyHostToDevice));
         EC(cudaMemcpy(e->d_body_sys, body_sys.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
         EC(cudaMemcpy(e->d_user_of, user_of.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice));
-        EC(cudaMemcpy(e->d_dsys, dsys.data(), sizeof(int32_t) * dsys.size(), cudaMemcpyHostToDevice));
+        if (e->ndwork) EC(cudaMemcpy(e->d_dwork, dwork.data(), sizeof(int2) * dwork.size(), cudaMemcpyHostToDevice));
+        EC(cudaMemcpy(e->d_ework, ework.data(), sizeof(int2) * ework.size(), cudaMemcpyHostToDevice));
+        EC(cudaMemcpy(e->d_echunk0, echunk0.data(), sizeof(int32_t) * (nsys + 1), cudaMemcpyHostToDevice));
     }
     if (e->nsys_tree > 0) {
         hc_params p = {params->tol, params->eps, params->fcells > 0 ? params->fcells : 1.0, params->usequad, 0};
@@ -590,8 +685,9 @@ int hc_ens_create(hc_ens **out, int nsys, const int64_t *counts, const hc_ens_pa
     }
     for (auto &ev : e->ev) EC(cudaEventCreate(&ev));
     if (e->max_direct_n > 0) {
-        const size_t smem = sizeof(float4) * 2 * (size_t)e->max_direct_n;
-        EC(cudaFuncSetAttribute(k_ens_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the kernel's attribute is the process's, not this ensemble's: always the largest
+        EC(cudaFuncSetAttribute(k_ens_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)ens_direct_smem(HC_ENS_DIRECT_LIMIT, 512)));
     }
     EC(cudaStreamSynchronize(e->stream));
     return HC_OK;
@@ -611,7 +707,7 @@ void hc_ens_destroy(hc_ens *e)
         cudaStreamDestroy(e->stream);
     }
     void *ptrs[] = {e->mass, e->px, e->py, e->pz, e->vx, e->vy, e->vz, e->ax, e->ay, e->az, e->phi, e->d_off,
-                    e->d_body_sys, e->d_user_of, e->d_dsys, e->d_root, e->d_depth, e->d_box, e->d_origin,
+                    e->d_body_sys, e->d_user_of, e->d_dwork, e->d_ework, e->d_epart, e->d_echunk0, e->d_root, e->d_depth, e->d_box, e->d_origin,
                     e->d_energy, e->d_stage, e->d_user0};
     for (void *p : ptrs)
         if (p) cudaFree(p);

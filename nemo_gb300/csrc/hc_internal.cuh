@@ -292,6 +292,18 @@ __device__ __forceinline__ void hc_diag_body(double *acc, double m, const double
     acc[35] += m;
 }
 
+// FP32 value of a double from its high word (sign, exponent, top 20 mantissa
+// bits) with integer operations only: relative error below 2^-20; false for
+// zeros, denormals, infinities, NaNs and magnitudes outside the FP32 range.
+__device__ __forceinline__ bool hc_approx_f32(double x, float *f)
+{
+    const int hi = __double2hiint(x);
+    const int e = ((hi >> 20) & 0x7ff) - 1023 + 127;
+    if (e < 1 || e > 254) return false;
+    *f = __int_as_float((hi & (int)0x80000000) | (e << 23) | ((hi & 0xfffff) << 3));
+    return true;
+}
+
 // Operands of the packed FP32x2 instructions (__ffma2_rn and relatives): a
 // float2 is one register pair.  Lists stored in pairs keep both entries'
 // values of one quantity adjacent, so lo2 / hi2 of a float4 row give them.

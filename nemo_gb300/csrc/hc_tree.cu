@@ -73,18 +73,6 @@ __device__ __forceinline__ bool inbox(double x, double y, double z, const double
 
 // ---------------- expandbox replay ----------------
 
-// FP32 value of a double from its high word (sign, exponent, top 20 mantissa
-// bits) with integer operations only: relative error below 2^-20; false for
-// zeros, denormals, infinities, NaNs and magnitudes outside the FP32 range.
-__device__ __forceinline__ bool approx_f32(double x, float *f)
-{
-    const int hi = __double2hiint(x);
-    const int e = ((hi >> 20) & 0x7ff) - 1023 + 127;
-    if (e < 1 || e > 254) return false;
-    *f = __int_as_float((hi & (int)0x80000000) | (e << 23) | ((hi & 0xfffff) << 3));
-    return true;
-}
-
 // the two smallest of two pairs of ascending body indices (INT_MAX: none)
 __device__ __forceinline__ int2 min2(int2 a, int2 b)
 {
@@ -145,7 +133,7 @@ __global__ void __launch_bounds__(256) k_box_outside(const double *mass, const d
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 float f;
-                if (!approx_f32(x[k], &f)) {
+                if (!hc_approx_f32(x[k], &f)) {
                     clear = false;
                     continue;
                 }
