@@ -142,6 +142,7 @@ struct hc_ctx {
     double4_32a *nodeD;
     int cofm_grid;                        // co-resident blocks of the upward-pass kernel
     int walk_blocks[20];                  // resident blocks of each walk variant
+    int walk_sms;
     hc_walk_split split;                  // buffers of split walks
     // learned opening criterion: network, training state, samples
     struct MlpSmem *mlp_packed;           // BF16 image used by the walk

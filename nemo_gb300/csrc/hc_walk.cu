@@ -79,6 +79,18 @@ struct WarpSmem {
     float light;
     int nentry, room, entry0;
 };
+// Team walk (a block of W warps per group), after the warps' areas; then the
+// shared traversal stack and the candidates of an iteration.
+struct TeamSmem {
+    int grp, sp, ncand, pad;
+    unsigned nodes[16], pushed[16];     // per warp
+};
+constexpr int TEAM_MAX = 16;
+__host__ __device__ constexpr int team_stack(int W) { return 192 * W + 256; }
+__host__ __device__ constexpr size_t team_smem(int W)
+{
+    return sizeof(TeamSmem) + sizeof(uint2) * (team_stack(W) + 32 * W);
+}
 enum { ST_N2B, ST_NBC, ST_CAND, ST_MIXED, ST_EB, ST_EC, ST_MLP, ST_ROUNDS };
 
 // dynamic shared memory of one block: the warps' areas, the learned walk's
@@ -391,8 +403,16 @@ __device__ __noinline__ int split_finish(const WalkArgs &g, WarpSmem &S, const S
 // 128 (4 blocks) for the group, error and learned rules.
 // SPLIT: the walk's split phases (groups walked in parts), compiled apart so
 // that the walk of whole groups carries none of their code.
-template <bool QUAD, bool COUNT, int MODE, bool COLLECT = false, bool SPLIT = false>
-__global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs g)
+// TEAM: the W warps of a block walk one group together.  A warp's iteration
+// takes 2 to 3 us however idle the GPU is (two round trips to L2, up to 32
+// mixed tests, two list evaluations), so while there are fewer groups than
+// resident warps the walk takes as long as its longest chain of iterations.  A
+// team shares one stack: each iteration takes up to 32 W candidates, every warp
+// classifies its 32 and keeps lists of its own; the warps' sums are added in
+// warp order.  The candidates' distribution follows from the group alone, so
+// the results do not depend on timing.
+template <bool QUAD, bool COUNT, int MODE, bool COLLECT = false, bool SPLIT = false, bool TEAM = false>
+__global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : (MODE == 0 ? 5 : 4)) k_walk(WalkArgs g)
 {
     if (g.run_flag && *g.run_flag == 0) return;   // guard passed: no fallback walk
     // group criteria accept a cell for the whole group (a cell holding the
@@ -415,9 +435,13 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
     // its shared memory.  (One atomic per accepted node on 33 global words set
     // the time of the counting walk: 50,021 bodies at theta = 0.6 took 1.04 ms
     // of walk, 0.38 ms with the block's own words.)
-    unsigned *const hist = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(smem_raw) + walk_smem(MODE, false));
+    const int W = TEAM ? (int)(blockDim.x >> 5) : WARPS, wid = threadIdx.x >> 5;
+    TeamSmem &T = *reinterpret_cast<TeamSmem *>(reinterpret_cast<WarpSmem *>(smem_raw) + W);
+    uint2 *const tstack = reinterpret_cast<uint2 *>(&T + 1), *const tcand = tstack + team_stack(W);
+    unsigned *const hist = reinterpret_cast<unsigned *>(
+        reinterpret_cast<char *>(smem_raw) + (TEAM ? sizeof(WarpSmem) * W + team_smem(W) : walk_smem(MODE, false)));
     if (COUNT) {
-        for (int i = threadIdx.x; i < 33; i += WARPS * 32) hist[i] = 0u;
+        for (int i = threadIdx.x; i < 33; i += 32 * W) hist[i] = 0u;
         __syncthreads();
     }
     const int lane = threadIdx.x & 31;
@@ -451,12 +475,19 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
         __syncwarp();
     } else if (BUDGET && ngroups <= g.sp.out_cap) {
         budget = split_budget(g, ngroups);
+        if (TEAM) budget = max(24, budget / W);
     }
 
     while (true) {
         int64_t grp;
         int item;
-        {
+        if (TEAM) {
+            __syncthreads();                     // the team is done with the last group
+            if (threadIdx.x == 0) T.grp = (int)atomicAdd(&g.sp.ctl->fetch[0], 1u);
+            __syncthreads();
+            item = T.grp;
+            grp = (int64_t)(unsigned)item;
+        } else {
             unsigned v = 0;
             if (lane == 0) v = atomicAdd(&g.sp.ctl->fetch[g.phase], 1u);
             grp = (int64_t)__shfl_sync(FULL, v, 0);
@@ -710,9 +741,11 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             sp = task.n;
             for (int i = lane; i < sp; i += 32) S.stack[i] = g.sp.entry[g.phase - 2][task.entry0 + i];
         } else if (nnode > 0) {
-            if (lane == 0) S.stack[0] = make_uint2((unsigned)root << 3, vmask);   // root, one node
+            // root, one node
+            if (TEAM ? threadIdx.x == 0 : lane == 0) (TEAM ? tstack : S.stack)[0] = make_uint2((unsigned)root << 3, vmask);
             sp = 1;
         }
+        if (TEAM) __syncthreads();
         if (SPLIT && lane == 0) {
             S.nentry = 0;
             S.entry0 = item * rule.entries;
@@ -755,9 +788,40 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             // taking at most half the free entries keeps the stack within
             // capacity; near it the walk takes fewer candidates per iteration,
             // down to one, instead of dropping to one at a fixed threshold.
-            const int gfree = (STACK - sp) / 2;
-            const int gmax = gfree >= 32 ? 32 : (gfree >= 1 ? gfree : 1);
-            if (!mlp_round) {
+            const int gfree = ((TEAM ? team_stack(W) : STACK) - sp) / 2, gfull = TEAM ? 32 * W : 32;
+            const int gmax = gfree >= gfull ? gfull : (gfree >= 1 ? gfree : 1);
+            if (TEAM) {
+                // thread t holds the t-th entry from the top and writes its nodes'
+                // slots; entries further down than the iteration's candidates, or
+                // nodes beyond them, stay
+                const int t = threadIdx.x;
+                const bool entry = t < sp;
+                const uint2 e = entry ? tstack[sp - 1 - t] : make_uint2(0u, 0u);
+                const unsigned in = __ballot_sync(FULL, entry), b0 = __ballot_sync(FULL, e.x & 1u),
+                               b1 = __ballot_sync(FULL, e.x & 2u), b2 = __ballot_sync(FULL, e.x & 4u);
+                if (lane == 0) T.nodes[wid] = __popc(in) + __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+                __syncthreads();
+                const int before = (int)__reduce_add_sync(FULL, lane < wid ? T.nodes[lane & 15] : 0u);
+                const int first = before + __popc(in & lt) + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+                const int ecnt = (int)(e.x & 7u) + 1;
+                if (entry && first < gmax) {
+                    const int take = min(ecnt, gmax - first);
+                    for (int i = 0; i < take; i++)
+                        tcand[first + i] = make_uint2((e.x >> 3) + (unsigned)(ecnt - take + i), e.y);
+                    if (take < ecnt) tstack[sp - 1 - t].x = e.x - (unsigned)take;
+                    if (first + ecnt >= gmax || t == sp - 1) {
+                        T.ncand = first + take;
+                        T.sp = sp - t - (int)(take == ecnt);
+                    }
+                }
+                __syncthreads();
+                ncand = min(max(T.ncand - 32 * wid, 0), 32);
+                sp = T.sp;
+                if (lane < ncand) {
+                    my_node = (int)tcand[threadIdx.x].x;
+                    my_mask = tcand[threadIdx.x].y;
+                }
+            } else if (!mlp_round) {
                 // Lane i holds the i-th entry from the top; its nodes take the
                 // slots [first, first + count).  The prefix sums come from one
                 // ballot per bit of the counts, and slot j finds its entry as
@@ -995,13 +1059,21 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
                 }
             }
             const unsigned pb = __ballot_sync(FULL, push);
-            const int npush = __popc(pb);
-            if (sp + npush > STACK) {
+            int npush = __popc(pb), pos0 = sp;
+            if (TEAM) {
+                if (lane == 0) T.pushed[wid] = npush;
+                __syncthreads();
+                const unsigned c = lane < W ? T.pushed[lane & 15] : 0u;
+                pos0 += (int)__reduce_add_sync(FULL, lane < wid ? c : 0u);
+                npush = (int)__reduce_add_sync(FULL, c);
+            }
+            if (sp + npush > (TEAM ? team_stack(W) : STACK)) {
                 overflow = true;
                 break;
             }
             if (push)
-                S.stack[sp + __popc(pb & lt)] = make_uint2(((unsigned)C.x << 3) | (unsigned)((C.y & 255) - 1), openm);
+                (TEAM ? tstack : S.stack)[pos0 + __popc(pb & lt)] =
+                    make_uint2(((unsigned)C.x << 3) | (unsigned)((C.y & 255) - 1), openm);
             sp += npush;
             if (sp > max_sp) max_sp = sp;
 
@@ -1061,11 +1133,12 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
                 flush_cells(nc);
                 nc = 0;
             }
-            __syncwarp();
+            if (TEAM) __syncthreads();           // the pushes, before the next iteration reads them
+            else __syncwarp();
         }
 #undef GUV
         if (BUDGET && left < 0) {
-            if (lane == 0) g.sp.out[atomicAdd(&g.sp.ctl->nout, 1)] = (int)grp;
+            if (TEAM ? threadIdx.x == 0 : lane == 0) g.sp.out[atomicAdd(&g.sp.ctl->nout, 1)] = (int)grp;
             continue;
         }
         if (overflow) {
@@ -1090,6 +1163,39 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
             }
         }
         __syncwarp();
+        if (TEAM) {
+            // the warps' sums, in their (no longer used) list areas, added in warp
+            // order by the first one: pairs of floats, each addition's error kept
+#pragma unroll
+            for (int k = 0; k < BPL; k++) {
+                (&S.bp[0][0])[2 * (lane + 32 * k)] = make_float4(sax[k], say[k], saz[k], sphi[k]);
+                (&S.bp[0][0])[2 * (lane + 32 * k) + 1] = make_float4(cax[k], cay[k], caz[k], cphi[k]);
+                if (COUNT) reinterpret_cast<int2 *>(&S.cp[0][0])[lane + 32 * k] = make_int2(myb[k], myc[k]);
+            }
+            __syncthreads();
+            if (wid > 0) continue;
+            auto add = [](float &s, float &c, float x, float e) {      // (s - c) + (x - e)
+                const float t = __fadd_rn(s, x), u = __fsub_rn(t, s);
+                c = __fsub_rn(c, __fsub_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(x, u)), e));
+                s = t;
+            };
+#pragma unroll
+            for (int k = 0; k < BPL; k++) {
+                for (int w = 1; w < W; w++) {
+                    const WarpSmem &R = reinterpret_cast<const WarpSmem *>(smem_raw)[w];
+                    const float4 a = (&R.bp[0][0])[2 * (lane + 32 * k)], e = (&R.bp[0][0])[2 * (lane + 32 * k) + 1];
+                    add(sax[k], cax[k], a.x, e.x);
+                    add(say[k], cay[k], a.y, e.y);
+                    add(saz[k], caz[k], a.z, e.z);
+                    add(sphi[k], cphi[k], a.w, e.w);
+                    if (COUNT) {
+                        const int2 q = reinterpret_cast<const int2 *>(&R.cp[0][0])[lane + 32 * k];
+                        myb[k] += q.x;
+                        myc[k] += q.y;
+                    }
+                }
+            }
+        }
         // slot of the partial sums of a split walk (-1: the results are final)
         const int slot = SPLIT ? split_finish(g, S, rule, item, task, (int)grp, (int)s0, (int)cnt, lane) : -1;
 
@@ -1125,7 +1231,7 @@ __global__ void __launch_bounds__(WARPS * 32, MODE == 0 ? 5 : 4) k_walk(WalkArgs
     }
     if (COUNT) {
         __syncthreads();
-        for (int i = threadIdx.x; i < 33; i += WARPS * 32)
+        for (int i = threadIdx.x; i < 33; i += 32 * W)
             if (hist[i]) atomicAdd(&g.st->mask_hist[i], (unsigned long long)hist[i]);
     }
     // interaction totals and stats
@@ -1239,6 +1345,9 @@ int configure(hc_ctx *c, int variant)
 {
     const size_t smem = walk_smem(M, C);
     HC_CUDA(cudaFuncSetAttribute(k_walk<Q, C, M, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if constexpr (M != 3)
+        HC_CUDA(cudaFuncSetAttribute(k_walk<Q, C, M, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(WarpSmem) * TEAM_MAX + team_smem(TEAM_MAX) + (C ? 33 * sizeof(unsigned) : 0))));
     if constexpr (M != 0 && !L)
         HC_CUDA(cudaFuncSetAttribute(k_walk<Q, C, M, L, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int dev = 0, nsm = 0, per_sm = 0;
@@ -1246,7 +1355,25 @@ int configure(hc_ctx *c, int variant)
     HC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     HC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk<Q, C, M, L>, WARPS * 32, smem));
     c->walk_blocks[variant] = nsm * (per_sm < 1 ? 1 : per_sm);
+    c->walk_sms = nsm;
     return HC_OK;
+}
+
+// Warps per group.  The more warps, the shorter the chain of iterations, but a
+// team's first iterations are mostly empty and its barriers cost, so a full GPU
+// is better off with one warp per group.  Walk times (us) with W = 1, 4, 8, 16
+// at theta = 0.6 with quadrupoles: 4096 bodies 166, 97, 71, 62; 8192: 205, 111,
+// 82, 113; 16,384: 235, 129, 137, 204; 50,021: 323, 289, 344, 555; 100,000: 469,
+// 571, 731, 1204.  Error rule (tree groups of about 44 bodies, two per lane):
+// 4096: 352, 225, 216, 135; 16,384: 447, 270, 244, 285; 50,021: 575, 424, 475, 641;
+// 100,000: 720, 670, 772, 1147; 200,000: 946, 1099.
+inline int team_warps(const hc_ctx *c, int64_t ntarget, bool table)
+{
+    const int64_t groups = (ntarget + 31) / (table ? 44 : 32), sms = c->walk_sms;
+    if (ntarget <= 512) return 4;            // chains of ten iterations: 31 us, 35 with W = 16
+    if (groups <= sms) return 16;
+    if (2 * groups <= 5 * sms) return 8;
+    return groups <= (table ? 16 : 12) * sms ? 4 : 1;
 }
 
 // No CUDA queries here: this runs inside stream capture.
@@ -1261,7 +1388,15 @@ int launch(hc_ctx *c, WalkArgs &a, int variant)
     if (blocks < 1) blocks = 1;
     a.warps = (int)(full * WARPS);
     a.phase = 0;
-    k_walk<Q, C, M, L><<<(unsigned)blocks, WARPS * 32, smem, c->stream>>>(a);
+    const int team = M == 3 || a.run_flag || a.sys_root ? 1 : team_warps(c, a.ntarget, a.use_table);
+    if (team > 1) {
+        if constexpr (M != 3)
+            k_walk<Q, C, M, false, false, true>
+                <<<(unsigned)(16 * c->walk_sms / team), 32 * team,
+                   sizeof(WarpSmem) * team + team_smem(team) + (C ? 33 * sizeof(unsigned) : 0), c->stream>>>(a);
+    } else {
+        k_walk<Q, C, M, L><<<(unsigned)blocks, WARPS * 32, smem, c->stream>>>(a);
+    }
     c->launches++;
     if constexpr (M != 0 && !L) {
         for (a.phase = 1; a.phase < 4; a.phase++) {
