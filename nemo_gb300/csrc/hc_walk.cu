@@ -66,7 +66,11 @@ struct QueueSmem {
 // that both entries' values of one quantity are adjacent floats, the operands
 // of one packed FP32x2 instruction.
 struct WarpSmem {
-    uint2 stack[STACK];         // x = first node << 3 | (count - 1), y = lane mask
+    // traversal stack: x = first node << 3 | (count - 1), y = lane mask.  Mixed
+    // candidates are staged at its end, two entries each (in a team, whose stack
+    // is another, in pairs); an iteration takes at most half as many as there
+    // are free entries, or one: the spare entries are that one's room.
+    uint2 stack[STACK + 4];
     float4 bp[BCAP / 2][4];     // body pairs, each quantity for both entries: (hx hy) (hz m) (lx ly) (lz mask)
                                 // (hi and lo parts of the position relative to the group, mass, accept mask)
     float4 cp[CCAP / 2][5];     // cell pairs, likewise: (x y) (z m) (-Qxx -Qxy) (-Qxz -Qyy) (-Qyz -Qzz)
@@ -78,6 +82,7 @@ struct WarpSmem {
     int split;
     float light;
     int nentry, room, entry0;
+    int width;                  // lanes that the group's second bodies take (32, 16 or 8)
 };
 // Team walk (a block of W warps per group), after the warps' areas; then the
 // shared traversal stack and the candidates of an iteration.
@@ -514,10 +519,21 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
         bool valid[BPL];
         uint32_t o[BPL];
         double xd[BPL], yd[BPL], zd[BPL];
+        // Second bodies of a lane: where there are at most 16 (8) of them, 16 (8)
+        // lanes hold them and the other lanes hold them again, so that two (four)
+        // pairs of list entries are evaluated for them at once; the copies' sums
+        // are added at the end.  Over the groups of a Plummer sphere (45 bodies on
+        // average) 1.59 instead of 1.80 evaluations per pair and lane: error rule,
+        // 2^20 bodies 3.69 -> 3.60 ms, Hernquist 2^22 10.8 -> 10.45, galaxy 2^24
+        // 39.1 -> 37.8.  Without quadrupoles a pair costs too little beside its
+        // loads (262,143 bodies: 0.60 -> 0.62 ms): not used there.
+        constexpr bool NARROW = BPL == 2 && QUAD && !COUNT && !COLLECT;
+        const int width = !NARROW || cnt > 48 ? 32 : (cnt > 40 ? 16 : 8);
 #pragma unroll
         for (int k = 0; k < BPL; k++) {
-            valid[k] = lane + 32 * k < cnt;
-            o[k] = valid[k] ? g.tsorted[s0 + lane + 32 * k] : (k == 0 ? g.tsorted[s0] : o[0]);
+            const int b = k == 0 ? lane : 32 + (lane & (width - 1));     // body's place in the group
+            valid[k] = b < cnt;
+            o[k] = valid[k] ? g.tsorted[s0 + b] : (k == 0 ? g.tsorted[s0] : o[0]);
             xd[k] = g.tx[o[k]];
             yd[k] = g.ty[o[k]];
             zd[k] = g.tz[o[k]];
@@ -572,6 +588,7 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             const float v[15] = {ghx, ghy, ghz, glx, gly, glz, gminx, gmaxx, gminy, gmaxy, gminz, gmaxz, rg2, amin, cR};
 #pragma unroll
             for (int k = 0; k < 15; k++) gu[k] = v[k];
+            S.width = width;
         }
         __syncwarp();
 
@@ -602,45 +619,59 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             f[4] = 1.0e4f;
             for (int k = 3; k < nq; k++) f[2 * k] = 0.f;
         };
-        auto flush_bodies = [&](int nb) {
-            if (lane == 0) {
-                S.stat[ST_EB] += nb;
-                if (nb & 1) {
-                    pad_entry(S.bp[nb >> 1], nb, 8);
-                    if (MODE != 0) pair_slot(S.bp[nb >> 1], nb)[14] = __int_as_float(-1);
-                }
+        // An odd list is padded to whole pairs, and for narrow second bodies to
+        // whole rounds of their pairs; returns the rounds.
+        auto pad_list = [&](float4 *row, int rowlen, int n, int nq) {
+            const int per = NARROW ? 32 / S.width : 1, rounds = ((n + 1) / 2 + per - 1) / per, e = n + lane;
+            if (NARROW ? e < 2 * per * rounds : lane == 0 && (n & 1)) {
+                pad_entry(row + (e >> 1) * rowlen, e, nq);
+                if (MODE != 0 && nq == 8) pair_slot(row + (e >> 1) * rowlen, e)[14] = __int_as_float(-1);
             }
+            return rounds;
+        };
+        auto flush_bodies = [&](int nb) {
+            if (lane == 0) S.stat[ST_EB] += nb;
+            const int rounds = pad_list(S.bp[0], 4, nb, 8);
             __syncwarp();
             float2 nphi[BPL], ax[BPL], ay[BPL], az[BPL];
 #pragma unroll
             for (int k = 0; k < BPL; k++) nphi[k] = ax[k] = ay[k] = az[k] = splat2(0.f);
             const float2 e2 = splat2(eps2);
+            auto eval = [&](const float4 H0, const float4 H1, const float4 L0, const float4 L1, int k, int self) {
+                const float2 dx = __fadd2_rn(__fadd2_rn(lo2(H0), splat2(-bx[k])), __fadd2_rn(lo2(L0), splat2(-blx[k])));
+                const float2 dy = __fadd2_rn(__fadd2_rn(hi2(H0), splat2(-by[k])), __fadd2_rn(hi2(L0), splat2(-bly[k])));
+                const float2 dz = __fadd2_rn(__fadd2_rn(lo2(H1), splat2(-bz[k])), __fadd2_rn(lo2(L1), splat2(-blz[k])));
+                const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+                bool b0, b1;
+                if (MODE == 0) {
+                    b0 = __float_as_uint(L1.z) & lanebit;
+                    b1 = __float_as_uint(L1.w) & lanebit;
+                } else {
+                    b0 = __float_as_int(L1.z) != self;
+                    b1 = __float_as_int(L1.w) != self;
+                }
+                const float2 w = make_float2(b0 ? rsqrtf(r2.x) : 0.f, b1 ? rsqrtf(r2.y) : 0.f);
+                const float2 mr = __fmul2_rn(hi2(H1), w);
+                const float2 mr3 = __fmul2_rn(mr, __fmul2_rn(w, w));
+                nphi[k] = __fadd2_rn(nphi[k], mr);
+                ax[k] = __ffma2_rn(mr3, dx, ax[k]);
+                ay[k] = __ffma2_rn(mr3, dy, ay[k]);
+                az[k] = __ffma2_rn(mr3, dz, az[k]);
+                if (COUNT) myb[k] += (int)b0 + (int)b1;
+            };
+            const int fused = NARROW && S.width < 32 ? 1 : nact;       // bodies per lane evaluated together
             for (int p = 0; p < (nb + 1) >> 1; p++) {
                 const float4 H0 = S.bp[p][0], H1 = S.bp[p][1], L0 = S.bp[p][2], L1 = S.bp[p][3];
 #pragma unroll
                 for (int k = 0; k < BPL; k++) {
-                    if (k > 0 && k >= nact) continue;
-                    const float2 dx = __fadd2_rn(__fadd2_rn(lo2(H0), splat2(-bx[k])), __fadd2_rn(lo2(L0), splat2(-blx[k])));
-                    const float2 dy = __fadd2_rn(__fadd2_rn(hi2(H0), splat2(-by[k])), __fadd2_rn(hi2(L0), splat2(-bly[k])));
-                    const float2 dz = __fadd2_rn(__fadd2_rn(lo2(H1), splat2(-bz[k])), __fadd2_rn(lo2(L1), splat2(-blz[k])));
-                    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-                    bool b0, b1;
-                    if (MODE == 0) {
-                        b0 = __float_as_uint(L1.z) & lanebit;
-                        b1 = __float_as_uint(L1.w) & lanebit;
-                    } else {
-                        b0 = __float_as_int(L1.z) != lane + 32 * k;
-                        b1 = __float_as_int(L1.w) != lane + 32 * k;
-                    }
-                    const float2 w = make_float2(b0 ? rsqrtf(r2.x) : 0.f, b1 ? rsqrtf(r2.y) : 0.f);
-                    const float2 mr = __fmul2_rn(hi2(H1), w);
-                    const float2 mr3 = __fmul2_rn(mr, __fmul2_rn(w, w));
-                    nphi[k] = __fadd2_rn(nphi[k], mr);
-                    ax[k] = __ffma2_rn(mr3, dx, ax[k]);
-                    ay[k] = __ffma2_rn(mr3, dy, ay[k]);
-                    az[k] = __ffma2_rn(mr3, dz, az[k]);
-                    if (COUNT) myb[k] += (int)b0 + (int)b1;
+                    if (k > 0 && k >= fused) continue;
+                    eval(H0, H1, L0, L1, k, lane + 32 * k);
                 }
+            }
+            if (NARROW && fused < nact) {
+                const int wd = S.width, self = 32 + (lane & (wd - 1));
+                for (int r = 0, p = lane / wd; r < rounds; r++, p += 32 / wd)
+                    eval(S.bp[p][0], S.bp[p][1], S.bp[p][2], S.bp[p][3], BPL - 1, self);
             }
 #pragma unroll
             for (int k = 0; k < BPL; k++) {
@@ -654,16 +685,47 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
         auto flush_cells = [&](int nc) {
             if (lane == 0) {
                 S.stat[ST_EC] += nc;
-                if (nc & 1) {
-                    pad_entry(S.cp[nc >> 1], nc, QUAD ? 10 : 4);
-                    if (MASKED) S.cmask[nc >> 1].y = 0u;
-                }
+                if (MASKED && (nc & 1)) S.cmask[nc >> 1].y = 0u;
             }
+            const int rounds = pad_list(S.cp[0], 5, nc, QUAD ? 10 : 4);
             __syncwarp();
             float2 nphi[BPL], ax[BPL], ay[BPL], az[BPL];
 #pragma unroll
             for (int k = 0; k < BPL; k++) nphi[k] = ax[k] = ay[k] = az[k] = splat2(0.f);
             const float2 e2 = splat2(eps2);
+            auto eval = [&](const float4 P0, const float4 P1, const float4 Q0, const float4 Q1, const float4 Q2, bool m0,
+                            bool m1, int k) {
+                const float2 dx = __fadd2_rn(lo2(P0), splat2(-bx[k])), dy = __fadd2_rn(hi2(P0), splat2(-by[k])),
+                             dz = __fadd2_rn(lo2(P1), splat2(-bz[k]));
+                const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+                float2 w = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+                const float2 rinv2 = __fmul2_rn(w, w);
+                if (MASKED) w = make_float2(m0 ? w.x : 0.f, m1 ? w.y : 0.f);
+                const float2 mr = __fmul2_rn(hi2(P1), w);            // m / r (0 for a masked lane)
+                const float2 mr3 = __fmul2_rn(mr, rinv2);
+                if (!QUAD) {
+                    nphi[k] = __fadd2_rn(nphi[k], mr);
+                    ax[k] = __ffma2_rn(mr3, dx, ax[k]);
+                    ay[k] = __ffma2_rn(mr3, dy, ay[k]);
+                    az[k] = __ffma2_rn(mr3, dz, az[k]);
+                    return;
+                }
+                // gravsub's quadrupole term (grav.c:62-72) with the list's -Q:
+                // q = -Q.dr, t = -dr.Q.dr / r^5
+                const float2 qx = __ffma2_rn(lo2(Q0), dx, __ffma2_rn(hi2(Q0), dy, __fmul2_rn(lo2(Q1), dz)));
+                const float2 qy = __ffma2_rn(hi2(Q0), dx, __ffma2_rn(hi2(Q1), dy, __fmul2_rn(lo2(Q2), dz)));
+                const float2 qz = __ffma2_rn(lo2(Q1), dx, __ffma2_rn(lo2(Q2), dy, __fmul2_rn(hi2(Q2), dz)));
+                const float2 dqd = __ffma2_rn(qx, dx, __ffma2_rn(qy, dy, __fmul2_rn(qz, dz)));
+                const float2 r5 = __fmul2_rn(__fmul2_rn(w, rinv2), rinv2);
+                const float2 t = __fmul2_rn(dqd, r5);
+                // -phi += m/r + dr.Q.dr / (2 r^5);  a += dr (m/r^3 + 5/2 dr.Q.dr/r^7) - Q.dr / r^5
+                nphi[k] = __ffma2_rn(splat2(-0.5f), t, __fadd2_rn(nphi[k], mr));
+                const float2 c = __ffma2_rn(__fmul2_rn(splat2(-2.5f), rinv2), t, mr3);
+                ax[k] = __ffma2_rn(c, dx, __ffma2_rn(r5, qx, ax[k]));
+                ay[k] = __ffma2_rn(c, dy, __ffma2_rn(r5, qy, ay[k]));
+                az[k] = __ffma2_rn(c, dz, __ffma2_rn(r5, qz, az[k]));
+            };
+            const int fused = NARROW && S.width < 32 ? 1 : nact;       // bodies per lane evaluated together
 #pragma unroll 2
             for (int p = 0; p < (nc + 1) >> 1; p++) {
                 const float4 P0 = S.cp[p][0], P1 = S.cp[p][1];
@@ -682,36 +744,21 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                 }
 #pragma unroll
                 for (int k = 0; k < BPL; k++) {
-                    if (k > 0 && k >= nact) continue;
-                    const float2 dx = __fadd2_rn(lo2(P0), splat2(-bx[k])), dy = __fadd2_rn(hi2(P0), splat2(-by[k])),
-                                 dz = __fadd2_rn(lo2(P1), splat2(-bz[k]));
-                    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-                    float2 w = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                    const float2 rinv2 = __fmul2_rn(w, w);
-                    if (MASKED) w = make_float2(m0 ? w.x : 0.f, m1 ? w.y : 0.f);
-                    const float2 mr = __fmul2_rn(hi2(P1), w);            // m / r (0 for a masked lane)
-                    const float2 mr3 = __fmul2_rn(mr, rinv2);
-                    if (!QUAD) {
-                        nphi[k] = __fadd2_rn(nphi[k], mr);
-                        ax[k] = __ffma2_rn(mr3, dx, ax[k]);
-                        ay[k] = __ffma2_rn(mr3, dy, ay[k]);
-                        az[k] = __ffma2_rn(mr3, dz, az[k]);
-                        continue;
+                    if (k > 0 && k >= fused) continue;
+                    eval(P0, P1, Q0, Q1, Q2, m0, m1, k);
+                }
+            }
+            if (NARROW && fused < nact) {
+                const int wd = S.width;
+#pragma unroll 2
+                for (int r = 0, p = lane / wd; r < rounds; r++, p += 32 / wd) {
+                    float4 Q0, Q1, Q2;
+                    if (QUAD) {
+                        Q0 = S.cp[p][2];
+                        Q1 = S.cp[p][3];
+                        Q2 = S.cp[p][4];
                     }
-                    // gravsub's quadrupole term (grav.c:62-72) with the list's -Q:
-                    // q = -Q.dr, t = -dr.Q.dr / r^5
-                    const float2 qx = __ffma2_rn(lo2(Q0), dx, __ffma2_rn(hi2(Q0), dy, __fmul2_rn(lo2(Q1), dz)));
-                    const float2 qy = __ffma2_rn(hi2(Q0), dx, __ffma2_rn(hi2(Q1), dy, __fmul2_rn(lo2(Q2), dz)));
-                    const float2 qz = __ffma2_rn(lo2(Q1), dx, __ffma2_rn(lo2(Q2), dy, __fmul2_rn(hi2(Q2), dz)));
-                    const float2 dqd = __ffma2_rn(qx, dx, __ffma2_rn(qy, dy, __fmul2_rn(qz, dz)));
-                    const float2 r5 = __fmul2_rn(__fmul2_rn(w, rinv2), rinv2);
-                    const float2 t = __fmul2_rn(dqd, r5);
-                    // -phi += m/r + dr.Q.dr / (2 r^5);  a += dr (m/r^3 + 5/2 dr.Q.dr/r^7) - Q.dr / r^5
-                    nphi[k] = __ffma2_rn(splat2(-0.5f), t, __fadd2_rn(nphi[k], mr));
-                    const float2 c = __ffma2_rn(__fmul2_rn(splat2(-2.5f), rinv2), t, mr3);
-                    ax[k] = __ffma2_rn(c, dx, __ffma2_rn(r5, qx, ax[k]));
-                    ay[k] = __ffma2_rn(c, dy, __ffma2_rn(r5, qy, ay[k]));
-                    az[k] = __ffma2_rn(c, dz, __ffma2_rn(r5, qz, az[k]));
+                    eval(S.cp[p][0], S.cp[p][1], Q0, Q1, Q2, true, true, BPL - 1);
                 }
             }
 #pragma unroll
@@ -1004,12 +1051,11 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                 S.stat[ST_CAND] += ncand;
                 S.stat[ST_MIXED] += __popc(mixedb);
             }
-            // Mixed candidates are re-tested per body.  Their centres and sizes
-            // are read back from the free end of the stack (one broadcast read
-            // each instead of four shuffles): taking at most half the free
-            // entries left room for a float4 per candidate above sp.
-            if (MODE == 0 && mixedb) {
-                float4 *const mixed_c = reinterpret_cast<float4 *>(S.stack) + STACK / 2 - 1;
+            // Mixed candidates are re-tested per body.  Their centres and sizes are
+            // read back from the free end of the stack (one broadcast read each
+            // instead of four shuffles).
+            if (MODE == 0 && !TEAM && mixedb) {
+                float4 *const mixed_c = reinterpret_cast<float4 *>(S.stack + STACK + 4) - 1;
                 if (mixed) mixed_c[-lane] = make_float4(cx, cy, cz, B.w);
                 __syncwarp();
                 while (mixedb) {
@@ -1037,6 +1083,58 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                         accm = ab;
                     }
                 }
+            }
+            // In a team, where the iteration's latency counts, two at a time in
+            // packed FP32x2 arithmetic (50,021 bodies: walk 303 -> 283 us; with one
+            // warp per group, where the FMA pipe does, the odd partners cost more
+            // than the instructions saved: 2^20 bodies 6.24 -> 6.26 ms).
+            if (MODE == 0 && TEAM && mixedb) {
+                float4 *const top = reinterpret_cast<float4 *>(S.stack + STACK + 4) - 2;   // pair p at top - 2 p
+                const int at = __popc(mixedb & lt);
+                if (mixed) {               // (x x' y y') (z z' size^2 size^2')
+                    float *f = reinterpret_cast<float *>(top - (at & ~1)) + (at & 1);
+                    f[0] = cx;
+                    f[2] = cy;
+                    f[4] = cz;
+                    f[6] = B.w;
+                }
+                __syncwarp();
+                const float4 *pair = top;
+                const float2 nx = splat2(-bx[0]), ny = splat2(-by[0]), nz = splat2(-bz[0]);
+                for (; mixedb; mixedb &= mixedb - 1, mixedb &= mixedb - 1) {
+                    // the candidates' lanes; a lone one is its own partner
+                    const unsigned rest = mixedb & (mixedb - 1);
+                    const int j0 = __ffs(mixedb) - 1, j1 = rest ? __ffs(rest) - 1 : j0;
+                    const float4 P0 = pair[0], P1 = pair[1];
+                    pair -= 2;
+                    const unsigned m0 = __shfl_sync(FULL, my_mask, j0), m1 = rest ? __shfl_sync(FULL, my_mask, j1) : 0u;
+                    const float2 dx = __fadd2_rn(lo2(P0), nx), dy = __fadd2_rn(hi2(P0), ny), dz = __fadd2_rn(lo2(P1), nz);
+                    const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                    const float2 t = __ffma2_rn(splat2(tol2), d2, make_float2(-P1.z, -P1.w));
+                    const float2 edge = __ffma2_rn(splat2(8e-6f * tol2), d2, splat2(cR));
+                    const bool in0 = (m0 >> lane) & 1u, in1 = (m1 >> lane) & 1u;
+                    bool op0 = t.x < 0.f, op1 = t.y < 0.f;
+                    const bool e0 = in0 && fabsf(t.x) <= edge.x, e1 = in1 && fabsf(t.y) <= edge.y;
+                    if (__any_sync(FULL, e0 || e1)) {
+                        // borderline: decide exactly as subdivp does, in FP64
+#pragma unroll 1
+                        for (int h = 0; h < 2; h++) {
+                            const int j = h ? j1 : j0;
+                            const int jn = __shfl_sync(FULL, my_node, j), jdepth = __shfl_sync(FULL, C.y, j) >> 8;
+                            if (h ? e1 : e0) {
+                                const double4_32a nd = g.nodeD[jn];
+                                const bool op =
+                                    open_exact(nd.x, nd.y, nd.z, xd[0], yd[0], zd[0], g.tol2d, g.box->dsq[jdepth]);
+                                (h ? op1 : op0) = op;
+                                nborder++;
+                            }
+                        }
+                    }
+                    const unsigned o0 = __ballot_sync(FULL, in0 && op0), o1 = __ballot_sync(FULL, in1 && op1);
+                    if (lane == j1) openm = o1;
+                    if (lane == j0) openm = o0;
+                }
+                if (mixed) accm = my_mask & ~openm;
             }
 
             // ---- push opened cells' child ranges ----
@@ -1163,6 +1261,22 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             }
         }
         __syncwarp();
+        // (s - c) + (x - e) in pairs of floats, the addition's error kept
+        auto add_pair = [](float &s, float &c, float x, float e) {
+            const float t = __fadd_rn(s, x), u = __fsub_rn(t, s);
+            c = __fsub_rn(c, __fsub_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(x, u)), e));
+            s = t;
+        };
+        if (NARROW) {
+            constexpr int k = BPL - 1;
+            for (int o = S.width; o < 32; o <<= 1) {
+                add_pair(sax[k], cax[k], __shfl_xor_sync(FULL, sax[k], o), __shfl_xor_sync(FULL, cax[k], o));
+                add_pair(say[k], cay[k], __shfl_xor_sync(FULL, say[k], o), __shfl_xor_sync(FULL, cay[k], o));
+                add_pair(saz[k], caz[k], __shfl_xor_sync(FULL, saz[k], o), __shfl_xor_sync(FULL, caz[k], o));
+                add_pair(sphi[k], cphi[k], __shfl_xor_sync(FULL, sphi[k], o), __shfl_xor_sync(FULL, cphi[k], o));
+            }
+            valid[k] = valid[k] && lane < S.width;
+        }
         if (TEAM) {
             // the warps' sums, in their (no longer used) list areas, added in warp
             // order by the first one: pairs of floats, each addition's error kept
@@ -1174,20 +1288,15 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             }
             __syncthreads();
             if (wid > 0) continue;
-            auto add = [](float &s, float &c, float x, float e) {      // (s - c) + (x - e)
-                const float t = __fadd_rn(s, x), u = __fsub_rn(t, s);
-                c = __fsub_rn(c, __fsub_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(x, u)), e));
-                s = t;
-            };
 #pragma unroll
             for (int k = 0; k < BPL; k++) {
                 for (int w = 1; w < W; w++) {
                     const WarpSmem &R = reinterpret_cast<const WarpSmem *>(smem_raw)[w];
                     const float4 a = (&R.bp[0][0])[2 * (lane + 32 * k)], e = (&R.bp[0][0])[2 * (lane + 32 * k) + 1];
-                    add(sax[k], cax[k], a.x, e.x);
-                    add(say[k], cay[k], a.y, e.y);
-                    add(saz[k], caz[k], a.z, e.z);
-                    add(sphi[k], cphi[k], a.w, e.w);
+                    add_pair(sax[k], cax[k], a.x, e.x);
+                    add_pair(say[k], cay[k], a.y, e.y);
+                    add_pair(saz[k], caz[k], a.z, e.z);
+                    add_pair(sphi[k], cphi[k], a.w, e.w);
                     if (COUNT) {
                         const int2 q = reinterpret_cast<const int2 *>(&R.cp[0][0])[lane + 32 * k];
                         myb[k] += q.x;
