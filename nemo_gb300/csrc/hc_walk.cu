@@ -40,6 +40,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include "hc_internal.cuh"
 #include "hc_mlp.cuh"
 
@@ -637,7 +638,8 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
 #pragma unroll
             for (int k = 0; k < BPL; k++) nphi[k] = ax[k] = ay[k] = az[k] = splat2(0.f);
             const float2 e2 = splat2(eps2);
-            auto eval = [&](const float4 H0, const float4 H1, const float4 L0, const float4 L1, int k, int self) {
+            auto eval = [&](auto normal, const float4 H0, const float4 H1, const float4 L0, const float4 L1, int k,
+                            int self) {
                 const float2 dx = __fadd2_rn(__fadd2_rn(lo2(H0), splat2(-bx[k])), __fadd2_rn(lo2(L0), splat2(-blx[k])));
                 const float2 dy = __fadd2_rn(__fadd2_rn(hi2(H0), splat2(-by[k])), __fadd2_rn(hi2(L0), splat2(-bly[k])));
                 const float2 dz = __fadd2_rn(__fadd2_rn(lo2(H1), splat2(-bz[k])), __fadd2_rn(lo2(L1), splat2(-blz[k])));
@@ -650,7 +652,8 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                     b0 = __float_as_int(L1.z) != self;
                     b1 = __float_as_int(L1.w) != self;
                 }
-                const float2 w = make_float2(b0 ? rsqrtf(r2.x) : 0.f, b1 ? rsqrtf(r2.y) : 0.f);
+                constexpr bool N = decltype(normal)::value;
+                const float2 w = make_float2(b0 ? rsqrt_sq<N>(r2.x) : 0.f, b1 ? rsqrt_sq<N>(r2.y) : 0.f);
                 const float2 mr = __fmul2_rn(hi2(H1), w);
                 const float2 mr3 = __fmul2_rn(mr, __fmul2_rn(w, w));
                 nphi[k] = __fadd2_rn(nphi[k], mr);
@@ -660,19 +663,23 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                 if (COUNT) myb[k] += (int)b0 + (int)b1;
             };
             const int fused = NARROW && S.width < 32 ? 1 : nact;       // bodies per lane evaluated together
-            for (int p = 0; p < (nb + 1) >> 1; p++) {
-                const float4 H0 = S.bp[p][0], H1 = S.bp[p][1], L0 = S.bp[p][2], L1 = S.bp[p][3];
+            auto run = [&](auto normal) {
+                for (int p = 0; p < (nb + 1) >> 1; p++) {
+                    const float4 H0 = S.bp[p][0], H1 = S.bp[p][1], L0 = S.bp[p][2], L1 = S.bp[p][3];
 #pragma unroll
-                for (int k = 0; k < BPL; k++) {
-                    if (k > 0 && k >= fused) continue;
-                    eval(H0, H1, L0, L1, k, lane + 32 * k);
+                    for (int k = 0; k < BPL; k++) {
+                        if (k > 0 && k >= fused) continue;
+                        eval(normal, H0, H1, L0, L1, k, lane + 32 * k);
+                    }
                 }
-            }
-            if (NARROW && fused < nact) {
-                const int wd = S.width, self = 32 + (lane & (wd - 1));
-                for (int r = 0, p = lane / wd; r < rounds; r++, p += 32 / wd)
-                    eval(S.bp[p][0], S.bp[p][1], S.bp[p][2], S.bp[p][3], BPL - 1, self);
-            }
+                if (NARROW && fused < nact) {
+                    const int wd = S.width, self = 32 + (lane & (wd - 1));
+                    for (int r = 0, p = lane / wd; r < rounds; r++, p += 32 / wd)
+                        eval(normal, S.bp[p][0], S.bp[p][1], S.bp[p][2], S.bp[p][3], BPL - 1, self);
+                }
+            };
+            if (eps2 >= FLT_MIN) run(std::true_type{});
+            else run(std::false_type{});
 #pragma unroll
             for (int k = 0; k < BPL; k++) {
                 if (COUNT && MODE != 0 && (nb & 1)) myb[k] -= 1;      // the pad counted as a body
@@ -693,12 +700,13 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
 #pragma unroll
             for (int k = 0; k < BPL; k++) nphi[k] = ax[k] = ay[k] = az[k] = splat2(0.f);
             const float2 e2 = splat2(eps2);
-            auto eval = [&](const float4 P0, const float4 P1, const float4 Q0, const float4 Q1, const float4 Q2, bool m0,
-                            bool m1, int k) {
+            auto eval = [&](auto normal, const float4 P0, const float4 P1, const float4 Q0, const float4 Q1,
+                            const float4 Q2, bool m0, bool m1, int k) {
                 const float2 dx = __fadd2_rn(lo2(P0), splat2(-bx[k])), dy = __fadd2_rn(hi2(P0), splat2(-by[k])),
                              dz = __fadd2_rn(lo2(P1), splat2(-bz[k]));
                 const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-                float2 w = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+                constexpr bool N = decltype(normal)::value;
+                float2 w = make_float2(rsqrt_sq<N>(r2.x), rsqrt_sq<N>(r2.y));
                 const float2 rinv2 = __fmul2_rn(w, w);
                 if (MASKED) w = make_float2(m0 ? w.x : 0.f, m1 ? w.y : 0.f);
                 const float2 mr = __fmul2_rn(hi2(P1), w);            // m / r (0 for a masked lane)
@@ -726,41 +734,45 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                 az[k] = __ffma2_rn(c, dz, __ffma2_rn(r5, qz, az[k]));
             };
             const int fused = NARROW && S.width < 32 ? 1 : nact;       // bodies per lane evaluated together
+            auto run = [&](auto normal) {
 #pragma unroll 2
-            for (int p = 0; p < (nc + 1) >> 1; p++) {
-                const float4 P0 = S.cp[p][0], P1 = S.cp[p][1];
-                bool m0 = true, m1 = true;
-                if (MASKED) {
-                    const uint2 mk = S.cmask[p];
-                    m0 = mk.x & lanebit;
-                    m1 = mk.y & lanebit;
-                    if (COUNT) myc[0] += (int)m0 + (int)m1;
-                }
-                float4 Q0, Q1, Q2;
-                if (QUAD) {
-                    Q0 = S.cp[p][2];
-                    Q1 = S.cp[p][3];
-                    Q2 = S.cp[p][4];
-                }
-#pragma unroll
-                for (int k = 0; k < BPL; k++) {
-                    if (k > 0 && k >= fused) continue;
-                    eval(P0, P1, Q0, Q1, Q2, m0, m1, k);
-                }
-            }
-            if (NARROW && fused < nact) {
-                const int wd = S.width;
-#pragma unroll 2
-                for (int r = 0, p = lane / wd; r < rounds; r++, p += 32 / wd) {
+                for (int p = 0; p < (nc + 1) >> 1; p++) {
+                    const float4 P0 = S.cp[p][0], P1 = S.cp[p][1];
+                    bool m0 = true, m1 = true;
+                    if (MASKED) {
+                        const uint2 mk = S.cmask[p];
+                        m0 = mk.x & lanebit;
+                        m1 = mk.y & lanebit;
+                        if (COUNT) myc[0] += (int)m0 + (int)m1;
+                    }
                     float4 Q0, Q1, Q2;
                     if (QUAD) {
                         Q0 = S.cp[p][2];
                         Q1 = S.cp[p][3];
                         Q2 = S.cp[p][4];
                     }
-                    eval(S.cp[p][0], S.cp[p][1], Q0, Q1, Q2, true, true, BPL - 1);
+#pragma unroll
+                    for (int k = 0; k < BPL; k++) {
+                        if (k > 0 && k >= fused) continue;
+                        eval(normal, P0, P1, Q0, Q1, Q2, m0, m1, k);
+                    }
                 }
-            }
+                if (NARROW && fused < nact) {
+                    const int wd = S.width;
+#pragma unroll 2
+                    for (int r = 0, p = lane / wd; r < rounds; r++, p += 32 / wd) {
+                        float4 Q0, Q1, Q2;
+                        if (QUAD) {
+                            Q0 = S.cp[p][2];
+                            Q1 = S.cp[p][3];
+                            Q2 = S.cp[p][4];
+                        }
+                        eval(normal, S.cp[p][0], S.cp[p][1], Q0, Q1, Q2, true, true, BPL - 1);
+                    }
+                }
+            };
+            if (eps2 >= FLT_MIN) run(std::true_type{});
+            else run(std::false_type{});
 #pragma unroll
             for (int k = 0; k < BPL; k++) {
                 if (COUNT && !MASKED) myc[k] += nc;

@@ -2,7 +2,7 @@
 gives every lane one body and lays its other 1 to 32 over 8, 16 or 32 lanes, the
 free lanes taking other entries of the list; the walk that counts per body keeps
 one entry for all lanes.  Both decide alike, so their forces differ by the order
-of FP32 sums."""
+of FP32 sums.  And of the softening's two forms of the inverse root."""
 import numpy as np
 import pytest
 
@@ -20,15 +20,16 @@ def hc():
     return hackcode
 
 
-def _run(hc, m, pos, criterion, theta, quad, prev, count):
+def _run(hc, m, pos, criterion, theta, quad, prev, count, eps=0.02):
     n = len(m)
     ph = np.zeros((n, 2, 3))
     ph[:, 0] = pos
-    with hc.Context(n, tol=0.6, eps=0.02, usequad=quad, count_per_body=count) as ctx:
+    with hc.Context(n, tol=0.6, eps=eps, usequad=quad, count_per_body=count) as ctx:
         ctx.upload(m, ph)
         ctx.set_box((-8.0, -8.0, -8.0), 16.0)
         ctx.set_grouping("tree")
-        ctx.set_criterion(criterion, theta)
+        if criterion != "body":
+            ctx.set_criterion(criterion, theta)
         ctx.set_forces(prev)
         ctx.evaluate()
         _, acc, phi = ctx.download(phase=False)
@@ -56,3 +57,18 @@ def test_second_bodies_narrow_and_wide(hc, clusters, k, criterion, theta, quad):
     size = np.linalg.norm(a1, axis=1) + scale
     assert (np.linalg.norm(a - a1, axis=1) <= 4e-6 * size / 0.02).all()
     assert np.median(np.linalg.norm(a - a1, axis=1) / np.linalg.norm(a1, axis=1)) <= 1e-6
+
+
+@pytest.mark.parametrize("criterion,theta", [("body", 0.0), ("group", 0.6), ("error", 0.05)])
+@pytest.mark.parametrize("quad", [False, True])
+def test_softenings_on_both_sides_of_the_smallest_normal_square(hc, criterion, theta, quad):
+    """1e-19 squared is a denormal FP32 number and 1.1e-19 squared is not: the
+    lists take their inverse roots by different instructions.  Neither changes a
+    separation of these bodies (1e-19 against 1e-7 and more), so nor any bit."""
+    rng = np.random.default_rng(3)
+    pos = rng.normal(0.0, 1.0, (20000, 3)).clip(-7.5, 7.5)
+    m = rng.uniform(0.5, 1.5, len(pos)) / len(pos)
+    prev = -pos / (np.linalg.norm(pos, axis=1)[:, None] + 0.3) ** 3
+    a, p = _run(hc, m, pos, criterion, theta, quad, prev, False, eps=1.0e-19)
+    a1, p1 = _run(hc, m, pos, criterion, theta, quad, prev, False, eps=1.1e-19)
+    assert np.isfinite(p).all() and np.array_equal(p, p1) and np.array_equal(a, a1)
