@@ -368,7 +368,6 @@ int hc_create(hc_ctx **out, int64_t nbody, const hc_params *params)
     HC_CUDA(cudaMemset(c->st, 0, 2 * sizeof(hc_status)));
     HC_CUDA(cudaMallocHost((void **)&c->h_diag, (64 + std::min<int64_t>(10 * c->n, HC_SMALL_COPY)) * sizeof(double)));
     c->h_small = c->h_diag + 64;
-    HC_TRY(hc_guard_setup(c));
     int r2 = hc_tree_setup(c);
     return r2 != HC_OK ? r2 : hc_walk_setup(c);
 }

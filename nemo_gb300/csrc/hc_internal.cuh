@@ -177,7 +177,6 @@ struct hc_ctx {
     int64_t guard_n;                      // sampled bodies (0: off)
     double guard_rms_max;
     int guard_slices;                     // source slices of the direct sum
-    int guard_smem;                       // dynamic shared memory reserved per guard block (residency)
     int64_t *guard_idx;                   // sampled body indices (ascending)
     float4 *guard_part;                   // [slices][guard_n] partial accelerations
     struct hc_guard_state *guard;
@@ -252,7 +251,6 @@ void hc_guard_launch(hc_ctx *c);
 // the guard in two parts: the sampled direct sum (on any stream), then the
 // comparison with the walk's forces and the check (on c->stream)
 void hc_guard_direct_launch(hc_ctx *c, cudaStream_t s);
-int hc_guard_setup(hc_ctx *c);
 void hc_guard_check_launch(hc_ctx *c);
 int hc_fma_peak_impl(hc_ctx *c, double *tflops);
 
