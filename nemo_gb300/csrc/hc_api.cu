@@ -75,7 +75,7 @@ void free_all(hc_ctx *c)
                     c->tax, c->tay, c->taz, c->tphi, c->tkhi[0], c->tkhi[1], c->tkval[0], c->tkval[1], c->thist};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    void *mptrs[] = {c->mlp_p, c->mlp_m, c->mlp_v, c->mlp_grad, c->mlp_loss, c->mlp_gpart, c->mlp_lpart,
+    void *mptrs[] = {c->mlp_p, c->mlp_m, c->mlp_v, c->mlp_grad, c->mlp_loss, c->mlp_gpart, c->mlp_image, c->mlp_lpart,
                      c->mlp_packed, c->sample_count, c->sample_x, c->sample_amin, c->sample_y, c->sample_rel,
                      c->sample_w, c->sample_group, c->sample_node, c->guard_idx, c->guard_part, c->guard,
                      c->rcrit2, c->phi_ext, c->split.ctl, c->split.out, c->split.task[0], c->split.task[1],
@@ -129,7 +129,8 @@ int alloc_all(hc_ctx *c)
     HC_TRY(dalloc(c, &c->mlp_grad, hc_mlp_nparams()));
     HC_TRY(dalloc(c, &c->mlp_loss, 1));
     c->mlp_gcap = 128;
-    HC_TRY(dalloc(c, &c->mlp_gpart, (int64_t)c->mlp_gcap * hc_mlp_nparams()));
+    HC_TRY(dalloc(c, &c->mlp_gpart, hc_mlp_partials(c->mlp_gcap)));
+    HC_TRY(dalloc(c, &c->mlp_image, hc_mlp_image_floats()));
     HC_TRY(dalloc(c, &c->mlp_lpart, c->mlp_gcap));
     {
         char *pk = nullptr;
@@ -1239,6 +1240,7 @@ int hc_learn_gradient(hc_ctx *ctx, const float *x, const float *y, const float *
         wsum = 0;
         for (int64_t i = 0; i < n; i++) wsum += w[i];
     }
+    HC_TRY(hc_mlp_train_setup(c));
     HC_TRY(hc_mlp_grad_impl(c, dx, dy, w ? dw : nullptr, n, (float)(1.0 / wsum), c->mlp_grad, c->mlp_loss));
     HC_CUDA(cudaMemcpyAsync(grad, c->mlp_grad, sizeof(float) * hc_mlp_nparams(), cudaMemcpyDeviceToHost,
                             c->stream));
@@ -1372,6 +1374,22 @@ __global__ void k_gather_samples(const int *perm, int n, const float *x, const f
     }
 }
 
+// Sum of each mini-batch's weights (FP64), a block per batch.
+__global__ void __launch_bounds__(256) k_batch_weights(const float *w, int n, int batch, double *sum)
+{
+    __shared__ double red[256];
+    const int b0 = blockIdx.x * batch, nb = n - b0 < batch ? n - b0 : batch;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nb; i += 256) s += w[b0 + i];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o; o >>= 1) {
+        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) sum[blockIdx.x] = red[0];
+}
+
 int hc_learn_train(hc_ctx *ctx, int epochs, int batch, double lr, uint64_t seed, double *loss)
 {
     if (!ctx || epochs < 1 || batch < 64 || !(lr > 0)) return HC_ERR_ARG;
@@ -1386,6 +1404,8 @@ int hc_learn_train(hc_ctx *ctx, int epochs, int batch, double lr, uint64_t seed,
     HC_TRY(staging(c, c->stage, (int64_t)n * 8 + 8));
     float *sx = (float *)c->stage.d, *sy = sx + 12 * (int64_t)n, *sw = sy + n;
     int *dperm = (int *)(sw + n);
+    const int batches = (n + batch - 1) / batch;              // at most n / 64: they fit the permutation's place
+    double *dsum = (double *)(((uintptr_t)dperm + 7) & ~(uintptr_t)7);
     std::vector<int> perm(n);
     for (int i = 0; i < n; i++) perm[i] = i;
     uint64_t st = seed * 2862933555777941757ULL + 3037000493ULL;
@@ -1396,20 +1416,21 @@ int hc_learn_train(hc_ctx *ctx, int epochs, int batch, double lr, uint64_t seed,
     }
     HC_CUDA(cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
     k_gather_samples<<<hc_grid(n, 256), 256, 0, c->stream>>>(dperm, n, c->sample_x, c->sample_y, c->sample_w, sx, sy, sw);
+    k_batch_weights<<<batches, 256, 0, c->stream>>>(sw, n, batch, dsum);
+    c->launches += 2;
     double last = 0;
-    std::vector<float> wv(n);
-    HC_CUDA(cudaMemcpyAsync(wv.data(), sw, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
+    std::vector<double> wsum(batches);
+    HC_CUDA(cudaMemcpyAsync(wsum.data(), dsum, sizeof(double) * batches, cudaMemcpyDeviceToHost, c->stream));
     HC_CUDA(cudaStreamSynchronize(c->stream));
+    HC_TRY(hc_mlp_train_setup(c));
     for (int e = 0; e < epochs; e++) {
         double esum = 0, wtot = 0;
         for (int b0 = 0; b0 + 64 <= n; b0 += batch) {
             const int nb = std::min(batch, n - b0);
-            double ws = 0;
-            for (int i = 0; i < nb; i++) ws += wv[b0 + i];
-            HC_TRY(hc_mlp_grad_impl(c, sx + 12 * (int64_t)b0, sy + b0, sw + b0, nb, (float)(1.0 / ws), c->mlp_grad,
-                                    c->mlp_loss));
+            const double ws = wsum[b0 / batch];
             c->mlp_step++;
-            HC_TRY(hc_mlp_adam_impl(c, c->mlp_grad, (float)lr, c->mlp_step));
+            HC_TRY(hc_mlp_step_impl(c, sx + 12 * (int64_t)b0, sy + b0, sw + b0, nb, (float)(1.0 / ws), c->mlp_loss, (float)lr,
+                                    c->mlp_step));
             float l = 0;
             if (b0 + batch >= n - 63 || (b0 / batch) % 16 == 0) {
                 HC_CUDA(cudaMemcpyAsync(&l, c->mlp_loss, sizeof(float), cudaMemcpyDeviceToHost, c->stream));

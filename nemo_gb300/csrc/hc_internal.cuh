@@ -149,6 +149,7 @@ struct hc_ctx {
     struct MlpSmem *mlp_packed;           // BF16 image used by the walk
     float *mlp_p, *mlp_m, *mlp_v;         // FP32 master weights, Adam moments
     float *mlp_gpart, *mlp_lpart, *mlp_grad, *mlp_loss;
+    float *mlp_image;                     // the weights as the gradient kernel lays them out
     int mlp_gcap;                         // blocks of one training mini-batch
     int mlp_step;                         // Adam step count
     float mlp_threshold;
@@ -237,7 +238,11 @@ int hc_mlp_pack(hc_ctx *c);
 int hc_mlp_infer_impl(hc_ctx *c, const float *x_dev, int64_t n, float *logits_dev);
 int hc_mlp_grad_impl(hc_ctx *c, const float *x, const float *y, const float *w, int64_t n, float inv_norm,
                      float *grad_dev, float *loss_dev);
-int hc_mlp_adam_impl(hc_ctx *c, const float *grad_dev, float lr, int t);
+int hc_mlp_step_impl(hc_ctx *c, const float *x, const float *y, const float *w, int64_t n, float inv_norm, float *loss_dev,
+                     float lr, int t);
+int hc_mlp_train_setup(hc_ctx *c);
+int64_t hc_mlp_partials(int blocks);
+int64_t hc_mlp_image_floats();
 int hc_relabel_impl(hc_ctx *c, float thr);
 // step (hc_step.cu)
 void hc_kick_drift(hc_ctx *c, double dt);

@@ -8,6 +8,7 @@
 // weights and activations to BF16 exactly where inference does (straight-
 // through gradients), so the trained network is the one the walk evaluates.
 #include <cmath>
+#include <cuda_pipeline_primitives.h>
 #include "hc_internal.cuh"
 #include "hc_mlp.cuh"
 
@@ -57,142 +58,303 @@ __global__ void k_mlp_infer(const MlpSmem *params, const float *x, int64_t n, fl
 
 // Gradient of the mean (weighted) binary cross-entropy over rows [0, n) of
 // one mini-batch: each block takes TB rows and writes its partial gradient
-// (NP floats) and loss.
+// (NP floats, NPS apart) and loss.
+//
+// A batch of 4096 rows is 64 blocks and a chain of 64 x 64 x 64 products (the
+// second layer, its transpose, its weights' gradient): bound by the latency of
+// one block, and in the products by what shared memory returns.  A warp takes 8
+// rows of a product, whose operand is one address for all lanes (half the
+// cycles of distinct ones), and a lane two columns: 3400 cycles a product, 4100
+// with a 4 x 4 tile per thread.  Operands needed along both dimensions are
+// stored twice, in rows of LD floats so that neither store meets a bank more
+// than twice; the weights come rounded and in that layout from the step before
+// (MlpImage: 900 cycles to load, 4700 from the parameters).  Pre-activations
+// stay in registers from the forward to the backward pass.  Every sum keeps one
+// order (inputs, rows, blocks ascending).  A step of 4096 rows, gradient and
+// update: 46 us with one output at a time and operands strided over the banks,
+// 14 us so.
 constexpr int TB = 64;
 constexpr int GT = 256;
+constexpr int LD = MLP_H + 4;
+constexpr int NPS = (NP + 3) / 4 * 4;
 
-__global__ void __launch_bounds__(GT) k_mlp_grad(const float *p, const float *x, const float *y, const float *wt,
+struct alignas(16) MlpImage {                  // weights bf16-rounded
+    float W2[MLP_H * LD], W2T[MLP_H * LD];     // W2[j][k], W2T[k][j]
+    float W1T[MLP_IN * LD];                    // W1[k][j]
+    float W3[MLP_H], b1[MLP_H], b2[MLP_H], b3[4];
+};
+
+struct GradSmem {
+    MlpImage P;                                // W2T later dz1[s][k]
+    float H1[TB * LD], H1T[MLP_H * LD];        // H1[s][k], H1T[k][s]
+    float D2[TB * LD], D2T[MLP_H * LD];        // dz2[s][j], dz2[j][s]
+    float H2T[MLP_H * LD];                     // H2[j][s]
+    float XT[MLP_IN * LD], X[TB * 16];         // inputs [k][s]; [s][k], then 1 and zeros
+    float D[TB], red[32];                      // D: dL/dz3
+};
+static_assert(sizeof(GradSmem) <= 227 * 1024, "shared memory of a block");
+
+__device__ __forceinline__ void image_put(MlpImage *m, int i, float v)
+{
+    if (i < OFF_B1) {
+        m->W1T[i % MLP_IN * LD + i / MLP_IN] = bf(v);
+    } else if (i < OFF_W2) {
+        m->b1[i - OFF_B1] = v;
+    } else if (i < OFF_B2) {
+        const int j = (i - OFF_W2) / MLP_H, k = (i - OFF_W2) % MLP_H;
+        m->W2[j * LD + k] = m->W2T[k * LD + j] = bf(v);
+    } else if (i < OFF_W3) {
+        m->b2[i - OFF_B2] = v;
+    } else if (i < OFF_B3) {
+        m->W3[i - OFF_W3] = bf(v);
+    } else {
+        m->b3[0] = v;
+    }
+}
+
+__global__ void k_mlp_image(const float *p, MlpImage *m)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < NP) image_put(m, i, p[i]);
+}
+
+// Programmatic dependent launch: a kernel of the training loop starts while its
+// predecessor drains, and waits here for all of it.
+__device__ __forceinline__ void wait_predecessor()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+
+// out[i][q] += sum over r < rows of a[r][i] b[r][q], r ascending: rows in
+// packed pairs (a scalar multiply-add holds the pipe as long as a packed one)
+template <int ROWS>
+__device__ __forceinline__ void tile_product(const float *a, const float *b, float (&out)[8][2])
+{
+    float2 o[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int q = 0; q < 2; q++) o[i][q] = make_float2(out[2 * i][q], out[2 * i + 1][q]);
+#pragma unroll 8
+    for (int r = 0; r < ROWS; r++) {
+        const float4 u0 = ld4(a + r * LD), u1 = ld4(a + r * LD + 4);
+        const float2 v = *reinterpret_cast<const float2 *>(b + r * LD);
+        const float2 u[4] = {lo2(u0), hi2(u0), lo2(u1), hi2(u1)};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            o[i][0] = __ffma2_rn(u[i], splat2(v.x), o[i][0]);
+            o[i][1] = __ffma2_rn(u[i], splat2(v.y), o[i][1]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            out[2 * i][q] = o[i][q].x;
+            out[2 * i + 1][q] = o[i][q].y;
+        }
+}
+
+// rows i of a tile (the lanes' pairs beside each other), and its transpose
+__device__ __forceinline__ void tile_rows(const float (&t)[8][2], float *rows)
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) *reinterpret_cast<float2 *>(rows + i * LD) = make_float2(t[i][0], t[i][1]);
+}
+__device__ __forceinline__ void tile_cols(const float (&t)[8][2], float *cols)
+{
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < 8; i += 4)
+            *reinterpret_cast<float4 *>(cols + q * LD + i) = make_float4(t[i][q], t[i + 1][q], t[i + 2][q], t[i + 3][q]);
+}
+
+#define TILE_EACH                                                                                                      \
+    _Pragma("unroll") for (int i = 0; i < 8; i++) _Pragma("unroll") for (int q = 0; q < 2; q++)
+
+__global__ void __launch_bounds__(GT) k_mlp_grad(const MlpImage *img, const float *x, const float *y, const float *wt,
                                                  int64_t n, float inv_norm, float *gpart, float *lpart)
 {
-    extern __shared__ float sm[];
-    float *W2 = sm;                          // [64][64] (bf16-rounded)
-    float *X = W2 + MLP_H * MLP_H;           // [TB][12]
-    float *Z1 = X + TB * MLP_IN;             // [TB][64] pre-activations
-    float *H1 = Z1 + TB * MLP_H;             // [TB][64]
-    float *Z2 = H1 + TB * MLP_H;
-    float *H2 = Z2 + TB * MLP_H;
-    float *D = H2 + TB * MLP_H;              // [TB] dL/dz3
-    float *W1 = D + TB;                      // [64][12]
-    float *W3 = W1 + MLP_H * MLP_IN;         // [64]
-    float *red = W3 + MLP_H;                 // [GT]
-    const int tid = threadIdx.x;
+    extern __shared__ float4 grad_sm[];
+    GradSmem &S = *reinterpret_cast<GradSmem *>(grad_sm);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int R = 8 * w, C = 2 * lane;                    // this thread's tile: rows R.., columns C..
     const int64_t r0 = (int64_t)blockIdx.x * TB;
-    for (int i = tid; i < MLP_H * MLP_H; i += GT) W2[i] = bf(p[OFF_W2 + i]);
-    for (int i = tid; i < MLP_H * MLP_IN; i += GT) W1[i] = bf(p[OFF_W1 + i]);
-    for (int i = tid; i < MLP_H; i += GT) W3[i] = bf(p[OFF_W3 + i]);
-    for (int i = tid; i < TB * MLP_IN; i += GT) {
-        const int64_t r = r0 + i / MLP_IN;
-        X[i] = r < n ? bf(x[r * MLP_IN + i % MLP_IN]) : 0.f;
+    // the rows do not depend on the step before
+    for (int i = tid; i < TB * 16; i += GT) {
+        const int k = i & 15;
+        const int64_t r = r0 + (i >> 4);
+        const float v = k < MLP_IN ? (r < n ? bf(x[r * MLP_IN + k]) : 0.f) : k == MLP_IN ? 1.f : 0.f;
+        S.X[i] = v;
+        if (k < MLP_IN) S.XT[k * LD + (i >> 4)] = v;
     }
-    __syncthreads();
-    // forward
-    for (int i = tid; i < TB * MLP_H; i += GT) {
-        const int s = i / MLP_H, j = i % MLP_H;
-        float z = p[OFF_B1 + j];
-        for (int k = 0; k < MLP_IN; k++) z = fmaf(W1[j * MLP_IN + k], X[s * MLP_IN + k], z);
-        Z1[i] = z;
-        H1[i] = bf(silu(z));
+    float yy = 0.f, ww = 0.f;
+    if (tid < TB && r0 + tid < n) {
+        yy = y[r0 + tid];
+        ww = wt ? wt[r0 + tid] : 1.f;
     }
+    wait_predecessor();
+    for (int i = tid; i < (int)(sizeof(MlpImage) / 16); i += GT)
+        __pipeline_memcpy_async(reinterpret_cast<float4 *>(&S.P) + i, reinterpret_cast<const float4 *>(img) + i, 16);
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
     __syncthreads();
-    for (int i = tid; i < TB * MLP_H; i += GT) {
-        const int s = i / MLP_H, j = i % MLP_H;
-        float z = p[OFF_B2 + j];
-        for (int k = 0; k < MLP_H; k++) z = fmaf(W2[j * MLP_H + k], H1[s * MLP_H + k], z);
-        Z2[i] = z;
-        H2[i] = bf(silu(z));
+    // forward: hidden units R.., rows C..
+    float z1[8][2], z2[8][2], t[8][2];
+    TILE_EACH
+    {
+        z1[i][q] = S.P.b1[R + i];
+        z2[i][q] = S.P.b2[R + i];
     }
+    tile_product<MLP_IN>(S.P.W1T + R, S.XT + C, z1);
+    TILE_EACH t[i][q] = bf(silu(z1[i][q]));
+    tile_rows(t, S.H1T + R * LD + C);
+    tile_cols(t, S.H1 + C * LD + R);
     __syncthreads();
-    float lsum = 0.f;
-    for (int s = tid; s < TB; s += GT) {
-        const int64_t r = r0 + s;
-        float z = p[OFF_B3];
-        for (int k = 0; k < MLP_H; k++) z = fmaf(W3[k], H2[s * MLP_H + k], z);
-        float d = 0.f;
-        if (r < n) {
-            const float yy = y[r], ww = wt ? wt[r] : 1.f;
+    tile_product<MLP_H>(S.P.W2T + R, S.H1T + C, z2);
+    TILE_EACH t[i][q] = bf(silu(z2[i][q]));
+    tile_rows(t, S.H2T + R * LD + C);
+    __syncthreads();
+    if (tid < TB) {
+        float z = S.P.b3[0];
+#pragma unroll 16
+        for (int k = 0; k < MLP_H; k++) z = fmaf(S.P.W3[k], S.H2T[k * LD + tid], z);
+        float d = 0.f, lsum = 0.f;
+        if (r0 + tid < n) {
             // BCE with logits: max(z,0) - z y + log(1 + exp(-|z|))
             lsum += ww * (fmaxf(z, 0.f) - z * yy + log1pf(__expf(-fabsf(z))));
             d = ww * (sig_out(z) - yy) * inv_norm;
         }
-        D[s] = d;
-    }
-    red[tid] = lsum;
-    __syncthreads();
-    // backward: dz2 = d * w3 * silu'(z2)  (stored over Z2)
-    for (int i = tid; i < TB * MLP_H; i += GT) {
-        const int s = i / MLP_H, j = i % MLP_H;
-        const float z = Z2[i], sg = sigm(z);
-        Z2[i] = D[s] * W3[j] * sg * (1.f + z * (1.f - sg));
+        S.D[tid] = d;
+        if (tid >= 32) S.red[lane] = lsum;
+        yy = lsum;                                   // the first warp's losses, added below
     }
     __syncthreads();
-    // dh1 = W2^T dz2 ; dz1 = dh1 * silu'(z1)  (stored over Z1)
-    for (int i = tid; i < TB * MLP_H; i += GT) {
-        const int s = i / MLP_H, k = i % MLP_H;
-        float dh = 0.f;
-        for (int j = 0; j < MLP_H; j++) dh = fmaf(W2[j * MLP_H + k], Z2[s * MLP_H + j], dh);
-        const float z = Z1[i], sg = sigm(z);
-        Z1[i] = dh * sg * (1.f + z * (1.f - sg));
+    // backward: dz2 = d * w3 * silu'(z2)
+    TILE_EACH
+    {
+        const float z = z2[i][q], sg = sigm(z);
+        t[i][q] = S.D[C + q] * S.P.W3[R + i] * sg * (1.f + z * (1.f - sg));
     }
+    tile_rows(t, S.D2T + R * LD + C);
+    tile_cols(t, S.D2 + C * LD + R);
+    if (w == 0) {
+        float l = yy + S.red[lane];
+        for (int o = 16; o; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+        if (lane == 0) lpart[blockIdx.x] = l;
+    }
+    __syncthreads();
+    // dh1 = W2^T dz2 ; dz1 = dh1 * silu'(z1), over W2T
+    TILE_EACH t[i][q] = 0.f;
+    tile_product<MLP_H>(S.P.W2 + R, S.D2T + C, t);
+    TILE_EACH
+    {
+        const float z = z1[i][q], sg = sigm(z);
+        t[i][q] = t[i][q] * sg * (1.f + z * (1.f - sg));
+    }
+    float *dz1 = S.P.W2T;
+    tile_cols(t, dz1 + C * LD + R);
     __syncthreads();
     // parameter gradients (sums over this block's rows)
-    float *gp = gpart + (int64_t)blockIdx.x * NP;
-    for (int i = tid; i < NP; i += GT) {
-        float g = 0.f;
-        if (i < OFF_B1) {
-            const int j = i / MLP_IN, k = i % MLP_IN;
-            for (int s = 0; s < TB; s++) g = fmaf(Z1[s * MLP_H + j], X[s * MLP_IN + k], g);
-        } else if (i < OFF_W2) {
-            const int j = i - OFF_B1;
-            for (int s = 0; s < TB; s++) g += Z1[s * MLP_H + j];
-        } else if (i < OFF_B2) {
-            const int j = (i - OFF_W2) / MLP_H, k = (i - OFF_W2) % MLP_H;
-            for (int s = 0; s < TB; s++) g = fmaf(Z2[s * MLP_H + j], H1[s * MLP_H + k], g);
-        } else if (i < OFF_W3) {
-            const int j = i - OFF_B2;
-            for (int s = 0; s < TB; s++) g += Z2[s * MLP_H + j];
-        } else if (i < OFF_B3) {
-            const int k = i - OFF_W3;
-            for (int s = 0; s < TB; s++) g = fmaf(D[s], H2[s * MLP_H + k], g);
-        } else {
-            for (int s = 0; s < TB; s++) g += D[s];
+    float *gp = gpart + (int64_t)blockIdx.x * NPS;
+    TILE_EACH t[i][q] = 0.f;
+    tile_product<TB>(S.D2 + R, S.H1 + C, t);
+#pragma unroll
+    for (int i = 0; i < 8; i++) *reinterpret_cast<float2 *>(gp + OFF_W2 + (R + i) * MLP_H + C) = make_float2(t[i][0], t[i][1]);
+    {
+        // first layer: units R.., input `lane`; the column of ones gives the biases
+        float2 g[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) g[i] = splat2(0.f);
+#pragma unroll 8
+        for (int s = 0; s < TB; s++) {
+            const float4 u0 = ld4(dz1 + s * LD + R), u1 = ld4(dz1 + s * LD + R + 4);
+            const float2 v = splat2(S.X[s * 16 + (lane & 15)]);
+            g[0] = __ffma2_rn(lo2(u0), v, g[0]);
+            g[1] = __ffma2_rn(hi2(u0), v, g[1]);
+            g[2] = __ffma2_rn(lo2(u1), v, g[2]);
+            g[3] = __ffma2_rn(hi2(u1), v, g[3]);
         }
-        gp[i] = g;
+        if (lane <= MLP_IN) {
+            const bool wt1 = lane < MLP_IN;
+            float *o = gp + (wt1 ? OFF_W1 + R * MLP_IN + lane : OFF_B1 + R);
+            const int step = wt1 ? MLP_IN : 1;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                o[2 * i * step] = g[i].x;
+                o[(2 * i + 1) * step] = g[i].y;
+            }
+        }
     }
-    for (int o = GT / 2; o > 0; o >>= 1) {
-        if (tid < o) red[tid] += red[tid + o];
-        __syncthreads();
-    }
-    if (tid == 0) lpart[blockIdx.x] = red[0];
-}
-
-__global__ void k_mlp_reduce(const float *gpart, int nblk, float *grad, const float *lpart, float *loss)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NP; i += gridDim.x * blockDim.x) {
+    // the other vectors: two warps each for b2 and W3, one lane for b3
+    if (w < 2) {
         float g = 0.f;
-        for (int b = 0; b < nblk; b++) g += gpart[(int64_t)b * NP + i];
-        grad[i] = g;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && loss) {
-        float l = 0.f;
-        for (int b = 0; b < nblk; b++) l += lpart[b];
-        *loss = l;
+#pragma unroll 16
+        for (int s = 0; s < TB; s++) g += S.D2[s * LD + tid];
+        gp[OFF_B2 + tid] = g;
+    } else if (w < 4) {
+        const int k = tid - 64;
+        float g = 0.f;
+#pragma unroll 4
+        for (int s = 0; s < TB; s += 4) {
+            const float4 h = ld4(S.H2T + k * LD + s), d = ld4(S.D + s);
+            g = fmaf(d.x, h.x, g);
+            g = fmaf(d.y, h.y, g);
+            g = fmaf(d.z, h.z, g);
+            g = fmaf(d.w, h.w, g);
+        }
+        gp[OFF_W3 + k] = g;
+    } else if (tid == 128) {
+        float g = 0.f;
+#pragma unroll 16
+        for (int s = 0; s < TB; s++) g += S.D[s];
+        gp[OFF_B3] = g;
     }
 }
 
-__global__ void k_adam(float *p, const float *grad, float *m, float *v, float lr, float b1, float b2, float eps, int t)
+__device__ __forceinline__ float sum_blocks(const float *part, int nblk, int64_t stride)
 {
+    float g = 0.f;
+#pragma unroll 32
+    for (int b = 0; b < nblk; b++) g += part[b * stride];
+    return g;
+}
+
+constexpr int RT = 32;                                   // one warp per block: a parameter per thread over all SMs
+constexpr int RB = (NP + RT - 1) / RT + 1;               // the last block adds the losses
+
+__global__ void __launch_bounds__(RT) k_mlp_reduce(const float *gpart, int nblk, float *grad, const float *lpart, float *loss)
+{
+    const int i = blockIdx.x * RT + threadIdx.x;
+    if (i < NP) grad[i] = sum_blocks(gpart + i, nblk, NPS);
+    if (blockIdx.x == RB - 1 && threadIdx.x == 0 && loss) *loss = sum_blocks(lpart, nblk, 1);
+}
+
+// the gradient's sum over the blocks and Adam's step
+__global__ void __launch_bounds__(RT) k_mlp_adam(const float *gpart, int nblk, const float *lpart, float *loss, float *p, float *m,
+                                                 float *v, MlpImage *img, float lr, float b1, float b2, float eps, int t)
+{
+    const int i = blockIdx.x * RT + threadIdx.x;
     const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NP; i += gridDim.x * blockDim.x) {
-        const float g = grad[i];
-        m[i] = b1 * m[i] + (1.f - b1) * g;
-        v[i] = b2 * v[i] + (1.f - b2) * g * g;
-        p[i] -= lr * (m[i] / c1) / (sqrtf(v[i] / c2) + eps);
+    wait_predecessor();
+    if (blockIdx.x == RB - 1) {
+        if (threadIdx.x == 0) *loss = sum_blocks(lpart, nblk, 1);
+        return;
     }
-}
-
-constexpr size_t grad_smem()
-{
-    return sizeof(float) * (MLP_H * MLP_H + TB * MLP_IN + 4 * TB * MLP_H + TB + MLP_H * MLP_IN + MLP_H + GT);
+    if (i >= NP) return;
+    const float mi = m[i], vi = v[i], pi = p[i];
+    const float g = sum_blocks(gpart + i, nblk, NPS);
+    const float mn = b1 * mi + (1.f - b1) * g;
+    const float vn = b2 * vi + (1.f - b2) * g * g;
+    m[i] = mn;
+    v[i] = vn;
+    const float pn = pi - lr * (mn / c1) / (sqrtf(vn / c2) + eps);
+    p[i] = pn;
+    image_put(img, i, pn);
 }
 
 }  // namespace
@@ -214,25 +376,57 @@ int hc_mlp_infer_impl(hc_ctx *c, const float *x_dev, int64_t n, float *logits_de
     return HC_OK;
 }
 
+int64_t hc_mlp_partials(int blocks) { return (int64_t)blocks * NPS; }
+
+int64_t hc_mlp_image_floats() { return sizeof(MlpImage) / sizeof(float); }
+
+// Before a gradient or a training: the image of the current parameters.  The
+// attribute is set here, per call of the library: it belongs to the current device,
+// and a process may drive contexts on several
+int hc_mlp_train_setup(hc_ctx *c)
+{
+    HC_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem)));
+    k_mlp_image<<<(NP + 255) / 256, 256, 0, c->stream>>>(c->mlp_p, reinterpret_cast<MlpImage *>(c->mlp_image));
+    c->launches++;
+    return HC_OK;
+}
+
 // mean-loss gradient over rows [0, n) (norm = 1/sum of weights), into grad_dev
 int hc_mlp_grad_impl(hc_ctx *c, const float *x, const float *y, const float *w, int64_t n, float inv_norm,
                      float *grad_dev, float *loss_dev)
 {
-    // per call: the attribute belongs to the current device, and a process may
-    // drive contexts on several
-    HC_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_smem()));
     const int nblk = (int)((n + TB - 1) / TB);
     if (nblk > c->mlp_gcap) return HC_ERR_ARG;
-    k_mlp_grad<<<nblk, GT, grad_smem(), c->stream>>>(c->mlp_p, x, y, w, n, inv_norm, c->mlp_gpart, c->mlp_lpart);
-    k_mlp_reduce<<<(NP + 255) / 256, 256, 0, c->stream>>>(c->mlp_gpart, nblk, grad_dev, c->mlp_lpart, loss_dev);
+    k_mlp_grad<<<nblk, GT, sizeof(GradSmem), c->stream>>>(reinterpret_cast<const MlpImage *>(c->mlp_image), x, y, w, n, inv_norm, c->mlp_gpart, c->mlp_lpart);
+    k_mlp_reduce<<<RB, RT, 0, c->stream>>>(c->mlp_gpart, nblk, grad_dev, c->mlp_lpart, loss_dev);
     c->launches += 2;
     return HC_OK;
 }
 
-int hc_mlp_adam_impl(hc_ctx *c, const float *grad_dev, float lr, int t)
+// One step of the training: the gradient of rows [0, n) and Adam's update t,
+// each launched while the kernel before it drains.
+int hc_mlp_step_impl(hc_ctx *c, const float *x, const float *y, const float *w, int64_t n, float inv_norm, float *loss_dev,
+                     float lr, int t)
 {
-    k_adam<<<(NP + 255) / 256, 256, 0, c->stream>>>(c->mlp_p, grad_dev, c->mlp_m, c->mlp_v, lr, 0.9f, 0.999f, 1e-8f, t);
-    c->launches++;
+    const int nblk = (int)((n + TB - 1) / TB);
+    if (nblk > c->mlp_gcap) return HC_ERR_ARG;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nblk);
+    cfg.blockDim = dim3(GT);
+    cfg.dynamicSmemBytes = sizeof(GradSmem);
+    cfg.stream = c->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    HC_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_grad, reinterpret_cast<const MlpImage *>(c->mlp_image), x, y, w, n, inv_norm, c->mlp_gpart, c->mlp_lpart));
+    cfg.gridDim = dim3(RB);
+    cfg.blockDim = dim3(RT);
+    cfg.dynamicSmemBytes = 0;
+    HC_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_adam, (const float *)c->mlp_gpart, nblk, (const float *)c->mlp_lpart, loss_dev,
+                               c->mlp_p, c->mlp_m, c->mlp_v, reinterpret_cast<MlpImage *>(c->mlp_image), lr, 0.9f, 0.999f, 1e-8f, t));
+    c->launches += 2;
     return HC_OK;
 }
 
