@@ -8,7 +8,7 @@
 // stays in body order and is looked up through the index where high keys tie.
 //
 // One-sweep LSD radix sort: the key kernel counts the digits of all passes, then
-// one kernel per 8-bit pass.  A pass's tiles (4096 keys) count their digits,
+// one kernel per 8-bit pass.  A pass's tiles (1024 to 4096 keys) count their digits,
 // find the counts of all earlier tiles by decoupled look-back (hc_scan.cuh) and
 // scatter through shared memory, stable, so that each digit's run is written
 // contiguously.  Bound by latency up to 10^6 bodies (about 17 us a pass), above
@@ -22,15 +22,22 @@
 namespace {
 
 constexpr int SORT_THREADS = 256;
-constexpr int SORT_ITEMS = 16;
-constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-constexpr int WARP_KEYS = SORT_TILE / SORT_WARPS;      // contiguous keys ranked by one warp
 constexpr int NPASS = 8;
+
+// Keys a thread of a pass takes: few where tiles of 4096 leave most SMs idle and
+// a pass is one tile's latency, many where the tiles' counts (1 KB a tile and
+// pass) and the length of the digits' runs matter.  Build of 2^14, 2^16, 2^18,
+// 2^19, 2^20 bodies with 4 keys: 160, 175, 259, 365, 536 us, with 8: 165, 176,
+// 245, 343, 503, with 16: 179, 189, 253, 333, 485.
+int sort_items(int64_t n) { return n <= 1 << 15 ? 4 : n <= 1 << 18 ? 8 : 16; }
 
 // dynamic shared memory of k_sort_pass: the tile's keys and values in digit
 // order (staged so that each digit's run is written out contiguously)
-constexpr size_t SORT_PASS_SMEM = (size_t)SORT_TILE * (sizeof(unsigned long long) + sizeof(uint32_t));
+constexpr size_t sort_pass_smem(int items)
+{
+    return (size_t)items * SORT_THREADS * (sizeof(unsigned long long) + sizeof(uint32_t));
+}
 
 // Rank of each of a warp's keys among the warp's earlier keys of the same digit,
 // rounds of 32 keys in index order, with warp-private digit counters (no block
@@ -59,13 +66,15 @@ __device__ __forceinline__ uint32_t rank_round(C *cnt, int dr, int lane)
 
 // counts: digit counts of this pass over all keys; look: look-back words.
 // first: the values are the indices themselves (not read).
+template <int ITEMS>
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
     const unsigned long long *__restrict__ ihi, const uint32_t *__restrict__ ival,
     unsigned long long *__restrict__ ohi, uint32_t *__restrict__ oval, int64_t n, int shift, bool first,
     const uint32_t *counts, uint32_t *look, uint32_t *tile_ctr, int *err)
 {
-    extern __shared__ unsigned long long stage_k[];                    // [SORT_TILE]
-    uint32_t *stage_v = reinterpret_cast<uint32_t *>(stage_k + SORT_TILE);   // [SORT_TILE]
+    constexpr int TILE = ITEMS * SORT_THREADS, WARP_KEYS = ITEMS * 32;   // a warp ranks contiguous keys
+    extern __shared__ unsigned long long stage_k[];                    // [TILE]
+    uint32_t *stage_v = reinterpret_cast<uint32_t *>(stage_k + TILE);  // [TILE]
     __shared__ uint32_t s_tile;
     __shared__ uint32_t gbase[256];        // global position of the tile's first key of each digit
     __shared__ uint32_t lbase[256];        // start of each digit's run in the stage
@@ -77,20 +86,20 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
 #pragma unroll
     for (int w = 0; w < SORT_WARPS; w++) wcnt[w][tid] = 0;
     __syncthreads();
-    const int64_t tile = s_tile, base = tile * SORT_TILE;
-    const int tn = (int)(n - base < SORT_TILE ? n - base : SORT_TILE);
+    const int64_t tile = s_tile, base = tile * TILE;
+    const int tn = (int)(n - base < TILE ? n - base : TILE);
     // each warp loads and ranks its contiguous slice [wid * WARP_KEYS, +WARP_KEYS)
-    unsigned long long k[SORT_ITEMS];
-    uint32_t va[SORT_ITEMS];
+    unsigned long long k[ITEMS];
+    uint32_t va[ITEMS];
 #pragma unroll
-    for (int r = 0; r < SORT_ITEMS; r++) {
+    for (int r = 0; r < ITEMS; r++) {
         const int e = wid * WARP_KEYS + r * 32 + lane;
         k[r] = e < tn ? ihi[base + e] : 0ull;
         va[r] = first ? (uint32_t)(base + e) : (e < tn ? ival[base + e] : 0u);
     }
-    uint32_t rk[SORT_ITEMS / 2];           // ranks in the warp, two 16-bit values per word
+    uint32_t rk[ITEMS / 2];           // ranks in the warp, two 16-bit values per word
 #pragma unroll
-    for (int r = 0; r < SORT_ITEMS; r++) {
+    for (int r = 0; r < ITEMS; r++) {
         const int e = wid * WARP_KEYS + r * 32 + lane;
         const uint32_t rank = rank_round(wcnt[wid], e < tn ? (int)((k[r] >> shift) & 255u) : 256 + lane, lane);
         if (r & 1) rk[r >> 1] |= rank << 16;
@@ -111,7 +120,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
     __syncthreads();
     // stage in digit order: run start + earlier warps' keys of the digit + rank in the warp
 #pragma unroll
-    for (int r = 0; r < SORT_ITEMS; r++) {
+    for (int r = 0; r < ITEMS; r++) {
         const int e = wid * WARP_KEYS + r * 32 + lane;
         if (e >= tn) continue;
         const int dr = (int)((k[r] >> shift) & 255u);
@@ -282,7 +291,7 @@ void small_launch(hc_ctx *c, const unsigned long long *ihi, int64_t n, unsigned 
 // once per context, before any capture
 int hc_sort_setup(hc_ctx *c)
 {
-    HC_CUDA(cudaFuncSetAttribute(k_sort_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_PASS_SMEM));
+    HC_CUDA(cudaFuncSetAttribute(k_sort_pass<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_pass_smem(16)));
     int r = small_setup<1>(c);
     if (r == HC_OK) r = small_setup<2>(c);
     if (r == HC_OK) r = small_setup<4>(c);
@@ -294,7 +303,7 @@ int hc_sort_setup(hc_ctx *c)
 // [4096, ...) look-back words, ntiles x 256 per pass
 int64_t hc_sort_scratch_words(int64_t n)
 {
-    const int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
+    const int64_t tile = sort_items(n) * SORT_THREADS, ntiles = (n + tile - 1) / tile;
     return 4096 + (int64_t)NPASS * 256 * (ntiles < 1 ? 1 : ntiles);
 }
 
@@ -317,11 +326,13 @@ int hc_radix_sort_keys(hc_ctx *c, uint32_t *scratch, unsigned long long *khi[2],
         c->launches++;
         return 1;
     }
-    const int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
+    const int items = sort_items(n);
+    const int64_t tile = items * SORT_THREADS, ntiles = (n + tile - 1) / tile;
+    auto *pass = items == 4 ? k_sort_pass<4> : items == 8 ? k_sort_pass<8> : k_sort_pass<16>;
     uint32_t *counts = scratch, *ctr = scratch + 2048, *look = scratch + 4096;
     int sel = 0;
     for (int p = 0; p < NPASS; p++) {
-        k_sort_pass<<<(unsigned)ntiles, SORT_THREADS, SORT_PASS_SMEM, c->stream>>>(
+        pass<<<(unsigned)ntiles, SORT_THREADS, sort_pass_smem(items), c->stream>>>(
             khi[sel], kval[sel], khi[sel ^ 1], kval[sel ^ 1], n, 8 * p, p == 0, counts + 256 * p,
             look + (int64_t)p * 256 * ntiles, ctr + p, &c->st->error);
         c->launches++;

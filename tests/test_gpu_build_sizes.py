@@ -101,3 +101,21 @@ def test_points_of_any_number(hc, O, n):
         a, p = ctx.forces_at(pts)
     assert (np.linalg.norm(a - ra, axis=1) <= 1e-5 * np.linalg.norm(ra, axis=1)).mean() >= 0.999
     assert (np.abs(p - rp) <= 1e-5 * np.abs(rp)).mean() >= 0.999
+
+
+# the passes' tiles: 1024 keys to 2^15 bodies, 2048 to 2^18, then 4096
+@pytest.mark.parametrize("n", [9216, 9217, 32768, 32769, 34817, 262144, 262145])
+@pytest.mark.parametrize("kind", ["massless", "ties"])
+def test_tree_at_the_passes_tile_sizes(hc, O, n, kind):
+    m, pos = _bodies(n, kind, 5)
+    ph = np.zeros((n, 2, 3))
+    ph[:, 0] = pos
+    T = O.Tree(n, 12.0)
+    assert T.build(m, pos, True) == 0
+    ref = T.dump()
+    with hc.Context(n, tol=0.6, eps=0.02, fcells=12.0, usequad=True) as ctx:
+        ctx.upload(m, ph)
+        ctx.build_tree()
+        c, r = _canon(ctx.dump_tree()), _canon(ref)
+        for f in c:
+            assert np.array_equal(c[f], r[f]), f
