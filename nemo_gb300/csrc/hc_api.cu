@@ -1363,33 +1363,6 @@ int hc_learn_load_samples(hc_ctx *ctx, const float *x, const float *y, const flo
     return HC_OK;
 }
 
-__global__ void k_gather_samples(const int *perm, int n, const float *x, const float *y, const float *w, float *ox,
-                                 float *oy, float *ow)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int j = perm[i];
-        for (int k = 0; k < 12; k++) ox[(int64_t)i * 12 + k] = x[(int64_t)j * 12 + k];
-        oy[i] = y[j];
-        ow[i] = w[j];
-    }
-}
-
-// Sum of each mini-batch's weights (FP64), a block per batch.
-__global__ void __launch_bounds__(256) k_batch_weights(const float *w, int n, int batch, double *sum)
-{
-    __shared__ double red[256];
-    const int b0 = blockIdx.x * batch, nb = n - b0 < batch ? n - b0 : batch;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += 256) s += w[b0 + i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) sum[blockIdx.x] = red[0];
-}
-
 int hc_learn_train(hc_ctx *ctx, int epochs, int batch, double lr, uint64_t seed, double *loss)
 {
     if (!ctx || epochs < 1 || batch < 64 || !(lr > 0)) return HC_ERR_ARG;
@@ -1406,18 +1379,8 @@ int hc_learn_train(hc_ctx *ctx, int epochs, int batch, double lr, uint64_t seed,
     int *dperm = (int *)(sw + n);
     const int batches = (n + batch - 1) / batch;              // at most n / 64: they fit the permutation's place
     double *dsum = (double *)(((uintptr_t)dperm + 7) & ~(uintptr_t)7);
-    std::vector<int> perm(n);
-    for (int i = 0; i < n; i++) perm[i] = i;
-    uint64_t st = seed * 2862933555777941757ULL + 3037000493ULL;
-    for (int i = n - 1; i > 0; i--) {
-        st = st * 6364136223846793005ULL + 1442695040888963407ULL;
-        const int j = (int)((st >> 33) % (uint64_t)(i + 1));
-        std::swap(perm[i], perm[j]);
-    }
-    HC_CUDA(cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
-    k_gather_samples<<<hc_grid(n, 256), 256, 0, c->stream>>>(dperm, n, c->sample_x, c->sample_y, c->sample_w, sx, sy, sw);
-    k_batch_weights<<<batches, 256, 0, c->stream>>>(sw, n, batch, dsum);
-    c->launches += 2;
+    HC_TRY(hc_mlp_shuffle(c, seed, n, (unsigned *)sx, dperm));     // the rows' place is its scratch
+    HC_TRY(hc_mlp_gather(c, dperm, n, sx, sy, sw, batch, batches, dsum));
     double last = 0;
     std::vector<double> wsum(batches);
     HC_CUDA(cudaMemcpyAsync(wsum.data(), dsum, sizeof(double) * batches, cudaMemcpyDeviceToHost, c->stream));

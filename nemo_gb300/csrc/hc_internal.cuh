@@ -241,6 +241,10 @@ int hc_mlp_grad_impl(hc_ctx *c, const float *x, const float *y, const float *w, 
 int hc_mlp_step_impl(hc_ctx *c, const float *x, const float *y, const float *w, int64_t n, float inv_norm, float *loss_dev,
                      float lr, int t);
 int hc_mlp_train_setup(hc_ctx *c);
+// perm: the samples' shuffle; scratch: 4 n words
+int hc_mlp_shuffle(hc_ctx *c, uint64_t seed, int n, unsigned *scratch, int *perm);
+// the samples in that order, and each batch's sum of weights
+int hc_mlp_gather(hc_ctx *c, const int *perm, int n, float *x, float *y, float *w, int batch, int batches, double *sum);
 int64_t hc_mlp_partials(int blocks);
 int64_t hc_mlp_image_floats();
 int hc_relabel_impl(hc_ctx *c, float thr);

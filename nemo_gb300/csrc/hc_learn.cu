@@ -431,6 +431,89 @@ int hc_mlp_step_impl(hc_ctx *c, const float *x, const float *y, const float *w, 
 }
 
 namespace {
+
+// ---- the training set's shuffle ----
+// perm is that of Fisher and Yates's loop
+//     for i = n - 1 ... 1: j(i) = draw(n - 1 - i) mod (i + 1); swap(perm[i], perm[j(i)])
+// with draws of a 64-bit linear congruential generator, found without the loop.
+// Step i fixes perm[i] as what stands at j(i), and moves what stood at i there.
+// What stands at p before step i was moved there by the latest step before it,
+// the smallest i' > i with j(i') = p, from i'; if there is none it is p.  So with
+// first(p) the smallest i' > p with j(i') = p, what stands at p before step p is
+// found by following first from p to its end, about ln(n / p) links.
+// (262,144 samples: an epoch of 64 steps 1.85 -> 0.99 ms against the loop on the
+// host; the steps themselves take 0.92.)
+constexpr unsigned NONE = 0xffffffffu;
+constexpr int DRAWS = 16;                                // consecutive draws per thread
+
+__global__ void __launch_bounds__(256) k_shuffle_draw(uint64_t seed, int n, unsigned *j_of, unsigned *head, unsigned *next,
+                                                      unsigned *first)
+{
+    const uint64_t A = 6364136223846793005ULL, C = 1442695040888963407ULL;
+    const int k0 = (blockIdx.x * blockDim.x + threadIdx.x) * DRAWS;
+    if (k0 >= n - 1) return;
+    // the state after k0 draws: k0-fold composition of s -> A s + C by squaring
+    uint64_t s = seed * 2862933555777941757ULL + 3037000493ULL, a = A, c = C;
+    for (int k = k0; k; k >>= 1) {
+        if (k & 1) s = a * s + c;
+        c = a * c + c;
+        a = a * a;
+    }
+    for (int k = k0; k < k0 + DRAWS && k < n - 1; k++) {
+        s = A * s + C;
+        const unsigned i = (unsigned)(n - 1 - k), j = (unsigned)(s >> 33) % (i + 1);
+        j_of[i] = j;
+        next[i] = atomicExch(&head[j], i);               // the steps that draw j
+        if (j < i) atomicMin(&first[j], i);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_shuffle_resolve(int n, const unsigned *j_of, const unsigned *head, const unsigned *next,
+                                                         const unsigned *first, int *perm)
+{
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (unsigned)n) return;
+    unsigned p = 0, from = 0;                            // what ends up at 0 stood there before "step 0"
+    if (i > 0) {
+        p = j_of[i];
+        from = NONE;
+        for (unsigned q = head[p]; q != NONE; q = next[q])
+            if (q > i && q < from) from = q;
+    }
+    if (from != NONE)
+        for (p = from; first[p] != NONE; p = first[p]) {}
+    perm[i] = (int)p;
+}
+
+// x: 48-byte rows
+__global__ void __launch_bounds__(256) k_gather_samples(const int *perm, int n, const float4 *x, const float *y, const float *w,
+                                                        float4 *ox, float *oy, float *ow)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int64_t j = perm[i];
+#pragma unroll
+        for (int k = 0; k < 3; k++) ox[3 * (int64_t)i + k] = x[3 * j + k];
+        oy[i] = y[j];
+        ow[i] = w[j];
+    }
+}
+
+// Sum of each mini-batch's weights (FP64), a block per batch.
+__global__ void __launch_bounds__(256) k_batch_weights(const float *w, int n, int batch, double *sum)
+{
+    __shared__ double red[256];
+    const int b0 = blockIdx.x * batch, nb = n - b0 < batch ? n - b0 : batch;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nb; i += 256) s += w[b0 + i];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o; o >>= 1) {
+        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) sum[blockIdx.x] = red[0];
+}
+
 __global__ void k_relabel(const float *rel, int n, float thr, float *y)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = rel[i] <= thr ? 1.f : 0.f;
@@ -442,5 +525,24 @@ int hc_relabel_impl(hc_ctx *c, float thr)
     if (c->nsample <= 0) return HC_OK;
     k_relabel<<<hc_grid(c->nsample, 256), 256, 0, c->stream>>>(c->sample_rel, c->nsample, thr, c->sample_y);
     c->launches++;
+    return HC_OK;
+}
+
+int hc_mlp_shuffle(hc_ctx *c, uint64_t seed, int n, unsigned *scratch, int *perm)
+{
+    unsigned *j_of = scratch, *next = j_of + n, *head = next + n, *first = head + n;
+    HC_CUDA(cudaMemsetAsync(head, 0xff, sizeof(unsigned) * 2 * (size_t)n, c->stream));
+    k_shuffle_draw<<<(unsigned)((n + 256 * DRAWS - 1) / (256 * DRAWS)), 256, 0, c->stream>>>(seed, n, j_of, head, next, first);
+    k_shuffle_resolve<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, j_of, head, next, first, perm);
+    c->launches += 2;
+    return HC_OK;
+}
+
+int hc_mlp_gather(hc_ctx *c, const int *perm, int n, float *x, float *y, float *w, int batch, int batches, double *sum)
+{
+    k_gather_samples<<<hc_grid(n, 256), 256, 0, c->stream>>>(perm, n, reinterpret_cast<const float4 *>(c->sample_x),
+                                                             c->sample_y, c->sample_w, reinterpret_cast<float4 *>(x), y, w);
+    k_batch_weights<<<batches, 256, 0, c->stream>>>(w, n, batch, sum);
+    c->launches += 2;
     return HC_OK;
 }
