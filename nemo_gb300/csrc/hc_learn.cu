@@ -62,17 +62,16 @@ __global__ void k_mlp_infer(const MlpSmem *params, const float *x, int64_t n, fl
 //
 // A batch of 4096 rows is 64 blocks and a chain of 64 x 64 x 64 products (the
 // second layer, its transpose, its weights' gradient): bound by the latency of
-// one block, and in the products by what shared memory returns.  A warp takes 8
-// rows of a product, whose operand is one address for all lanes (half the
-// cycles of distinct ones), and a lane two columns: 3400 cycles a product, 4100
-// with a 4 x 4 tile per thread.  Operands needed along both dimensions are
-// stored twice, in rows of LD floats so that neither store meets a bank more
-// than twice; the weights come rounded and in that layout from the step before
+// one block.  Four warps make the products, a tile of 8 x 4 per thread (3600
+// cycles a product; the arithmetic alone would take 2048), and the other four the
+// sums beside them: the last layer, the biases and the first layer's weights.  Operands needed along
+// both dimensions are stored twice, laid out so that neither store meets a bank
+// twice; the weights come rounded and in that layout from the step before
 // (MlpImage: 900 cycles to load, 4700 from the parameters).  Pre-activations
 // stay in registers from the forward to the backward pass.  Every sum keeps one
 // order (inputs, rows, blocks ascending).  A step of 4096 rows, gradient and
 // update: 46 us with one output at a time and operands strided over the banks,
-// 14 us so.
+// 12.8 us so (14.4 with all eight warps on every part).
 constexpr int TB = 64;
 constexpr int GT = 256;
 constexpr int LD = MLP_H + 4;
@@ -85,9 +84,9 @@ struct alignas(16) MlpImage {                  // weights bf16-rounded
 };
 
 struct GradSmem {
-    MlpImage P;                                // W2T later dz1[s][k]
-    float H1[TB * LD], H1T[MLP_H * LD];        // H1[s][k], H1T[k][s]
-    float D2[TB * LD], D2T[MLP_H * LD];        // dz2[s][j], dz2[j][s]
+    MlpImage P;                                // W2T later dz1[s][k] (turned rows)
+    float H1[TB * MLP_H], H1T[MLP_H * LD];     // H1[s][k] (turned rows), H1T[k][s]
+    float D2[TB * MLP_H], D2T[MLP_H * LD];     // dz2[s][j] (turned rows), dz2[j][s]
     float H2T[MLP_H * LD];                     // H2[j][s]
     float XT[MLP_IN * LD], X[TB * 16];         // inputs [k][s]; [s][k], then 1 and zeros
     float D[TB], red[32];                      // D: dL/dz3
@@ -128,53 +127,65 @@ __device__ __forceinline__ void wait_predecessor()
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-// out[i][q] += sum over r < rows of a[r][i] b[r][q], r ascending: rows in
-// packed pairs (half the instructions to issue: 3900 -> 3400 cycles)
-template <int ROWS>
-__device__ __forceinline__ void tile_product(const float *a, const float *b, float (&out)[8][2])
+// Row r of a transposed array (64 floats) is stored turned by r / 4 chunks of four, so
+// that lanes that write one chunk each of every fourth row meet no bank twice.
+__device__ __forceinline__ int turned(int r, int chunk) { return r * MLP_H + 4 * ((chunk + (r >> 2)) & (MLP_H / 4 - 1)); }
+
+// out[i][q] += sum over r < ROWS of a[r][R + i] b[r][C + q], r ascending (arrays of
+// turned rows or of rows LD apart): tile rows in packed pairs, half the instructions
+// to issue
+template <int ROWS, bool TURNED>
+__device__ __forceinline__ void tile_product(const float *a, const float *b, int R, int C, float (&out)[8][4])
 {
-    float2 o[4][2];
+    float2 o[4][4];
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int q = 0; q < 2; q++) o[i][q] = make_float2(out[2 * i][q], out[2 * i + 1][q]);
-#pragma unroll 8
-    for (int r = 0; r < ROWS; r++) {
-        const float4 u0 = ld4(a + r * LD), u1 = ld4(a + r * LD + 4);
-        const float2 v = *reinterpret_cast<const float2 *>(b + r * LD);
-        const float2 u[4] = {lo2(u0), hi2(u0), lo2(u1), hi2(u1)};
+        for (int q = 0; q < 4; q++) o[i][q] = make_float2(out[2 * i][q], out[2 * i + 1][q]);
+#pragma unroll 2
+    for (int r0 = 0; r0 < ROWS; r0 += 4) {
+        const float *a0 = a + (TURNED ? turned(r0, R / 4) : r0 * LD + R), *a1 = a + (TURNED ? turned(r0, R / 4 + 1) : r0 * LD + R + 4),
+                    *b0 = b + (TURNED ? turned(r0, C / 4) : r0 * LD + C);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            o[i][0] = __ffma2_rn(u[i], splat2(v.x), o[i][0]);
-            o[i][1] = __ffma2_rn(u[i], splat2(v.y), o[i][1]);
+        for (int d = 0; d < 4; d++) {
+            const int step = d * (TURNED ? MLP_H : LD);
+            const float4 u0 = ld4(a0 + step), u1 = ld4(a1 + step), v = ld4(b0 + step);
+            const float2 u[4] = {lo2(u0), hi2(u0), lo2(u1), hi2(u1)};
+            const float vq[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) o[i][q] = __ffma2_rn(u[i], splat2(vq[q]), o[i][q]);
         }
     }
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
+        for (int q = 0; q < 4; q++) {
             out[2 * i][q] = o[i][q].x;
             out[2 * i + 1][q] = o[i][q].y;
         }
 }
 
-// rows i of a tile (the lanes' pairs beside each other), and its transpose
-__device__ __forceinline__ void tile_rows(const float (&t)[8][2], float *rows)
+// a tile as rows LD apart, and its transpose as turned rows
+__device__ __forceinline__ void tile_rows(const float (&t)[8][4], int R, int C, float *rows)
 {
 #pragma unroll
-    for (int i = 0; i < 8; i++) *reinterpret_cast<float2 *>(rows + i * LD) = make_float2(t[i][0], t[i][1]);
+    for (int i = 0; i < 8; i++)
+        *reinterpret_cast<float4 *>(rows + (R + i) * LD + C) = make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
 }
-__device__ __forceinline__ void tile_cols(const float (&t)[8][2], float *cols)
+__device__ __forceinline__ void tile_cols(const float (&t)[8][4], int R, int C, float *cols)
 {
 #pragma unroll
-    for (int q = 0; q < 2; q++)
+    for (int q = 0; q < 4; q++)
 #pragma unroll
         for (int i = 0; i < 8; i += 4)
-            *reinterpret_cast<float4 *>(cols + q * LD + i) = make_float4(t[i][q], t[i + 1][q], t[i + 2][q], t[i + 3][q]);
+            *reinterpret_cast<float4 *>(cols + turned(C + q, (R + i) / 4)) =
+                make_float4(t[i][q], t[i + 1][q], t[i + 2][q], t[i + 3][q]);
 }
 
 #define TILE_EACH                                                                                                      \
-    _Pragma("unroll") for (int i = 0; i < 8; i++) _Pragma("unroll") for (int q = 0; q < 2; q++)
+    _Pragma("unroll") for (int i = 0; i < 8; i++) _Pragma("unroll") for (int q = 0; q < 4; q++)
 
 __global__ void __launch_bounds__(GT) k_mlp_grad(const MlpImage *img, const float *x, const float *y, const float *wt,
                                                  int64_t n, float inv_norm, float *gpart, float *lpart)
@@ -182,7 +193,10 @@ __global__ void __launch_bounds__(GT) k_mlp_grad(const MlpImage *img, const floa
     extern __shared__ float4 grad_sm[];
     GradSmem &S = *reinterpret_cast<GradSmem *>(grad_sm);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int R = 8 * w, C = 2 * lane;                    // this thread's tile: rows R.., columns C..
+    // the first four warps make the products, a tile of 8 x 4 per thread: rows R..,
+    // columns C..; the others the sums beside them
+    const bool tiles = w < 4;
+    const int R = 16 * (w & 3) + 8 * (lane >> 4), C = 4 * (lane & 15);
     const int64_t r0 = (int64_t)blockIdx.x * TB;
     // the rows do not depend on the step before
     for (int i = tid; i < TB * 16; i += GT) {
@@ -192,10 +206,11 @@ __global__ void __launch_bounds__(GT) k_mlp_grad(const MlpImage *img, const floa
         S.X[i] = v;
         if (k < MLP_IN) S.XT[k * LD + (i >> 4)] = v;
     }
+    const int row = tid - 128;                          // the row of a thread of the fifth and sixth warp
     float yy = 0.f, ww = 0.f;
-    if (tid < TB && r0 + tid < n) {
-        yy = y[r0 + tid];
-        ww = wt ? wt[r0 + tid] : 1.f;
+    if (row >= 0 && row < TB && r0 + row < n) {
+        yy = y[r0 + row];
+        ww = wt ? wt[r0 + row] : 1.f;
     }
     wait_predecessor();
     for (int i = tid; i < (int)(sizeof(MlpImage) / 16); i += GT)
@@ -204,100 +219,79 @@ __global__ void __launch_bounds__(GT) k_mlp_grad(const MlpImage *img, const floa
     __pipeline_wait_prior(0);
     __syncthreads();
     // forward: hidden units R.., rows C..
-    float z1[8][2], z2[8][2], t[8][2];
-    TILE_EACH
-    {
-        z1[i][q] = S.P.b1[R + i];
-        z2[i][q] = S.P.b2[R + i];
+    float z1[8][4], z2[8][4], t[8][4];
+    if (tiles) {
+        TILE_EACH
+        {
+            z1[i][q] = S.P.b1[R + i];
+            z2[i][q] = S.P.b2[R + i];
+        }
+        tile_product<MLP_IN, false>(S.P.W1T, S.XT, R, C, z1);
+        TILE_EACH t[i][q] = bf(silu(z1[i][q]));
+        tile_rows(t, R, C, S.H1T);
+        tile_cols(t, R, C, S.H1);
     }
-    tile_product<MLP_IN>(S.P.W1T + R, S.XT + C, z1);
-    TILE_EACH t[i][q] = bf(silu(z1[i][q]));
-    tile_rows(t, S.H1T + R * LD + C);
-    tile_cols(t, S.H1 + C * LD + R);
     __syncthreads();
-    tile_product<MLP_H>(S.P.W2T + R, S.H1T + C, z2);
-    TILE_EACH t[i][q] = bf(silu(z2[i][q]));
-    tile_rows(t, S.H2T + R * LD + C);
+    if (tiles) {
+        tile_product<MLP_H, false>(S.P.W2T, S.H1T, R, C, z2);
+        TILE_EACH t[i][q] = bf(silu(z2[i][q]));
+        tile_rows(t, R, C, S.H2T);
+    }
     __syncthreads();
-    if (tid < TB) {
+    float lsum = 0.f;
+    if (row >= 0 && row < TB) {
         float z = S.P.b3[0];
 #pragma unroll 16
-        for (int k = 0; k < MLP_H; k++) z = fmaf(S.P.W3[k], S.H2T[k * LD + tid], z);
-        float d = 0.f, lsum = 0.f;
-        if (r0 + tid < n) {
+        for (int k = 0; k < MLP_H; k++) z = fmaf(S.P.W3[k], S.H2T[k * LD + row], z);
+        float d = 0.f;
+        if (r0 + row < n) {
             // BCE with logits: max(z,0) - z y + log(1 + exp(-|z|))
             lsum += ww * (fmaxf(z, 0.f) - z * yy + log1pf(__expf(-fabsf(z))));
             d = ww * (sig_out(z) - yy) * inv_norm;
         }
-        S.D[tid] = d;
-        if (tid >= 32) S.red[lane] = lsum;
-        yy = lsum;                                   // the first warp's losses, added below
+        S.D[row] = d;
+        if (row >= 32) S.red[lane] = lsum;
     }
     __syncthreads();
-    // backward: dz2 = d * w3 * silu'(z2)
-    TILE_EACH
-    {
-        const float z = z2[i][q], sg = sigm(z);
-        t[i][q] = S.D[C + q] * S.P.W3[R + i] * sg * (1.f + z * (1.f - sg));
-    }
-    tile_rows(t, S.D2T + R * LD + C);
-    tile_cols(t, S.D2 + C * LD + R);
-    if (w == 0) {
-        float l = yy + S.red[lane];
+    if (tiles) {
+        // backward: dz2 = d * w3 * silu'(z2)
+        TILE_EACH
+        {
+            const float z = z2[i][q], sg = sigm(z);
+            t[i][q] = S.D[C + q] * S.P.W3[R + i] * sg * (1.f + z * (1.f - sg));
+        }
+        tile_rows(t, R, C, S.D2T);
+        tile_cols(t, R, C, S.D2);
+    } else if (w == 4) {
+        float l = lsum + S.red[lane];
         for (int o = 16; o; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
         if (lane == 0) lpart[blockIdx.x] = l;
     }
     __syncthreads();
-    // dh1 = W2^T dz2 ; dz1 = dh1 * silu'(z1), over W2T
-    TILE_EACH t[i][q] = 0.f;
-    tile_product<MLP_H>(S.P.W2 + R, S.D2T + C, t);
-    TILE_EACH
-    {
-        const float z = z1[i][q], sg = sigm(z);
-        t[i][q] = t[i][q] * sg * (1.f + z * (1.f - sg));
-    }
-    float *dz1 = S.P.W2T;
-    tile_cols(t, dz1 + C * LD + R);
-    __syncthreads();
-    // parameter gradients (sums over this block's rows)
-    float *gp = gpart + (int64_t)blockIdx.x * NPS;
-    TILE_EACH t[i][q] = 0.f;
-    tile_product<TB>(S.D2 + R, S.H1 + C, t);
-#pragma unroll
-    for (int i = 0; i < 8; i++) *reinterpret_cast<float2 *>(gp + OFF_W2 + (R + i) * MLP_H + C) = make_float2(t[i][0], t[i][1]);
-    {
-        // first layer: units R.., input `lane`; the column of ones gives the biases
-        float2 g[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) g[i] = splat2(0.f);
-#pragma unroll 8
-        for (int s = 0; s < TB; s++) {
-            const float4 u0 = ld4(dz1 + s * LD + R), u1 = ld4(dz1 + s * LD + R + 4);
-            const float2 v = splat2(S.X[s * 16 + (lane & 15)]);
-            g[0] = __ffma2_rn(lo2(u0), v, g[0]);
-            g[1] = __ffma2_rn(hi2(u0), v, g[1]);
-            g[2] = __ffma2_rn(lo2(u1), v, g[2]);
-            g[3] = __ffma2_rn(hi2(u1), v, g[3]);
+    float *dz1 = S.P.W2T, *gp = gpart + (int64_t)blockIdx.x * NPS;
+    if (tiles) {
+        // dh1 = W2^T dz2 ; dz1 = dh1 * silu'(z1), over W2T
+        TILE_EACH t[i][q] = 0.f;
+        tile_product<MLP_H, false>(S.P.W2, S.D2T, R, C, t);
+        TILE_EACH
+        {
+            const float z = z1[i][q], sg = sigm(z);
+            t[i][q] = t[i][q] * sg * (1.f + z * (1.f - sg));
         }
-        if (lane <= MLP_IN) {
-            const bool wt1 = lane < MLP_IN;
-            float *o = gp + (wt1 ? OFF_W1 + R * MLP_IN + lane : OFF_B1 + R);
-            const int step = wt1 ? MLP_IN : 1;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                o[2 * i * step] = g[i].x;
-                o[(2 * i + 1) * step] = g[i].y;
-            }
-        }
-    }
-    // the other vectors: two warps each for b2 and W3, one lane for b3
-    if (w < 2) {
-        float g = 0.f;
+        tile_cols(t, R, C, dz1);
+    } else if (w < 6) {
+        // b2, and b3 by one lane
+        const int j = tid - 128;
+        float g = 0.f, g3 = 0.f;
 #pragma unroll 16
-        for (int s = 0; s < TB; s++) g += S.D2[s * LD + tid];
-        gp[OFF_B2 + tid] = g;
-    } else if (w < 4) {
-        const int k = tid - 64;
+        for (int s = 0; s < TB; s++) {
+            g += S.D2[turned(s, j / 4) + (j & 3)];
+            g3 += S.D[s];
+        }
+        gp[OFF_B2 + j] = g;
+        if (j == 0) gp[OFF_B3] = g3;
+    } else {
+        const int k = tid - 192;
         float g = 0.f;
 #pragma unroll 4
         for (int s = 0; s < TB; s += 4) {
@@ -308,11 +302,39 @@ __global__ void __launch_bounds__(GT) k_mlp_grad(const MlpImage *img, const floa
             g = fmaf(d.w, h.w, g);
         }
         gp[OFF_W3 + k] = g;
-    } else if (tid == 128) {
-        float g = 0.f;
-#pragma unroll 16
-        for (int s = 0; s < TB; s++) g += S.D[s];
-        gp[OFF_B3] = g;
+    }
+    __syncthreads();
+    if (tiles) {
+        TILE_EACH t[i][q] = 0.f;
+        tile_product<TB, true>(S.D2, S.H1, R, C, t);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            *reinterpret_cast<float4 *>(gp + OFF_W2 + (R + i) * MLP_H + C) = make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
+    } else {
+        // first layer: units R.., input `in`; the column of ones gives the biases
+        const int in = lane & 15;
+        float2 g[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) g[i] = splat2(0.f);
+#pragma unroll 8
+        for (int s = 0; s < TB; s++) {
+            const float4 u0 = ld4(dz1 + turned(s, R / 4)), u1 = ld4(dz1 + turned(s, R / 4 + 1));
+            const float2 v = splat2(S.X[s * 16 + in]);
+            g[0] = __ffma2_rn(lo2(u0), v, g[0]);
+            g[1] = __ffma2_rn(hi2(u0), v, g[1]);
+            g[2] = __ffma2_rn(lo2(u1), v, g[2]);
+            g[3] = __ffma2_rn(hi2(u1), v, g[3]);
+        }
+        if (in <= MLP_IN) {
+            const bool wt1 = in < MLP_IN;
+            float *o = gp + (wt1 ? OFF_W1 + R * MLP_IN + in : OFF_B1 + R);
+            const int step = wt1 ? MLP_IN : 1;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                o[2 * i * step] = g[i].x;
+                o[(2 * i + 1) * step] = g[i].y;
+            }
+        }
     }
 }
 
