@@ -917,11 +917,13 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             // ---- classify each candidate against the group ----
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
             int2 C = make_int2(0, 0);
-            // The error rule reads the cell's radius beside its quadrupole: loading
-            // both with the node saves the accepted cells a second round trip
-            // (Hernquist 2^22: 10.86 -> 10.70 ms).  The other rules read the
-            // quadrupole of accepted cells only; early loads did not help there.
-            constexpr bool QEARLY = QUAD && MODE == 2;
+            // The error rule reads the cell's radius beside its quadrupole, the learned
+            // one also the quadrupole (features): loading both with the node saves a
+            // second round trip, and the accepted cells a third (Hernquist 2^22, error
+            // rule: 10.86 -> 10.70 ms; 2^20, learned rule 3.87 -> 3.77).  The other
+            // rules read the quadrupole of accepted cells only; early loads did not
+            // help there.
+            constexpr bool QEARLY = MODE == 3 || (QUAD && MODE == 2);
             float4 Q0 = A, Q1 = A;
             if (have) {
                 A = g.nodeAB[2 * (int64_t)my_node];
@@ -938,7 +940,6 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                 uint32_t *row = reinterpret_cast<uint32_t *>(Qs->x) + lane * (MLP_XS / 2);
                 uint32_t w[6] = {0u, 0u, 0u, 0u, 0u, 0u};
                 if (have) {
-                    const float4 Q0 = g.nodeQ[2 * (int64_t)my_node], Q1 = g.nodeQ[2 * (int64_t)my_node + 1];
                     float f[12];
                     cell_features_inl(f, q_dmin2, q_dmax2, B.w, A.w, Q1.w, q_dmin2 * rsqrtf(q_dmin2) - Q1.w, Q0, Q1, GUV(13, amin), GUV(12, rg2),
                                       eps2, C.y >> 8, (int)cnt,
@@ -989,7 +990,6 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                         if (acc) accm = my_mask;
                         else openm = my_mask;
                     } else if (MODE == 3) {
-                        const float4 Q1 = g.nodeQ[2 * (int64_t)my_node + 1];
                         const float b = Q1.w;
                         // approximate square root and reciprocal: the proxy decides
                         // nothing exactly (dmin2 = 0 gives a NaN gap: opened)
@@ -1011,7 +1011,7 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
                                 const int slot = atomicAdd(g.sample_count, 1);
                                 if (slot < g.sample_cap) {
                                     float f[12];
-                                    cell_features(f, dmin2, dmax2, dsq, A.w, b, gap, g.nodeQ[2 * (int64_t)my_node], Q1,
+                                    cell_features(f, dmin2, dmax2, dsq, A.w, b, gap, Q0, Q1,
                                                   GUV(13, amin), GUV(12, rg2), eps2, C.y >> 8, (int)cnt, p_raw);
                                     for (int k = 0; k < 12; k++) g.sample_x[(int64_t)slot * 12 + k] = f[k];
                                     g.sample_group[slot] = (int)grp;
