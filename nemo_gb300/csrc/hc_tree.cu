@@ -623,9 +623,9 @@ __device__ __forceinline__ int cell_group(int2 C) { return min((C.y >> 8), 31) *
 
 // Node records that do not need the upward pass: body leaves (from the bodies'
 // 32-byte records) and the child range of every cell; counts the cells of each
-// group.  Bound by the gather of the leaves' records and the stores: with the
-// four FP64 arrays gathered apart (four 32-byte sectors a leaf instead of one)
-// it took 56 us at N = 2^20, 380 at 2^22 and 1960 at 2^24.
+// group.  Bound by the gather of the leaves' records and the stores (36 us at
+// N = 2^20): with the four FP64 arrays gathered apart (four 32-byte sectors a
+// leaf instead of one) it took 56 us, 380 at 2^22 and 1960 at 2^24.
 __global__ void __launch_bounds__(256) k_node_init(const uint8_t *bdep, const uint32_t *ba, const int32_t *blink,
                                                    const uint32_t *midx, const double4_32a *body, const hc_box *box,
                                                    int2 *nodeC, float4 *nodeAB, float4 *nodeQ, double4_32a *nodeD,
