@@ -370,8 +370,10 @@ __global__ void __launch_bounds__(RT) k_mlp_adam(const float *gpart, int nblk, c
     if (i >= NP) return;
     const float mi = m[i], vi = v[i], pi = p[i];
     const float g = sum_blocks(gpart + i, nblk, NPS);
-    const float mn = b1 * mi + (1.f - b1) * g;
-    const float vn = b2 * vi + (1.f - b2) * g * g;
+    // contracted explicitly: which product is rounded first is amplified over
+    // hundreds of steps (weights rounded to BF16 change their neighbour)
+    const float mn = fmaf(1.f - b1, g, b1 * mi);
+    const float vn = fmaf((1.f - b2) * g, g, b2 * vi);
     m[i] = mn;
     v[i] = vn;
     const float pn = pi - lr * (mn / c1) / (sqrtf(vn / c2) + eps);
