@@ -903,50 +903,50 @@ __global__ void __cluster_dims__(COFM_CLUSTER, 1, 1) __launch_bounds__(COFM_THRE
 // at most gmax (<= HC_GROUP) bodies: the cells (and lone bodies) with <= gmax bodies
 // whose parent has more, consecutive siblings packed while they fit.
 
-// A node's first massive body (key order) and its body count: the upward
-// pass's count (FP32, exact below 2^24; above it only "more than gmax"
-// matters here).
-__device__ __forceinline__ int node_count(const uint32_t *ba, const float4 *nodeQ, int k, int *first)
-{
-    const int a = (int)ba[k];
-    if (a < 0) {
-        *first = -1 - a;
-        return 1;
-    }
-    *first = a;
-    return (int)fminf(nodeQ[2 * (int64_t)k + 1].z, 2.0e9f);
-}
+// A node's body count: the upward pass's, 1 for a leaf (FP32, exact below 2^24;
+// above it only "more than gmax" matters here).
+__device__ __forceinline__ int node_count(const float4 *nodeQ, int k) { return (int)fminf(nodeQ[2 * (int64_t)k + 1].z, 2.0e9f); }
 
 // Packs of node k's children into groups (for the root also itself, when it is
-// small): calls f(first body, bodies) for each and returns their number.
+// small): calls f(first body, bodies) for each and returns their number.  cnt:
+// the node's bodies.  The children are read together: one after the other they
+// were a chain of up to eight round trips, in a kernel that only waits (2^22
+// bodies 155 -> 120 us).
 template <typename F>
-__device__ __forceinline__ int node_packs(const uint32_t *ba, const float4 *nodeQ, const int2 *nodeC, int k, int gmax,
-                                          F f)
+__device__ __forceinline__ int node_packs(const uint32_t *ba, const float4 *nodeQ, const int2 *nodeC, int k, int cnt,
+                                          int gmax, F f)
 {
-    int first, packs = 0;
-    const int cnt = node_count(ba, nodeQ, k, &first);
+    int packs = 0;
     if (cnt <= gmax) {                         // only the root can be a small group on its own here
         if (k == 0) {
-            f(first, cnt);
+            const int a = (int)ba[k];
+            f(a < 0 ? -1 - a : a, cnt);
             packs = 1;
         }
         return packs;
     }
-    const int fc = nodeC[k].x, nc = nodeC[k].y & 255;
+    const int2 C = nodeC[k];
+    const int fc = C.x, nc = C.y & 255;
+    int first[8], cc[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        first[i] = i < nc ? (int)ba[fc + i] : 0;
+        cc[i] = i < nc ? node_count(nodeQ, fc + i) : 0;
+    }
     int cur = 0, cur_first = 0;
-    for (int i = 0; i < nc; i++) {
-        int g;
-        const int cc = node_count(ba, nodeQ, fc + i, &g);
-        if (cc > gmax || cur + cc > gmax) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        if (i >= nc) break;
+        if (cc[i] > gmax || cur + cc[i] > gmax) {
             if (cur > 0) {
                 f(cur_first, cur);
                 packs++;
                 cur = 0;
             }
-            if (cc > gmax) continue;
+            if (cc[i] > gmax) continue;
         }
-        if (cur == 0) cur_first = g;
-        cur += cc;
+        if (cur == 0) cur_first = first[i] < 0 ? -1 - first[i] : first[i];
+        cur += cc[i];
     }
     if (cur > 0) {
         f(cur_first, cur);
@@ -973,10 +973,13 @@ __global__ void __launch_bounds__(256) k_groups(const uint32_t *ba, const float4
         return;
     }
     uint32_t n[GI], ex[GI];
+    int cnt[GI];
+#pragma unroll
+    for (int r = 0; r < GI; r++) cnt[r] = base + r * 256 < nn ? node_count(nodeQ, (int)(base + r * 256)) : 0;
 #pragma unroll
     for (int r = 0; r < GI; r++) {
         const int64_t k = base + r * 256;
-        n[r] = k < nn ? (uint32_t)node_packs(ba, nodeQ, nodeC, (int)k, gmax, [](int, int) {}) : 0u;
+        n[r] = k < nn ? (uint32_t)node_packs(ba, nodeQ, nodeC, (int)k, cnt[r], gmax, [](int, int) {}) : 0u;
     }
 #pragma unroll
     for (int r = 0; r < GI; r++) {
@@ -1001,9 +1004,9 @@ __global__ void __launch_bounds__(256) k_groups(const uint32_t *ba, const float4
     for (int r = 0; r < GI; r++) {
         if (n[r] == 0) continue;
         uint32_t out = s_prefix + wsum[r][wid] + ex[r];
-        node_packs(ba, nodeQ, nodeC, (int)(base + r * 256), gmax, [&](int first, int cnt) {
+        node_packs(ba, nodeQ, nodeC, (int)(base + r * 256), cnt[r], gmax, [&](int first, int bodies) {
             gstart[out] = first;
-            gcount[out] = cnt;
+            gcount[out] = bodies;
             out++;
         });
     }
