@@ -195,7 +195,7 @@ int ensure_test_capacity(hc_ctx *c, int64_t nt)
         HC_TRY(dalloc(c, &c->tkhi[i], nt));
         HC_TRY(dalloc(c, &c->tkval[i], nt));
     }
-    HC_TRY(dalloc(c, &c->thist, hc_sort_scratch_words(nt)));
+    HC_TRY(dalloc(c, &c->thist, hc_sort_scratch_capacity(nt)));   // for any smaller number too
     c->tcap = nt;
     return HC_OK;
 }

@@ -206,6 +206,8 @@ struct hc_ctx {
 // sort (hc_sort.cu)
 // 32-bit words of sort scratch for sorting n keys (n < 2^30)
 int64_t hc_sort_scratch_words(int64_t n);
+// words that serve a sort of any number of keys up to n
+int64_t hc_sort_scratch_capacity(int64_t n);
 int hc_sort_setup(hc_ctx *c);
 // true: the sort of n keys needs no scratch and no digit counts
 bool hc_sort_counts_digits(int64_t n);

@@ -30,7 +30,8 @@ constexpr int NPASS = 8;
 // pass) and the length of the digits' runs matter.  Build of 2^14, 2^16, 2^18,
 // 2^19, 2^20 bodies with 4 keys: 160, 175, 259, 365, 536 us, with 8: 165, 176,
 // 245, 343, 503, with 16: 179, 189, 253, 333, 485.
-int sort_items(int64_t n) { return n <= 1 << 15 ? 4 : n <= 1 << 18 ? 8 : 16; }
+constexpr int64_t SORT_LINE4 = 1 << 15, SORT_LINE8 = 1 << 18;
+int sort_items(int64_t n) { return n <= SORT_LINE4 ? 4 : n <= SORT_LINE8 ? 8 : 16; }
 
 // dynamic shared memory of k_sort_pass: the tile's keys and values in digit
 // order (staged so that each digit's run is written out contiguously)
@@ -305,6 +306,14 @@ int64_t hc_sort_scratch_words(int64_t n)
 {
     const int64_t tile = sort_items(n) * SORT_THREADS, ntiles = (n + tile - 1) / tile;
     return 4096 + (int64_t)NPASS * 256 * (ntiles < 1 ? 1 : ntiles);
+}
+
+// Not the words of n itself: just below a line the tiles are smaller and more
+// (200,000 keys take 98 tiles, 300,000 take 74).
+int64_t hc_sort_scratch_capacity(int64_t n)
+{
+    return std::max({hc_sort_scratch_words(n), hc_sort_scratch_words(std::min(n, SORT_LINE4)),
+                     hc_sort_scratch_words(std::min(n, SORT_LINE8))});
 }
 
 // the small sort counts its digits itself and needs no scratch

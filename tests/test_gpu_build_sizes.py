@@ -119,3 +119,24 @@ def test_tree_at_the_passes_tile_sizes(hc, O, n, kind):
         c, r = _canon(ctx.dump_tree()), _canon(ref)
         for f in c:
             assert np.array_equal(c[f], r[f]), f
+
+
+def test_test_points_fewer_than_before_in_one_context(hc):
+    """A context that served more test points serves fewer of them as a fresh one
+    does: below 2^18 and 2^15 points the sort's tiles are smaller and more."""
+    n = 3000
+    m, ph = hc.mkplummer(n, 4)
+    test = np.random.default_rng(6).uniform(-1.5, 1.5, (300000, 3))
+
+    def fresh():
+        ctx = hc.Context(n, tol=0.7, eps=0.05, usequad=True)
+        ctx.upload(m, ph)
+        ctx.build_tree()
+        return ctx
+
+    with fresh() as one:
+        for k in (40000, 30000, 300000, 200000, 262144, 32768):
+            acc, phi = one.forces_at(test[:k])
+            with fresh() as ctx:
+                a, p = ctx.forces_at(test[:k])
+            assert np.array_equal(acc, a) and np.array_equal(phi, p), k

@@ -295,3 +295,20 @@ def test_mkgalaxy_moments():
         sel = (r > 0.9 * r0) & (r < 1.1 * r0)
         meas = np.mean(np.sum(v[sl][sel] ** 2, axis=1)) / 3
         assert abs(meas / s2 - 1) < 0.08, (r0, meas, s2)
+
+
+def test_test_point_sort_scratch_serves_every_smaller_number(lib):
+    """Test-point buffers are kept for calls with fewer points, so the sort's
+    scratch that a context allocates for n points holds what any smaller number
+    takes: the sort's tiles shrink at 2^15 and 2^18 keys, where the words grow."""
+    import ctypes as C
+    L = C.CDLL(lib.LIBPATH)
+    words, capacity = L._Z21hc_sort_scratch_wordsl, L._Z24hc_sort_scratch_capacityl      # (int64_t)
+    for f in (words, capacity):
+        f.restype, f.argtypes = C.c_int64, [C.c_int64]
+    sizes = sorted({1, 2, 8192, 8193, 30000, 40000, 65537, 200000, 300000, 10 ** 6, (1 << 20) + 1} |
+                   {b + d for b in (1 << 15, 1 << 18) for d in (-4096, -2048, -1024, -1, 0, 1, 1024, 2048, 4096)})
+    for n in sizes:
+        need = max(words(k) for k in sizes if k <= n)
+        assert capacity(n) >= need, (n, capacity(n), need)
+        assert capacity(n) <= max(words(n), words(1 << 15), words(1 << 18))      # and no more than that
