@@ -98,6 +98,11 @@ int hc_get_box(hc_ctx *ctx, double rmin[3], double *rsize);
 
 /* Build the octree of the massive bodies: expandbox replay, 90-bit keys,
  * radix sort, cell linking, monopole/quadrupole upward pass.
+ * HC_ERR_ARG, with the root box left as it was: a massive body's position is
+ * not finite, or the second massive body grows the box so far past the first
+ * one's that the one-body cells between them (load.c:74-93) reach below level
+ * 31, that is a final box of more than 2^32 times the size that held the first
+ * body alone (hc_set_box to a box of the system's size avoids them).
  * Replaces: maketree + hackcofm, load.c:32-248. */
 int hc_build_tree(hc_ctx *ctx);
 int hc_tree_summary(hc_ctx *ctx, hc_tree_info *info);

@@ -51,6 +51,12 @@ int status_result(hc_ctx *c)
     case HC_ERR_STACK:
         snprintf(buf, sizeof buf, "walk: traversal stack of %d entries exhausted", s.info);
         break;
+    case HC_ERR_ARG:
+        if (s.info < 0) snprintf(buf, sizeof buf, "expandbox: non-finite position of a massive body");
+        else
+            snprintf(buf, sizeof buf, "expandbox: one-body cells down to level %d, the tree's last is %d", s.info,
+                     HC_MAXLEVEL);
+        break;
     default:
         snprintf(buf, sizeof buf, "device error %d (info %d)", s.error, s.info);
     }

@@ -20,7 +20,7 @@
 #include "hc_f32split.h"
 
 #define HC_IMAX (1 << 30)     // defs.h:124-128
-#define HC_MAXLEVEL 31        // levels 0..30
+#define HC_MAXLEVEL 31        // deepest level of a cell: 29 by the keys, 31 in an expansion chain
 #define HC_GROUP 32           // bodies per walk group of the per-body rule (one warp, one body per lane)
 #define HC_BPL 2              // bodies per lane of the group criteria's walk (3 was measured: 6% slower
                               // with 64-body groups, and groups of more than 64 bodies ran 50 times
@@ -66,7 +66,7 @@ struct hc_box {
     int max_depth;            // deepest node depth of the last build
     int nnode;                // nmassive + ncell
     int ngroups;              // tree-aligned walk groups of the massive bodies
-    int level_start[HC_MAXLEVEL + 2];  // BFS offset of each depth
+    int level_start[HC_MAXLEVEL + 3];  // BFS offset of each depth (0..32) and the number of nodes
     double dsq[HC_MAXLEVEL + 1];       // rsize^2 / 4^level (grav.c:86,105)
 };
 

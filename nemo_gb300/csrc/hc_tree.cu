@@ -254,9 +254,12 @@ __global__ void __launch_bounds__(256) k_box_replay(const double *px, const doub
         __syncthreads();
         pos = f + 1;
     }
-    if (threadIdx.x == 0 && doublings < 0) {      // non-finite position of a massive body
-        atomicCAS(&st->error, 0, HC_ERR_ARG);
-        st->info = -1;
+    // A non-finite position of a massive body, or a chain whose cells lie deeper
+    // than the node arrays go: refused, the box stays as it was.
+    const int chain = chain_before >= 0 ? doublings - chain_before - 1 : -1;
+    if (threadIdx.x == 0 && (doublings < 0 || chain > HC_MAXLEVEL)) {
+        if (atomicCAS(&st->error, 0, HC_ERR_ARG) == 0) st->info = doublings < 0 ? -1 : chain;
+        box->chain_lmax = box->chain_lmin = -1;
         return;
     }
     if (threadIdx.x == 0) {
@@ -479,14 +482,14 @@ __global__ void __launch_bounds__(256) k_depth_count(const unsigned long long *m
         if (a + 1 < M) {
             dm = lcp_digits(k, mhi[a + 1], klo, midx, a, a + 1);
             if (dm >= 30) {                    // assert(l != 0), load.c:113
-                atomicCAS(&st->error, 0, HC_ERR_COINCIDENT);
-                st->info = (int)midx[a];
+                if (atomicCAS(&st->error, 0, HC_ERR_COINCIDENT) == 0) st->info = (int)midx[a];
                 dm = 29;
             }
         }
         dm = chain_level(dm, midx, a, chain, fm);
         for (int L = dp + 1; L <= dm; L++) h[wid][L][lane]++;
-        h[wid][max(dp, dm) + 1][lane]++;
+        const int leaf = max(dp, dm) + 1;
+        if (leaf <= HC_MAXLEVEL) h[wid][leaf][lane]++;     // else the chain's: k_emit_nodes adds it
     }
     __syncthreads();
     // warp w sums depths w, w + 8, ... over all warps' columns
@@ -528,10 +531,12 @@ __global__ void __launch_bounds__(256) k_emit_nodes(const unsigned long long *mh
         if (lane == 31) start[32] = (int)incl;
     }
     __syncthreads();
-    const int total = start[32], ncell = total - M;
+    // a chain down to the last level has its body one deeper, the only node there
+    const int total = start[32] + (chain == HC_MAXLEVEL ? 1 : 0), ncell = total - M;
     const bool fits = ncell <= maxcell;            // makecell, load.c:237-239
     if (tile == 0) {
         if (tid < 33) box->level_start[tid] = fits ? start[tid] : 0;
+        if (tid == 33) box->level_start[33] = fits ? total : 0;
         if (tid == 0) {
             int md = 0;
             for (int l = 0; l < 32; l++)
@@ -540,8 +545,7 @@ __global__ void __launch_bounds__(256) k_emit_nodes(const unsigned long long *mh
             box->ncell = fits ? ncell : 0;         // else later kernels see an empty tree
             box->nnode = fits ? total : 0;
             if (!fits) {
-                atomicCAS(&st->error, 0, HC_ERR_CELLS);
-                st->info = (int)maxcell;
+                if (atomicCAS(&st->error, 0, HC_ERR_CELLS) == 0) st->info = (int)maxcell;
             }
         }
     }
@@ -568,7 +572,7 @@ __global__ void __launch_bounds__(256) k_emit_nodes(const unsigned long long *mh
         if (e >= tn) continue;
         const int dp = lev[j], dm = chain_level(lev[j + 1], midx, (int)base + e, chain, fm);
         for (int L = dp + 1; L <= dm; L++) cnt[L][tid]++;
-        cnt[max(dp, dm) + 1][tid]++;
+        if (max(dp, dm) < HC_MAXLEVEL) cnt[max(dp, dm) + 1][tid]++;
     }
     __syncthreads();
     // warp w scans depths 4 w .. 4 w + 3 over the threads (eight per lane)
@@ -604,7 +608,7 @@ __global__ void __launch_bounds__(256) k_emit_nodes(const unsigned long long *mh
         const int leaf = max(dp, dm) + 1;          // its parent is the deepest cell holding the body
         for (int L = dp + 1; L <= leaf; L++) {
             if (L > dm) L = leaf;
-            const int k = place[L] + cnt[L][tid]++;
+            const int k = L <= HC_MAXLEVEL ? place[L] + cnt[L][tid]++ : total - 1;
             bfs_a[k] = L == leaf ? (uint32_t)(-1 - a) : (uint32_t)a;
             bfs_link[k] = L < 31 ? place[L + 1] + cnt[L + 1][tid] : start[32];
             bfs_d[k] = (uint8_t)L;
@@ -660,8 +664,7 @@ __global__ void __launch_bounds__(256) k_node_init(const uint8_t *bdep, const ui
             const int end = k + 1 < box->level_start[D + 1] ? blink[k + 1] : box->level_start[D + 2];
             int nc = end - fc;
             if (fc <= k || nc < 1 || nc > 8 || fc + nc > nn) {   // children follow their parent
-                atomicCAS(&st->error, 0, HC_ERR_STATE);
-                st->info = k;
+                if (atomicCAS(&st->error, 0, HC_ERR_STATE) == 0) st->info = k;
                 fc = k + 1;
                 nc = 0;
             }

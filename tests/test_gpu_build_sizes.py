@@ -140,3 +140,59 @@ def test_test_points_fewer_than_before_in_one_context(hc):
             with fresh() as ctx:
                 a, p = ctx.forces_at(test[:k])
             assert np.array_equal(acc, a) and np.array_equal(phi, p), k
+
+
+def _chain_bodies(n, far):
+    """One body near the origin, the second at `far` on every axis (the box of
+    size 4 at (-2, -2, -2) doubles until it reaches it), the others between."""
+    rng = np.random.default_rng([n, int(far)])
+    pos = far * rng.uniform(0.1, 1.0, (n, 3))
+    pos[0], pos[1] = (0.1, -0.2, 0.3), far
+    return rng.uniform(0.5, 1.5, n) / n, pos
+
+
+# a box of 4 * 2^k: one-body cells down to level k - 1, the body one deeper
+@pytest.mark.parametrize("n", [2, 5, 20000])
+@pytest.mark.parametrize("k", [30, 31, 32])
+def test_expansion_chain_to_the_last_level(hc, O, n, k):
+    m, pos = _chain_bodies(n, 0.7 * 4.0 * 2.0 ** k)
+    ph = np.zeros((n, 2, 3))
+    ph[:, 0] = pos
+    T = O.Tree(n, 40.0)
+    assert T.build(m, pos, False) == 0
+    ref = _canon(T.dump())
+    assert ref["level"].max() == k - 1
+    ra, rp, rb, rc = T.forces(0.6, 0.02, False)
+    with hc.Context(n, tol=0.6, eps=0.02, fcells=40.0, usequad=False, count_per_body=True) as ctx:
+        ctx.upload(m, ph)
+        for _ in range(2):                       # captured, then replayed
+            ctx.set_box((-2.0, -2.0, -2.0), 4.0)
+            ctx.evaluate()
+        assert ctx.box()[1] == T.box()[1]
+        got = _canon(ctx.dump_tree())
+        for f in got:
+            if f != "quad":
+                assert np.array_equal(got[f], ref[f]), f
+        b, c = ctx.body_counts()
+        _, a, p = ctx.download(phase=False)
+    assert np.array_equal(b, rb) and np.array_equal(c, rc)
+    assert (np.linalg.norm(a - ra, axis=1) <= 1e-5 * np.linalg.norm(ra, axis=1)).all()
+    assert (np.abs(p - rp) <= 1e-5 * np.abs(rp)).all()
+
+
+@pytest.mark.parametrize("n", [5, 20000])
+@pytest.mark.parametrize("k", [33, 36, 60])
+def test_expansion_chain_below_the_last_level_is_refused(hc, n, k):
+    m, pos = _chain_bodies(n, 0.7 * 4.0 * 2.0 ** k)
+    ph = np.zeros((n, 2, 3))
+    ph[:, 0] = pos
+    with hc.Context(n, tol=0.6, eps=0.02, fcells=40.0) as ctx:
+        ctx.upload(m, ph)
+        for call in (ctx.build_tree, ctx.evaluate, ctx.evaluate):
+            with pytest.raises(hc.HCError) as e:
+                call()
+            assert e.value.code == -1 and "level %d" % (k - 1) in str(e.value)
+            assert ctx.box()[1] == 4.0           # as it was
+        ctx.set_box((-2.0, -2.0, -2.0), 4.0 * 2.0 ** k)      # held from the start: no chain
+        ctx.evaluate()
+        assert ctx.tree_info().max_level <= 30
