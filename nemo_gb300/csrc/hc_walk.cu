@@ -77,6 +77,7 @@ struct WarpSmem {
     float4 cp[CCAP / 2][5];     // cell pairs, likewise: (x y) (z m) (-Qxx -Qxy) (-Qxz -Qyy) (-Qyz -Qzz)
     uint2 cmask[CCAP / 2];      // cell pairs: accept masks (per-body rule, counting walk)
     unsigned long long stat[8]; // warp totals (lane 0 writes): see the ST_* indices
+    unsigned long long before[8];   // of them at the group's start: a walk that is given up leaves no trace
     float gu[15];               // the group's uniform values (see GU_* below), read where used
     // split walks: whether this one is split, bodies of a cell that becomes a
     // task's entry, entries kept, room for entries, first entry
@@ -809,6 +810,7 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             S.nentry = 0;
             S.entry0 = item * rule.entries;
         }
+        if (BUDGET && lane < 8) S.before[lane] = S.stat[lane];
         __syncwarp();
         int qn = 0;                                          // MODE 3: queued band candidates
         while (sp > 0 || qn > 0) {
@@ -1248,6 +1250,14 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
         }
 #undef GUV
         if (BUDGET && left < 0) {
+            // its parts count everything again
+            if (lane == 0) {
+                if (COUNT)
+                    atomicSub(&hist[(int)(cnt + BPL - 1) / BPL],
+                              (unsigned)(S.stat[ST_EB] - S.before[ST_EB] + S.stat[ST_EC] - S.before[ST_EC]) + nb + nc);
+                for (int i = 0; i < 8; i++) S.stat[i] = S.before[i];
+            }
+            __syncwarp();
             if (TEAM ? threadIdx.x == 0 : lane == 0) g.sp.out[atomicAdd(&g.sp.ctl->nout, 1)] = (int)grp;
             continue;
         }

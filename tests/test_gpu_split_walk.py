@@ -99,3 +99,39 @@ def test_closing_kick_of_a_split_group(hc):
     v_half = p0[:, 1] + 0.5 * dt * a0             # v1/2, then v1/2 + a0 dt/2 before the evaluation
     want = (v_half + 0.5 * dt * a0) + (a1 - a0) * (0.5 * dt)
     assert np.abs(p1[:, 1] - want)[far].max() <= 1e-13 * np.abs(want).max()
+
+
+# prev: accelerations of a "previous evaluation", the same in both runs
+@pytest.mark.parametrize("n,extra", [(4001, 2 ** 20), (20011, 3 * 2 ** 20)])
+@pytest.mark.parametrize("criterion,theta", [("group", 0.7), ("error", 0.05), ("learned", 0.05)])
+def test_statistics_count_a_given_up_walk_once(hc, n, extra, criterion, theta):
+    """The spread group's walk is given up and walked in parts; the statistics are
+    those of a walk in one piece.  That walk comes from the same bodies beside so
+    many massless ones that the budget (it grows with the number of groups)
+    holds; each of their groups of 64, far away, accepts the root: one candidate
+    and one cell entry."""
+    m, pos, _ = _system(n)
+    prev = -pos / (np.linalg.norm(pos, axis=1)[:, None] + 0.3) ** 3
+    rng = np.random.default_rng(2)
+    got = []
+    for k in (0, extra):
+        phase = np.zeros((n + k, 2, 3))
+        phase[:n, 0] = pos
+        phase[n:, 0] = rng.uniform(1.0e4, 1.1e4, (k, 3))
+        with hc.Context(n + k, tol=0.5, eps=0.01, usequad=True, count_per_body=True) as ctx:
+            ctx.upload(np.concatenate([m, np.zeros(k)]), phase)
+            ctx.set_forces(np.concatenate([prev, np.full((k, 3), 0.1)]))
+            if criterion == "learned":
+                ctx.learn_init(3)
+            ctx.set_criterion(criterion, theta)
+            ctx.evaluate()
+            got.append(ctx.walk_stats())
+    parts, whole = got
+    groups = extra // 64
+    hist = list(whole["mask_hist"])
+    hist[32] -= groups
+    assert parts["mask_hist"] == hist
+    assert parts["candidates"] == whole["candidates"] - groups
+    assert parts["entries_cell"] == whole["entries_cell"] - groups
+    assert parts["entries_body"] == whole["entries_body"]
+    assert parts["network"] == whole["network"] and (parts["network"] > 0) == (criterion == "learned")
