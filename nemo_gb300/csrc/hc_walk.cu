@@ -388,8 +388,6 @@ __device__ __noinline__ int split_finish(const WalkArgs &g, WarpSmem &S, const S
             if (g.phase == 2) g.sp.sub[own] = make_int2(first, T);
             else g.sp.group[atomicAdd(&g.sp.ctl->ngroup, 1)] = hc_walk_parts{s0, cnt, own, first, T};
         }
-    } else if (g.phase == 2 && lane == 0) {
-        g.sp.sub[own] = make_int2(0, 0);
     }
     __syncwarp();
     return own;
@@ -809,6 +807,8 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
         if (SPLIT && lane == 0) {
             S.nentry = 0;
             S.entry0 = item * rule.entries;
+            // the combination reads it also where this walk ends with an error
+            if (g.phase == 2) g.sp.sub[task.slot] = make_int2(0, 0);
         }
         if (BUDGET && lane < 8) S.before[lane] = S.stat[lane];
         __syncwarp();
