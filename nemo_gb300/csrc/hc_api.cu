@@ -815,7 +815,7 @@ static int launch_evaluation(hc_ctx_ext *c, int slot, double kick_dthf, int64_t 
     // what the replayed build makes (its configuration is the current one: every
     // change drops the graphs)
     c->table_gmax = hc_table_gmax(c);
-    c->have_groups = hc_build_makes_groups(c);
+    c->groups_gmax = hc_build_makes_groups(c) ? c->table_gmax : 0;
     return HC_OK;
 }
 

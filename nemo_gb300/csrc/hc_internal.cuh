@@ -121,8 +121,8 @@ struct hc_ctx {
     double4_32a *body;        // bodies' (x, y, z, mass), body order
     int32_t *gstart, *gcount; // tree-aligned groups: first massive rank, count
     int group_kind;           // 0: 32 consecutive bodies, 1: tree-aligned groups
-    int table_gmax;           // largest tree-aligned group of the current tree
-    bool have_groups;         // the current tree has its group table
+    int table_gmax;           // largest tree-aligned group by the current tree's build
+    int groups_gmax;          // largest group of the group table as it stands (0: not made for this tree)
     bool all_massive;         // every body of the last upload has mass
 
     // massive bodies in key order: views of the sort's buffers, set by the build
@@ -219,7 +219,7 @@ int hc_tree_build(hc_ctx *c);
 int hc_tree_setup(hc_ctx *c);
 int64_t hc_build_scratch_words(int64_t n, int64_t maxnode);
 bool hc_build_makes_groups(const hc_ctx *c);
-void hc_groups_launch(hc_ctx *c);
+int hc_groups_launch(hc_ctx *c, int gmax);
 int hc_tree_dump_impl(hc_ctx *c, int32_t *level, int32_t *corner, int32_t *count, double *mass,
                       double *cm, double *quad, int32_t *bparent);
 void hc_keys_for_points(hc_ctx *c, const double *x, const double *y, const double *z, int64_t n,

@@ -1114,13 +1114,21 @@ BuildScratch build_scratch(uint32_t *p, int64_t n, int64_t maxnode)
 
 int64_t hc_build_scratch_words(int64_t n, int64_t maxnode) { return build_scratch(nullptr, n, maxnode).words; }
 
-// Walk groups aligned with the tree (for c->table_gmax, fixed by the build).
-void hc_groups_launch(hc_ctx *c)
+// The current tree's table of walk groups of at most gmax bodies.  The build leaves
+// the scratch zeroed; a table made before has used it.
+int hc_groups_launch(hc_ctx *c, int gmax)
 {
     const BuildScratch b = build_scratch(c->hist, c->n, c->maxnode);
-    k_groups<<<(unsigned)((c->maxnode + GTILE - 1) / GTILE), 256, 0, c->stream>>>(
-        c->bfs_a, c->nodeQ, c->nodeC, c->box, c->table_gmax, c->gstart, c->gcount, b.groups, b.ctr + 3, &c->st->error);
+    const int64_t tiles = (c->maxnode + GTILE - 1) / GTILE;
+    if (c->groups_gmax > 0) {
+        HC_CUDA(cudaMemsetAsync(b.groups, 0, sizeof(uint32_t) * tiles, c->stream));
+        HC_CUDA(cudaMemsetAsync(b.ctr + 3, 0, sizeof(uint32_t), c->stream));
+    }
+    k_groups<<<(unsigned)tiles, 256, 0, c->stream>>>(c->bfs_a, c->nodeQ, c->nodeC, c->box, gmax, c->gstart, c->gcount,
+                                                     b.groups, b.ctr + 3, &c->st->error);
+    c->groups_gmax = gmax;
     c->launches++;
+    return HC_OK;
 }
 
 // Whether a build of this configuration makes the group table: the per-body
@@ -1206,9 +1214,8 @@ int hc_tree_build(hc_ctx *c)
 
     // 7. walk groups aligned with the tree
     c->table_gmax = hc_table_gmax(c);
-    c->have_groups = hc_build_makes_groups(c);
-    if (c->have_groups) hc_groups_launch(c);
-    return HC_OK;
+    c->groups_gmax = 0;
+    return hc_build_makes_groups(c) ? hc_groups_launch(c, c->table_gmax) : HC_OK;
 }
 
 int hc_tree_setup(hc_ctx *c)

@@ -1593,11 +1593,14 @@ int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorte
     // criterion), else 32 consecutive bodies (also the guard's fallback walk)
     const bool per_body = body_rule || c->criterion == HC_CRITERION_BODY;
     a.use_table = (self && (!per_body || (c->criterion == HC_CRITERION_BODY && c->group_kind == 1))) ? 1 : 0;
-    if (a.use_table && !c->have_groups) {
-        // the tree was built for a walk without tree groups; inside a build's
-        // capture this cannot happen (the build makes what its walk uses)
-        hc_groups_launch(c);
-        c->have_groups = true;
+    // The table this walk needs: the per-body rule holds one body a lane, so its
+    // groups are of at most 32 also on a tree built for a group criterion.
+    const int gmax = per_body ? std::min(c->table_gmax, HC_GROUP) : c->table_gmax;
+    if (a.use_table && c->groups_gmax != gmax) {
+        // the tree was built for a walk without tree groups or with larger ones;
+        // inside a build's capture this cannot happen (the build makes what its walk uses)
+        const int r = hc_groups_launch(c, gmax);
+        if (r != HC_OK) return r;
     }
     HC_CUDA(cudaMemsetAsync(a.sp.ctl, 0, sizeof(hc_walk_ctl), c->stream));
     const bool count = c->prm.count_per_body && self && c->cnt_b;

@@ -196,3 +196,38 @@ def test_expansion_chain_below_the_last_level_is_refused(hc, n, k):
         ctx.set_box((-2.0, -2.0, -2.0), 4.0 * 2.0 ** k)      # held from the start: no chain
         ctx.evaluate()
         assert ctx.tree_info().max_level <= 30
+
+
+@pytest.mark.parametrize("n", [200, 5000, 60000])
+@pytest.mark.parametrize("criterion", ["group", "error"])
+def test_body_rule_on_a_tree_built_for_larger_groups(hc, O, n, criterion):
+    """The group criteria's table holds groups of up to 64 bodies, the per-body
+    rule walks at most 32 together: on a tree built for the one, the other's walk
+    over tree groups visits every body, and the group walk afterwards is the same
+    as before it."""
+    m, pos = _bodies(n, "plain", 7)
+    ph = np.zeros((n, 2, 3))
+    ph[:, 0] = pos
+    T = O.Tree(n, 12.0)
+    assert T.build(m, pos, True) == 0
+    ra, rp, rb, rc = T.forces(0.6, 0.02, True)
+    with hc.Context(n, tol=0.6, eps=0.02, fcells=12.0, usequad=True, count_per_body=True) as ctx:
+        ctx.upload(m, ph)
+        ctx.set_criterion(criterion, 0.5)
+        ctx.build_tree()
+        ctx.forces()
+        first = ctx.download(phase=False)[1:] + ctx.body_counts()
+        ctx.set_criterion("body", 0.0)
+        ctx.set_grouping("tree")
+        ctx.forces()
+        _, a, p = ctx.download(phase=False)
+        b, c = ctx.body_counts()
+        assert np.array_equal(b, rb) and np.array_equal(c, rc)
+        assert (np.linalg.norm(a - ra, axis=1) <= 1e-5 * np.linalg.norm(ra, axis=1)).mean() >= 0.999
+        assert (np.abs(p - rp) <= 1e-5 * np.abs(rp)).all()
+        ctx.set_criterion(criterion, 0.5)
+        ctx.set_forces(np.zeros((n, 3)))          # as before the first walk: the error rule reads them
+        ctx.forces()
+        again = ctx.download(phase=False)[1:] + ctx.body_counts()
+        for x, y in zip(first, again):
+            assert np.array_equal(x, y)
