@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(256) k_emit_nodes(const unsigned long long *mh
                                                     uint8_t *bfs_d, uint32_t *status, uint32_t *ctr, hc_status *st)
 {
     __shared__ unsigned long long sk[TB + 2];      // keys of bodies base - 1 .. base + TB
-    __shared__ uint16_t cnt[32][256];
+    __shared__ __align__(16) uint16_t cnt[32][256];    // scanned in 16-byte words
     __shared__ int start[33], place[33];
     __shared__ uint32_t s_tile;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
