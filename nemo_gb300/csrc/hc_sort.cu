@@ -140,17 +140,26 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
     }
 }
 
-// stable insertion sort of the run [i, e] of equal high keys by the low key
+// Stable insertion sort of the run [i, e] of equal high keys by the low key, which
+// is a gather through the index: not read again for keys in order (many massless
+// bodies outside the box share one key), found by bisection for the others.
 __device__ __forceinline__ void order_run(const uint32_t *lo, uint32_t *val, int64_t i, int64_t e)
 {
+    uint32_t top = lo[val[i]];                       // largest so far, at a - 1
     for (int64_t a = i + 1; a <= e; a++) {
         const uint32_t kv = val[a], kl = lo[kv];
-        int64_t b = a - 1;
-        while (b >= i && lo[val[b]] > kl) {
-            val[b + 1] = val[b];
-            b--;
+        if (kl >= top) {
+            top = kl;
+            continue;
         }
-        val[b + 1] = kv;
+        int64_t p = i, q = a - 1;                    // the first larger one
+        while (p < q) {
+            const int64_t mid = (p + q) >> 1;
+            if (lo[val[mid]] > kl) q = mid;
+            else p = mid + 1;
+        }
+        for (int64_t b = a; b > q; b--) val[b] = val[b - 1];
+        val[q] = kv;
     }
 }
 

@@ -231,3 +231,30 @@ def test_body_rule_on_a_tree_built_for_larger_groups(hc, O, n, criterion):
         again = ctx.download(phase=False)[1:] + ctx.body_counts()
         for x, y in zip(first, again):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [300, 8192, 8193, 40000])
+def test_long_runs_of_equal_high_keys(hc, O, n):
+    """Runs of 2 to 60 bodies (and, massless, of a hundred outside the box) that only
+    the low keys tell apart, in every order."""
+    rng = np.random.default_rng(n)
+    m, pos = _bodies(n, "plain", 8)
+    pos = np.clip(pos, -1.9, 1.9)                # the box stays the first one, of size 4
+    at = 0
+    for k in (2, 3, 7, 31, 60):
+        # within one cell of 2^-21 of the box: its corner from the first body
+        cell = 4.0 / (1 << 21)
+        box = np.floor((pos[at] + 64.0) / cell) * cell - 64.0
+        pos[at:at + k] = box + cell * rng.choice(512, (k, 1), replace=False) / 512.0 * np.ones(3)
+        at += k
+    m[at:at + 100], pos[at:at + 100] = 0.0, 60.0 + rng.random((100, 3))
+    ph = np.zeros((n, 2, 3))
+    ph[:, 0] = pos
+    T = O.Tree(n, 60.0)
+    assert T.build(m, pos, True) == 0
+    with hc.Context(n, tol=0.6, eps=0.02, fcells=60.0, usequad=True) as ctx:
+        ctx.upload(m, ph)
+        ctx.build_tree()
+        c, r = _canon(ctx.dump_tree()), _canon(T.dump())
+        for f in ("level", "corner", "count", "mass", "cm"):
+            assert np.array_equal(c[f], r[f]), f
