@@ -13,12 +13,14 @@ on a seeded sample of 16,384 bodies.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-Prints one JSON line (rank 0).  Under torchrun (N > 1) each rank runs an
+Prints one JSON line (rank 0) of at most 1500 characters; what it leaves out
+(comparisons, calibration, training, walk statistics, the companions' figures)
+goes to stderr as a second JSON object, or into the line with --details.  Under torchrun (N > 1) each rank runs an
 independent replica of the workload on its own GPU (the path does not shard
 across GPUs); the value is the whole-job throughput.  A single-GPU default
 run also runs the other configurations briefly in child processes (the
 one-evaluation + 100-step run, the Hernquist sphere, the ensemble, 100 steps
-of the composite galaxy) and summarises their lines under "workloads"
+of the composite galaxy) and gives their values under "workloads"
 (--no-cpu-baseline skips them and the CPU baseline).
 """
 from __future__ import annotations
@@ -605,16 +607,50 @@ def run_ours(args, world, rank, local):
     if world == 1 and rank == 0 and not args.no_cpu_baseline:
         out["workloads"] = companion_workloads()
     if rank == 0:
-        print(json.dumps(out), flush=True)
+        if args.details:
+            print(json.dumps(out), flush=True)
+        else:
+            print(json.dumps({"details": out}), file=sys.stderr, flush=True)
+            print(result_line(out), flush=True)
+
+
+# What the result line keeps: whole values, or of an object these keys (and of
+# the companions their values).  The whole of `out` is some 20 KB, more than a
+# reader that keeps the end of the output may see.
+LINE_KEYS = {
+    "metric": None, "value": None, "unit": None, "n_gpus": None, "steps": None, "warmup": None, "ms_per_step": None,
+    "higher_is_better": None, "scaling": None, "vs_baseline": None, "dtype": None, "data": None, "config": None,
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"), "gpu_launches": None,
+    "roofline": ("bound", "achieved", "peak", "unit", "frac"),
+    "headline": ("rms", "target_rms"),
+    "ratios": ("learned_vs_fixed_theta_equal_rms",), "clocks": None,
+    "cpu_baseline": ("value", "cores", "kind"), "workloads": "value",
+}
+
+
+def result_line(out):
+    def short(v):
+        return float(f"{v:.6g}") if isinstance(v, float) else v
+    line = {}
+    for key, keep in LINE_KEYS.items():
+        if key not in out:
+            continue
+        v = out[key]
+        if keep == "value":
+            v = {k: short(d.get("value")) for k, d in v.items()}
+        elif keep is not None:
+            v = {k: short(v[k]) for k in keep if k in v}
+        line[key] = v
+    return json.dumps(line, separators=(",", ":"))
 
 
 # the other configurations, each a short run of its own workload in a child
 # process (the headline's context is closed first); their lines are
-# summarised under "workloads" so that one default run records all of them
+# summarised in the details so that one default run records all of them
 COMPANIONS = (
     ("plummer-run", ["--workload", "plummer-run", "--no-cpu-baseline"],
      ("value", "unit", "ms_per_step", "steps", "ratio_learned_vs_fixed_theta", "rms_error", "clocks")),
-    ("hernquist", ["--workload", "hernquist", "--steps", "5", "--warmup", "2", "--no-cpu-baseline"],
+    ("hernquist", ["--workload", "hernquist", "--steps", "5", "--warmup", "2", "--no-cpu-baseline", "--details"],
      ("value", "unit", "ms_per_step", "steps", "ratios", "e2e", "force_error", "clocks")),
     ("ensemble", ["--workload", "ensemble", "--steps", "5", "--warmup", "2"],
      ("value", "unit", "ms_per_step", "steps", "phase_ms", "tuning", "energy_drift", "clocks")),
@@ -1045,6 +1081,8 @@ def main():
                     help="bodies walked by the one-core CPU baseline (about 5-10 s)")
     ap.add_argument("--no-cpu-baseline", action="store_true",
                     help="GPU headline only: no CPU baseline and no companion workload runs")
+    ap.add_argument("--details", action="store_true",
+                    help="everything in the one line (else the rest goes to stderr)")
     ap.add_argument("--no-falcon", action="store_true", help="reference arm: skip the gyrfalcON (falcON) leg")
     ap.add_argument("--workload", default="plummer",
                     choices=["plummer", "plummer-run", "hernquist", "ensemble", "galaxy"],
