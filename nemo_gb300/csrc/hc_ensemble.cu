@@ -19,8 +19,8 @@
 //   3. the single-system build (keys, sort, cells, upward pass, groups) on
 //      the forest -- cells never straddle systems, and every walk group lies
 //      in one system;
-//   4. the walk of each group starts at its system's root cell (found from
-//      the pre-order cells), so no system sees another;
+//   4. the walk of each group starts at its system's root cell (found among
+//      the nodes), so no system sees another;
 //   5. systems of at most direct_max bodies: FP32 direct sum, one block per
 //      64 bodies, positions split hi + lo relative to the system's first body;
 //   6. closing half-kick inside 3-5 (code.c:175-179), per-system energies,

@@ -2,8 +2,8 @@
 //
 // Data layout in HBM (one context = one system of nbody bodies):
 //   bodies, original order, FP64 SoA: mass, pos[3], vel[3], acc[3], phi
-//   keys, sorted order: 63-bit high key (top 21 bits per axis, Morton
-//     interleaved, x most significant) + 27-bit low key + original index
+//   keys: 63-bit high key (top 21 bits per axis, Morton interleaved, x most
+//     significant) + original index in sorted order, 27-bit low key in body order
 //   tree nodes (bodies and cells) in breadth-first order, children of a
 //     cell contiguous and in subindex order 0..7 (load.c:162-177):
 //       nodeAB 2 x float4 (cm_hi.xyz, mass | cm_lo.xyz, size^2)
@@ -27,7 +27,6 @@
                               // longer for a reason not yet found; not used)
 #define HC_GROUP2 (32 * HC_BPL)  // bodies per walk group of the group criteria
 
-// Device status word (written by kernels, read by the host after a sync).
 // Guard record, kept across evaluations.
 struct hc_guard_state {
     double last_rms;              // RMS relative force error of the last check
@@ -36,6 +35,7 @@ struct hc_guard_state {
     int pad;
 };
 
+// Device status word (written by kernels, read by the host after a sync).
 struct hc_status {
     int error;                // 0 or HC_ERR_*
     int info;
@@ -209,7 +209,8 @@ int64_t hc_sort_scratch_words(int64_t n);
 // words that serve a sort of any number of keys up to n
 int64_t hc_sort_scratch_capacity(int64_t n);
 int hc_sort_setup(hc_ctx *c);
-// true: the sort of n keys needs no scratch and no digit counts
+// true: one block sorts n keys and counts their digits itself (no scratch, no
+// counts from the key kernel)
 bool hc_sort_counts_digits(int64_t n);
 // scratch: hc_sort_scratch_words(n) words, zeroed, then filled by hc_keys_for_points
 int hc_radix_sort_keys(hc_ctx *c, uint32_t *scratch, unsigned long long *khi[2], uint32_t *kval[2], int64_t n,

@@ -1519,6 +1519,14 @@ int launch(hc_ctx *c, WalkArgs &a, int variant)
     if (blocks < 1) blocks = 1;
     a.warps = (int)(full * WARPS);
     a.phase = 0;
+    // One warp a group: the learned rule (its queues and feature tiles are laid out
+    // for blocks of four warps and its network rounds are a warp's: no team form
+    // exists), forests and the guard's fallback walk.  With the two latter let
+    // through, theta = 0.6: tree phase of 2 x 2048 bodies 242 -> 204 us, 4 x 4096
+    // 325 -> 293, 2 x 16,384 410 -> 374, but 4 x 16,384 445 -> 517, 16 x 5000
+    // 457 -> 528 and 64 x 3000 644 (one warp either way); a walk that trips the
+    // guard 215 -> 140 us at 2048 bodies, 462 -> 364 at 16,384, 730 -> 682 at 50,000.
+    // The trip is the exception, and a forest would need a line of its own.
     const int team = M == 3 || a.run_flag || a.sys_root ? 1 : team_warps(c, a.ntarget, a.use_table);
     if (team > 1) {
         if constexpr (M != 3)
