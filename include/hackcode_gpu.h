@@ -139,7 +139,8 @@ int hc_set_graphs(hc_ctx *ctx, int on);
 
 /* Forces at ntest separate test points that are not part of the tree
  * (hackforce test=, hackforce.c:206-213).  test_pos is host [ntest][3];
- * acc [ntest][3] / phi [ntest] receive the results (host). */
+ * acc [ntest][3] / phi [ntest] receive the results (host).  Under the error
+ * and learned criteria point i's share of its group's |a| is body i % nbody's. */
 int hc_forces_at(hc_ctx *ctx, const double *test_pos, int64_t ntest, double *acc, double *phi);
 
 /* Download PhaseSpace / Acceleration / Potential (any may be NULL).

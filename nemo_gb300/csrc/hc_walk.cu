@@ -133,6 +133,7 @@ struct WalkArgs {
     int use_table;                        // 1: table groups, then massless targets in 32s
     float eps_acc;                        // MODE 2/3 error budget relative to |a|
     const double *pax, *pay, *paz;        // MODE 2/3: accelerations of the previous evaluation
+    uint32_t nbody;                       // their number
     const int *run_flag;                  // when set: the walk runs only if *run_flag != 0
     int flush_at;                         // lists are evaluated once they hold more entries (<= 32;
                                           // one iteration appends at most 32)
@@ -571,7 +572,9 @@ __global__ void __launch_bounds__(TEAM ? TEAM_MAX * 32 : WARPS * 32, TEAM ? 1 : 
             float am = 3.0e38f;
 #pragma unroll
             for (int k = 0; k < BPL; k++) {
-                const float ax1 = (float)g.pax[o[k]], ay1 = (float)g.pay[o[k]], az1 = (float)g.paz[o[k]];
+                // test points have none of their own: the bodies' in turn stand for them
+                const uint32_t b = g.self_mode ? o[k] : o[k] % g.nbody;
+                const float ax1 = (float)g.pax[b], ay1 = (float)g.pay[b], az1 = (float)g.paz[b];
                 if (valid[k]) am = fminf(am, sqrtf(fmaf(ax1, ax1, fmaf(ay1, ay1, az1 * az1))));
             }
             amin = wmin(am);
@@ -1591,6 +1594,7 @@ int hc_walk_launch(hc_ctx *c, bool self, int64_t ntarget, const uint32_t *tsorte
     a.vz = c->vz;
     a.st = c->st;
     a.sp = c->split;
+    a.nbody = (uint32_t)c->n;
     a.pax = c->ax;
     a.pay = c->ay;
     a.paz = c->az;

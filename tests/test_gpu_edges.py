@@ -292,3 +292,27 @@ def test_evaluate_host_matches_the_device_path(hc, graphs, crit):
             out.append((a, p, a2, p2))
     for x, y in zip(out[0], out[1]):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n,nt", [(1, 70), (100, 5000), (3000, 3001)])
+def test_more_test_points_than_bodies_under_the_error_rule(hc, n, nt):
+    """Test points have no previous accelerations of their own: the bodies' stand
+    for them in turn, also where there are more points than bodies."""
+    m, ph = hc.mkplummer(n, 12)
+    rng = np.random.default_rng(5)
+    tp = rng.normal(0.0, 0.7, (nt, 3))
+    with hc.Context(n, tol=0.4, eps=0.05, usequad=True) as ctx:
+        ctx.upload(m, ph)
+        ctx.set_forces(np.tile([0.3, 0.0, 0.4], (n, 1)))
+        ctx.set_criterion("error", 0.001)
+        ctx.build_tree()
+        a, p = ctx.forces_at(tp)
+        part = [ctx.forces_at(tp[i:i + 1]) for i in (0, nt // 2, nt - 1)]
+    d = ph[None, :, 0] - tp[:, None]
+    w = m / np.sqrt((d * d).sum(2) + 0.05 ** 2)
+    ea, ep = ((w ** 3 / m ** 2)[:, :, None] * d).sum(1), -w.sum(1)
+    # every group's budget is 0.001 of |a| = 0.5: the same points alone have the same one
+    err = np.linalg.norm(a - ea, axis=1)
+    assert np.sqrt(np.mean(err ** 2)) < 5e-4 and err.max() < 5e-3
+    for i, (ai, pi) in zip((0, nt // 2, nt - 1), part):
+        assert np.linalg.norm(ai[0] - a[i]) < 5e-3 and abs(pi[0] - p[i]) < 5e-3 * abs(p[i])
