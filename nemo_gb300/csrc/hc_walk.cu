@@ -77,7 +77,6 @@ struct WarpSmem {
     float4 cp[CCAP / 2][5];     // cell pairs, likewise: (x y) (z m) (-Qxx -Qxy) (-Qxz -Qyy) (-Qyz -Qzz)
     uint2 cmask[CCAP / 2];      // cell pairs: accept masks (per-body rule, counting walk)
     unsigned long long stat[8]; // warp totals (lane 0 writes): see the ST_* indices
-    unsigned long long before[8];   // of them at the group's start: a walk that is given up leaves no trace
     float gu[15];               // the group's uniform values (see GU_* below), read where used
     // split walks: whether this one is split, bodies of a cell that becomes a
     // task's entry, entries kept, room for entries, first entry
@@ -85,6 +84,7 @@ struct WarpSmem {
     float light;
     int nentry, room, entry0;
     int width;                  // lanes that the group's second bodies take (32, 16 or 8)
+    unsigned long long before[8];   // stat at the group's start: a walk that is given up leaves no trace
 };
 // Team walk (a block of W warps per group), after the warps' areas; then the
 // shared traversal stack and the candidates of an iteration.
