@@ -558,6 +558,7 @@ int hc_tree_rcrit(hc_ctx *c, int criterion, double theta, double *rcrit2)
     }
     if (!c->rcrit2) HC_TRY(dalloc(c, &c->rcrit2, c->maxnode));
     hc_rcrit_launch(c, criterion - HC_CRITERION_BH86 + 1, theta);
+    c->radii_current = false;            // those asked for, not the walk's
     HC_CUDA(cudaStreamSynchronize(c->stream));
     HC_CUDA(cudaMemcpy(c->h_box, c->box, sizeof(hc_box), cudaMemcpyDeviceToHost));
     const int nn = c->h_box->nnode;
@@ -572,6 +573,14 @@ int hc_tree_rcrit(hc_ctx *c, int criterion, double theta, double *rcrit2)
     return HC_OK;
 }
 
+// treecode1's criteria: the current tree's critical radii, where they are not there yet
+static void ensure_radii(hc_ctx *c)
+{
+    if (c->criterion < HC_CRITERION_BH86 || c->radii_current) return;
+    hc_rcrit_launch(c, c->criterion - HC_CRITERION_BH86 + 1, c->group_theta);
+    c->radii_current = true;
+}
+
 static int forces_self(hc_ctx *c, double kick_dthf, int64_t nstep)
 {
     if (!c->have_tree) {
@@ -579,6 +588,7 @@ static int forces_self(hc_ctx *c, double kick_dthf, int64_t nstep)
         return HC_ERR_STATE;
     }
     reset_status(c);
+    ensure_radii(c);
     HC_CUDA(cudaEventRecord(c->ev[2], c->stream));
     HC_TRY(hc_walk_launch(c, true, c->n, c->tord, c->px, c->py, c->pz, c->ax, c->ay, c->az, c->phi, kick_dthf,
                           nstep));
@@ -612,6 +622,7 @@ int hc_forces_at(hc_ctx *ctx, const double *test_pos, int64_t ntest, double *acc
     HC_CUDA(cudaMemsetAsync(c->thist, 0, sizeof(uint32_t) * hc_sort_scratch_words(ntest), c->stream));
     hc_keys_for_points(c, c->tx, c->ty, c->tz, ntest, c->tkhi[0], nullptr, nullptr, c->thist);
     int sel = hc_radix_sort_keys(c, c->thist, c->tkhi, c->tkval, ntest, nullptr);
+    ensure_radii(c);
     HC_CUDA(cudaEventRecord(c->ev[2], c->stream));
     HC_TRY(hc_walk_launch(c, false, ntest, c->tkval[sel], c->tx, c->ty, c->tz, c->tax, c->tay, c->taz, c->tphi,
                           0.0, 0));
@@ -736,7 +747,7 @@ static int enqueue_evaluation(hc_ctx_ext *c, double kick_dthf, int64_t nstep, bo
         HC_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
     }
     if (rb != HC_OK) return rb;
-    if (c->criterion >= HC_CRITERION_BH86) hc_rcrit_launch(c, c->criterion - HC_CRITERION_BH86 + 1, c->group_theta);
+    ensure_radii(c);
     // inputs the walk alone reads (previous accelerations) may arrive beside the build
     if (before_walk)
         HC_CUDA(cudaStreamWaitEvent(c->stream, before_walk, capturing ? cudaEventWaitExternal : 0));
@@ -816,6 +827,7 @@ static int launch_evaluation(hc_ctx_ext *c, int slot, double kick_dthf, int64_t 
     // change drops the graphs)
     c->table_gmax = hc_table_gmax(c);
     c->groups_gmax = hc_build_makes_groups(c) ? c->table_gmax : 0;
+    c->radii_current = c->criterion >= HC_CRITERION_BH86;
     return HC_OK;
 }
 
@@ -944,6 +956,7 @@ int hc_set_criterion(hc_ctx *ctx, int criterion, double theta)
     if (criterion != HC_CRITERION_BODY) HC_TRY(ensure_split(c));
     c->criterion = criterion;
     c->group_theta = theta;
+    c->radii_current = false;
     for (auto &g : c->graphs)        // captured graphs bake the walk variant
         if (g.exec) {
             cudaGraphExecDestroy(g.exec);

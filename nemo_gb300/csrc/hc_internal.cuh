@@ -123,6 +123,7 @@ struct hc_ctx {
     int group_kind;           // 0: 32 consecutive bodies, 1: tree-aligned groups
     int table_gmax;           // largest tree-aligned group by the current tree's build
     int groups_gmax;          // largest group of the group table as it stands (0: not made for this tree)
+    bool radii_current;       // rcrit2 holds the current tree's radii under the current criterion
     bool all_massive;         // every body of the last upload has mass
 
     // massive bodies in key order: views of the sort's buffers, set by the build

@@ -1215,6 +1215,7 @@ int hc_tree_build(hc_ctx *c)
     // 7. walk groups aligned with the tree
     c->table_gmax = hc_table_gmax(c);
     c->groups_gmax = 0;
+    c->radii_current = false;
     return hc_build_makes_groups(c) ? hc_groups_launch(c, c->table_gmax) : HC_OK;
 }
 

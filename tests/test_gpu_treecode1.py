@@ -125,3 +125,40 @@ def test_radii_match_treecode1_setrcrit(hc, oracle_lib, criterion):
             assert len(got) == len(ref) == len(d["level"])
             rel = np.abs(got - ref) / ref
             assert rel.max() <= 1.2e-7, (criterion, theta, rel.max())
+
+
+@pytest.mark.parametrize("criterion", ["bh86", "sw94", "barnes"])
+def test_separate_build_and_forces_make_the_radii(hc, criterion):
+    """hc_build_tree + hc_forces (and test points) walk with the current tree's
+    radii under the current criterion, as hc_evaluate does, also after
+    hc_tree_rcrit asked for others."""
+    n = 20000
+    m, ph = hc.mkplummer(n, 9)
+    tp = ph[:3000, 0] * 1.1
+    ph2 = ph.copy()
+    ph2[:, 0] *= 1.3
+
+    def run(ctx):
+        ctx.forces()
+        return ctx.download(phase=False)[1:] + ctx.forces_at(tp)
+
+    want = {}
+    with hc.Context(n, tol=0.5, eps=0.02, usequad=True) as ctx:
+        for key, p in (("a", ph), ("b", ph2)):
+            ctx.upload(m, p)
+            ctx.set_criterion(criterion, 0.7)
+            ctx.evaluate()
+            want[key] = ctx.download(phase=False)[1:] + ctx.forces_at(tp)
+    with hc.Context(n, tol=0.5, eps=0.02, usequad=True) as ctx:
+        for key, p in (("a", ph), ("b", ph2)):
+            ctx.upload(m, p)
+            ctx.set_criterion(criterion, 0.7)
+            ctx.build_tree()
+            first = run(ctx)
+            ctx.tree_rcrit("bh86", 0.3)
+            again = run(ctx)
+            ctx.set_criterion(criterion, 0.9)
+            other = run(ctx)
+            for w, x, y, z in zip(want[key], first, again, other):
+                assert np.array_equal(w, x) and np.array_equal(w, y)
+                assert not np.array_equal(w, z)
