@@ -1341,8 +1341,7 @@ int hc_learn_collect(hc_ctx *ctx, double theta, int64_t target, int64_t *nsample
     HC_TRY(hc_label_launch(c, ns, (float)theta));
     std::vector<float> ones(ns > 0 ? ns : 1, 1.0f);
     if (ns > 0) HC_CUDA(cudaMemcpyAsync(c->sample_w, ones.data(), sizeof(float) * ns, cudaMemcpyHostToDevice, c->stream));
-    HC_CUDA(cudaStreamSynchronize(c->stream));
-    HC_CUDA(cudaGetLastError());
+    HC_TRY(check_status(c));
     c->nsample = ns;
     c->band_total = counts[0];
     if (nsamples) *nsamples = ns;

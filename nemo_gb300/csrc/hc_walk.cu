@@ -1733,7 +1733,9 @@ __global__ void __launch_bounds__(128) k_label(WalkArgs g, const int *gstart, co
     const int i = blockIdx.x * 4 + w;
     if (i >= nsample) return;
     const int grp = sample_group[i], node = sample_node[i];
-    const int s0 = gstart[grp], cnt = gcount[grp];
+    // the walk's groups: the table's, then the massless bodies
+    const int ng = g.box->ngroups, m0 = g.box->nmassive + (grp - ng) * HC_GROUP2;
+    const int s0 = grp < ng ? gstart[grp] : m0, cnt = grp < ng ? gcount[grp] : (int)min((int64_t)HC_GROUP2, g.ntarget - m0);
     // groups of up to 32 HC_BPL bodies: bodies lane + 32 k on each lane
     constexpr int BPL = HC_BPL;
     bool valid[BPL];
@@ -1870,6 +1872,9 @@ int hc_label_launch(hc_ctx *c, int nsample, float eps_label)
     a.nodeAB = c->nodeAB;
     a.nodeQ = c->nodeQ;
     a.nodeC = c->nodeC;
+    a.box = c->box;
+    a.st = c->st;
+    a.ntarget = c->n;
     a.eps2f = (float)(c->prm.eps * c->prm.eps);
     const int blocks = (nsample + 3) / 4;
     if (c->prm.usequad)

@@ -239,3 +239,34 @@ def test_guard(hc, plummer):
     st = ctx.guard_stats()
     assert st["checks"] == 4 and st["trips"] == 3, st
     ctx.set_guard(0)
+
+
+@pytest.mark.parametrize("n,extra", [(3000, 1), (3000, 100), (3000, 5000)])
+def test_labels_with_massless_bodies(hc, n, extra):
+    """Massless bodies are targets of the label walk in groups of their own, which
+    the tree's group table does not hold.  With every candidate kept the massive
+    groups' samples are those of the system without them, and the labels of the
+    massless groups are measured at their own bodies."""
+    m, ph = hc.mkplummer(n, 5)
+    rng = np.random.default_rng(extra)
+    far = np.zeros((extra, 2, 3))
+    far[:, 0] = rng.normal(0.0, 0.5, (extra, 3))
+    prev = np.tile([0.3, 0.0, 0.4], (n + extra, 1))
+    rows = []
+    for k in (0, extra):
+        with hc.Context(n + k, tol=0.5, eps=0.02, usequad=True) as ctx:
+            ctx.upload(np.concatenate([m, np.zeros(k)]), np.concatenate([ph, far[:k]]))
+            ctx.set_forces(prev[:n + k])
+            ctx.build_tree()
+            got = ctx.learn_collect(0.01, 4000000)
+            x, y, rel = ctx.learn_samples()
+            assert len(x) == got > 0
+            assert np.isfinite(x).all() and np.isfinite(rel).all() and (rel >= 0).all()
+            assert np.array_equal(y, (rel <= np.float32(0.01)).astype(np.float32))
+            rows.append(np.concatenate([x, rel[:, None]], axis=1))
+    without, whole = rows
+    a, b = {r.tobytes() for r in without}, [r.tobytes() for r in whole]
+    others = np.array([r for r, key in zip(whole, b) if key not in a])
+    assert a <= set(b) and len(others) > 0
+    # the band ends at 2^3 budgets of 0.01 * 0.5: a leading term of 0.04, 0.08 of |a|, and the tail beyond it
+    assert others[:, 12].max() < 0.8 and np.median(others[:, 12]) < 0.08
